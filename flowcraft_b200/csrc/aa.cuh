@@ -40,17 +40,17 @@ __device__ __forceinline__ long long aa_link(int p, const Geom& g) {
     return (long long)L::ex(p) + (long long)L::ey(p) * g.nx + (long long)L::ez(p) * g.nxy;
 }
 
-// Slot index (plane * n + cell) of post-collision population P of cell c.
+// Slot index (plane * stride + cell) of post-collision population P of cell c.
 template <int Q, int P>
 __device__ __forceinline__ size_t pop_slot(size_t c, int x, int y, int z, const Geom& g, int layout) {
     using L = Lattice<Q>;
-    if (layout == kLayoutPlanes) return (size_t)P * g.n + c;
+    if (layout == kLayoutPlanes) return (size_t)P * g.ps + c;
     if (layout == kLayoutAAEven) {
         const int tx = x + L::ex(P), ty = y + L::ey(P), tz = z + L::ez(P);
         if (tx >= 0 && ty >= 0 && tz >= 0 && tx < g.nx && ty < g.ny && tz < g.nz)
-            return (size_t)P * g.n + (size_t)((long long)c + aa_link<Q>(P, g));
+            return (size_t)P * g.ps + (size_t)((long long)c + aa_link<Q>(P, g));
     }
-    return (size_t)L::opp(P) * g.n + c;
+    return (size_t)L::opp(P) * g.ps + c;
 }
 
 // The same with a run-time direction.

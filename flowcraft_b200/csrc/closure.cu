@@ -242,7 +242,7 @@ __global__ void k_coarse_fields(const typename S::T* __restrict__ f, const uint8
             static_for<0, Q>([&](auto I) {
                 constexpr int i = decltype(I)::value;
                 constexpr int X = L::ex(i), Y = L::ey(i), Z = L::ez(i);
-                const float v = load_pop_c<Q, S, i>(f, fg.n, fc);
+                const float v = load_pop_c<Q, S, i>(f, fg.ps, fc);
                 rho += v;
                 if constexpr (X != 0) jx += (float)X * v;
                 if constexpr (Y != 0) jy += (float)Y * v;

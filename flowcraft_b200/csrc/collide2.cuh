@@ -188,4 +188,100 @@ __device__ __forceinline__ unsigned collide_offsets2(float2 (&h)[Q], float tau, 
     return bad;
 }
 
+// collide_regularized_fast for two cells in packed FP32x2 arithmetic: the
+// same operations in the same order on full populations, so each cell's
+// result has the bits of the one-cell form (the odd-nx kernels' 16-bit
+// collision). Returns the two-bit divergence mask.
+template <int Q>
+__device__ __forceinline__ unsigned collide_fast2(float2 (&f)[Q], float tau, float cs) {
+    using L = Lattice<Q>;
+    constexpr int NP = (Q - 1) / 2;
+    float2 sp[NP], dp[NP];
+    static_for<0, NP>([&](auto P) {
+        constexpr int k = decltype(P)::value, i = 2 * k + 1;
+        sp[k] = add2(f[i], f[i + 1]);
+        dp[k] = sub2(f[i], f[i + 1]);
+    });
+    float2 rho = f[0];
+    float2 jx = bc2(0.0f), jy = bc2(0.0f), jz = bc2(0.0f);
+    float2 sxx = bc2(0.0f), syy = bc2(0.0f), szz = bc2(0.0f), sxy = bc2(0.0f), sxz = bc2(0.0f), syz = bc2(0.0f);
+    static_for<0, NP>([&](auto P) {
+        constexpr int k = decltype(P)::value, i = 2 * k + 1;
+        constexpr int X = L::ex(i), Y = L::ey(i), Z = L::ez(i);
+        rho = add2(rho, sp[k]);
+        if constexpr (X > 0) jx = add2(jx, dp[k]);
+        if constexpr (X < 0) jx = sub2(jx, dp[k]);
+        if constexpr (Y > 0) jy = add2(jy, dp[k]);
+        if constexpr (Y < 0) jy = sub2(jy, dp[k]);
+        if constexpr (Z > 0) jz = add2(jz, dp[k]);
+        if constexpr (Z < 0) jz = sub2(jz, dp[k]);
+        if constexpr (X != 0) sxx = add2(sxx, sp[k]);
+        if constexpr (Y != 0) syy = add2(syy, sp[k]);
+        if constexpr (Z != 0) szz = add2(szz, sp[k]);
+        if constexpr (X * Y > 0) sxy = add2(sxy, sp[k]);
+        if constexpr (X * Y < 0) sxy = sub2(sxy, sp[k]);
+        if constexpr (X * Z > 0) sxz = add2(sxz, sp[k]);
+        if constexpr (X * Z < 0) sxz = sub2(sxz, sp[k]);
+        if constexpr (Y * Z > 0) syz = add2(syz, sp[k]);
+        if constexpr (Y * Z < 0) syz = sub2(syz, sp[k]);
+    });
+    const float2 inv = make_float2(rho.x > 1e-6f ? __fdividef(1.0f, rho.x) : 1.0f,
+                                   rho.y > 1e-6f ? __fdividef(1.0f, rho.y) : 1.0f);
+    const float2 ux = mul2(jx, inv), uy = mul2(jy, inv), uz = mul2(jz, inv);
+    const float2 u2 = fma2(ux, ux, fma2(uy, uy, mul2(uz, uz)));
+    const unsigned bad = (rho.x > 0.0f && rho.x < __int_as_float(0x7f800000) && u2.x <= 4.0f ? 0u : 1u) |
+                         (rho.y > 0.0f && rho.y < __int_as_float(0x7f800000) && u2.y <= 4.0f ? 0u : 2u);
+
+    constexpr float third = 1.0f / 3.0f;
+    const float2 rho3 = mul2(rho, bc2(third));
+    const float2 rux = mul2(rho, ux), ruy = mul2(rho, uy);
+    const float2 pxx = sub2(sxx, fma2(rux, ux, rho3));
+    const float2 pyy = sub2(syy, fma2(ruy, uy, rho3));
+    const float2 pzz = sub2(szz, fma2(mul2(rho, uz), uz, rho3));
+    const float2 nrux = mul2(rux, bc2(-1.0f)), nruy = mul2(ruy, bc2(-1.0f));
+    const float2 pxy = fma2(nrux, uy, sxy);
+    const float2 pxz = fma2(nrux, uz, sxz);
+    const float2 pyz = fma2(nruy, uz, syz);
+
+    const float2 off = fma2(pxy, pxy, fma2(pxz, pxz, mul2(pyz, pyz)));
+    const float2 pp = fma2(pxx, pxx, fma2(pyy, pyy, fma2(pzz, pzz, mul2(bc2(2.0f), off))));
+    auto relax = [&](float pp1, float rho1) {
+        const float pimag = pp1 > 0.0f ? pp1 * rsqrtf(pp1) : 0.0f;
+        const float rden = (rho1 < 1e-6f) ? 1e-6f : rho1;
+        const float k = __fdividef((18.0f * 1.41421356f) * cs * cs * pimag, rden);
+        const float t2 = fmaf(tau, tau, k);
+        const float omega = __fdividef(2.0f, tau + t2 * rsqrtf(t2));
+        return (1.0f - omega) * 4.5f;
+    };
+    const float2 g = make_float2(relax(pp.x, rho.x), relax(pp.y, rho.y));
+
+    const float2 tr3 = mul2(add2(add2(pxx, pyy), pzz), bc2(third));
+    const float2 ntr3 = mul2(tr3, bc2(-1.0f));
+    const float2 a = mul2(rho, fma2(bc2(-1.5f), u2, bc2(1.0f)));
+    f[0] = mul2(bc2(L::w(0)), fma2(g, ntr3, a));
+    static_for<0, NP>([&](auto P) {
+        constexpr int i = 2 * decltype(P)::value + 1;
+        constexpr int o = i + 1;
+        static_assert(L::opp(i) == o, "direction pairs must be adjacent");
+        constexpr int X = L::ex(i), Y = L::ey(i), Z = L::ez(i);
+        constexpr float w = L::w(i);
+        constexpr bool flip = !lead_positive<Q>(i);  // then o leads positive: e.u of i is exactly minus o's
+        const float2 eu = edotu2<Q, flip ? o : i>(ux, uy, uz);
+        const float2 re = mul2(rho, eu);
+        const float2 base = fma2(mul2(bc2(4.5f), re), eu, a);
+        const float2 s = mul2(bc2(3.0f), re);
+        float2 qp = ntr3;
+        if constexpr (X != 0) qp = add2(qp, pxx);
+        if constexpr (Y != 0) qp = add2(qp, pyy);
+        if constexpr (Z != 0) qp = add2(qp, pzz);
+        if constexpr (X * Y != 0) qp = fma2(bc2(2.0f * (float)(X * Y)), pxy, qp);
+        if constexpr (X * Z != 0) qp = fma2(bc2(2.0f * (float)(X * Z)), pxz, qp);
+        if constexpr (Y * Z != 0) qp = fma2(bc2(2.0f * (float)(Y * Z)), pyz, qp);
+        const float2 r = fma2(g, qp, base);
+        f[flip ? o : i] = mul2(bc2(w), add2(r, s));
+        f[flip ? i : o] = mul2(bc2(w), sub2(r, s));
+    });
+    return bad;
+}
+
 }  // namespace fc

@@ -537,9 +537,10 @@ int fc_lbm_init(fc_lbm* h, const fc_grid_desc* grid, int32_t model, const fc_opt
     for (int k = 0; k < 3; ++k) h->origin[k] = grid->origin[k];
     h->g.nxy = (long long)grid->nx * grid->ny;
     h->g.n = n;
+    h->g.ps = fc::plane_stride(n);
 
     const size_t elem = h->storage == FC_STORAGE_FP32 ? 4 : 2;
-    const size_t pop_bytes = (size_t)h->q * n * elem;
+    const size_t pop_bytes = (size_t)h->q * h->g.ps * elem + (grid->nx % 2 != 0 ? fc::kPopGuardBytes : 0);
     const size_t bits_bytes = (size_t)grid->ny * grid->nz * h->g.wpr * sizeof(uint32_t);
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) {
@@ -956,7 +957,7 @@ int fc_lbm_layer_copy(fc_lbm* h, int32_t z, int32_t next, void* buffer, int32_t 
     if (in_place(h)) return fail(h, FC_LBM_ERR_UNSUPPORTED, "layer copies need ping-pong streaming");
     DeviceGuard dg(h->device);
     const size_t elem = h->storage == FC_STORAGE_FP32 ? 4 : 2;
-    const size_t width = (size_t)h->g.nxy * elem, pitch = h->g.n * elem;
+    const size_t width = (size_t)h->g.nxy * elem, pitch = h->g.ps * elem;
     char* pop = static_cast<char*>(h->pop[next ? 1 - h->cur : h->cur]) + (size_t)z * width;
     cudaStream_t s = stream ? (cudaStream_t)stream : h->stream;
     FC_RC(enter_stream(h, s));
@@ -978,7 +979,7 @@ int fc_lbm_layer_copy_dir(fc_lbm* h, int32_t z, int32_t next, void* buffer, int3
     if (in_place(h)) return fail(h, FC_LBM_ERR_UNSUPPORTED, "layer copies need ping-pong streaming");
     DeviceGuard dg(h->device);
     const size_t elem = h->storage == FC_STORAGE_FP32 ? 4 : 2;
-    const size_t width = (size_t)h->g.nxy * elem, pitch = h->g.n * elem;
+    const size_t width = (size_t)h->g.nxy * elem, pitch = h->g.ps * elem;
     char* pop = static_cast<char*>(h->pop[next ? 1 - h->cur : h->cur]) + (size_t)z * width;
     char* buf = static_cast<char*>(buffer);
     cudaStream_t s = stream ? (cudaStream_t)stream : h->stream;
@@ -1465,8 +1466,8 @@ int batch_build(fc_lbm_batch* b) {
                                           h->g.nx +
                                       (long long)(b->q == 19 ? fc::Lattice<19>::ez(i) : fc::Lattice<15>::ez(i)) *
                                           h->g.nxy;
-                d.pp[side].src[i] = in + ((long long)i * (long long)h->g.n - off) * (long long)elem;
-                d.pp[side].dst[i] = out + (size_t)i * h->g.n * elem;
+                d.pp[side].src[i] = in + ((long long)i * (long long)h->g.ps - off) * (long long)elem;
+                d.pp[side].dst[i] = out + (size_t)i * h->g.ps * elem;
             }
         }
         d.pop[0] = h->pop[0];

@@ -13,8 +13,18 @@ struct Geom {
     int nx, ny, nz;
     int wpr;        // 32-bit words per x-row of the bulk bitmask = ceil(nx/32)
     long long nxy;  // nx*ny
-    size_t n;       // nx*ny*nz (SoA plane stride)
+    size_t n;       // nx*ny*nz
+    size_t ps;      // SoA plane stride in elements (plane_stride(n) in the solver's sets)
 };
+
+// Plane stride of the solver's population sets: even, so that every plane
+// starts on a two-element boundary and the odd-nx pair kernel can load and
+// store x-adjacent pairs whole (it differs from n only when nx, ny and nz are
+// all odd).
+constexpr size_t plane_stride(size_t n) { return n + (n & 1); }
+// Bytes behind the last plane of an odd-nx lattice: the pair kernel may read
+// (never use) one element past the last cell of a row, on the last row too.
+constexpr size_t kPopGuardBytes = 256;
 
 // Live parameters of one step (LbmSolver::Params, LbmSolver.h:61-100).
 struct StepParams {
@@ -37,17 +47,6 @@ struct StepParams {
 struct PlanePtrs {
     const void* src[19];
     void* dst[19];
-};
-
-// Work plan of the bulk shell kernel for one z range (see lbm_step.cu).
-struct ShellPlan {
-    unsigned long long n_a, n_b, n_c;  // warp items in the three regions
-    int z0;                            // first z of the range (region a)
-    int zi0;                           // first interior z (region c)
-    int nyf, yf[2];                    // Y-face rows
-    int nyi;                           // interior rows per layer (ny - 2)
-    int nzf, zf[2];                    // Z-face layers inside the range
-    int ncend, cend[2];                // end chunks of a row
 };
 
 // Per-link handling codes of a boundary-list cell, 3 bits per direction.
@@ -75,8 +74,8 @@ struct BoundaryList {
 
 // ---- launchers (defined in the .cu files) ----
 // storage: 0 fp32, 1 fp16 offset, 2 bf16 offset; q: 15 or 19.
-// Bulk cells of z range [z0, z0+zc): interior + shell kernels. *launched
-// receives the number of kernels enqueued (0..2).
+// Bulk cells of z range [z0, z0+zc). *launched receives the number of kernels
+// enqueued.
 // Learned closure (closure.cuh): fragment-ordered weights, the per-cell wall
 // distance and the input normalization, passed to the kernels by value.
 constexpr int kClosureIn = 5;

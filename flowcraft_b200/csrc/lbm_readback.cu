@@ -680,6 +680,7 @@ extern "C" FC_LBM_API int fc_lbm_stats_noalloc(const void* populations, const ui
     g.wpr = (nx + 31) / 32;
     g.nxy = (long long)nx * ny;
     g.n = n;
+    g.ps = n;  // the caller's planes: no padding
     const size_t want = (n + kNoAllocCellsPerBlock - 1) / kNoAllocCellsPerBlock;
     const int blocks = (int)(want < 1 ? 1 : (want > (size_t)kNoAllocMaxBlocks ? (size_t)kNoAllocMaxBlocks : want));
     const int q = model == FC_LATTICE_D3Q19 ? 19 : 15;

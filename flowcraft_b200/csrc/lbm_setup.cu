@@ -179,7 +179,7 @@ __global__ void k_seed_uniform(typename S::T* __restrict__ f, Geom g, float rho,
         if (layout == kLayoutPlanes) {
             static_for<0, Q>([&](auto I) {
                 constexpr int i = decltype(I)::value;
-                store_pop_c<Q, S, i>(f, g.n, c, e[i]);
+                store_pop_c<Q, S, i>(f, g.ps, c, e[i]);
             });
         } else {
             seed_cell<Q, S>(f, g, c, e, layout);

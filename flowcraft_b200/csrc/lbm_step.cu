@@ -3,15 +3,14 @@
 // twin shaders/lbm_step.comp.glsl:98-364), split into two kernels so the
 // kernel that touches >99% of the cells never branches on geometry:
 //
-//   k_bulk_interior  one thread per cell, warps on 32 consecutive x of one
-//   k_bulk_shell     row; a warp reads one 32-bit word of the bit-packed bulk
-//                    mask and every set lane gathers Q populations from its
-//                    upstream neighbours (coalesced SoA loads, the +-x shifts
-//                    misaligned by one element), collides, and writes Q
-//                    populations. Boundary and solid lanes just exit. The
-//                    shell kernel covers the warps that can hold a Y/Z-face
-//                    cell (mirror / bounce-back sources) or an inlet/outlet
-//                    cell; the interior kernel is a pure pull.
+//   k_bulk_pairs     two x-adjacent cells per thread; a warp covers 64 cells of
+//                    one row, reads their bits of the bit-packed bulk mask,
+//                    gathers Q populations per cell from the upstream
+//                    neighbours (aligned 2-element loads where a direction's
+//                    offset keeps the pair's alignment), collides, and writes
+//                    Q pairs. Boundary and solid cells are masked out. Warps
+//                    on a Y/Z face take mirror / bounce-back sources, warps at
+//                    a row end also update the inlet / outlet cell.
 //   k_boundary_pull  one thread per entry of the compacted boundary list:
 //                    fluid cells with a solid neighbour (halfway or Bouzidi
 //                    links) and the solid cells an outlet may read. Link kinds and
@@ -31,85 +30,21 @@
 
 namespace fc {
 
-// One bulk cell. General = false is the interior path: a pure pull from the
-// 19 (15) upstream neighbours. General = true adds the Y/Z domain-face
-// sources and the inlet/outlet lanes; it only runs in warps that can hold
-// such cells (face rows, and the first and last warp of each row), so the
-// interior never pays for the selects.
-template <int Q, class S, bool General>
-__device__ __forceinline__ void bulk_cell(const typename S::T* __restrict__ fin, typename S::T* __restrict__ fout,
-                                          const Geom& g, const StepParams& p, int x, int y, int z, uint32_t c,
-                                          int* __restrict__ diverged) {
-    using L = Lattice<Q>;
-    float f[Q];
-    if constexpr (!General) {
-        static_for<0, Q>([&](auto I) {
-            constexpr int i = decltype(I)::value;
-            f[i] = load_pop_i<Q, S, i>(fin, g.n, c - (uint32_t)link_offset<Q>(i, g));
-        });
-        if (collide<Q, S::kExact>(f, p.tau, p.cs)) atomicOr(diverged, 1);
-        static_for<0, Q>([&](auto I) {
-            constexpr int i = decltype(I)::value;
-            store_pop_i<Q, S, i>(fout, g.n, c, f[i]);
-        });
-    } else {
-        const bool inlet = x == p.inlet_x;
-        const bool outlet = !inlet && x == p.outlet_x;
-        const uint32_t nb = p.reverse ? c + 1u : c - 1u;  // outlet's upstream neighbour (LbmReference.cpp:320)
-        static_for<0, Q>([&](auto I) {
-            constexpr int i = decltype(I)::value;
-            const int py = y - L::ey(i), pz = z - L::ez(i);
-            const bool oy = py < 0 || py >= g.ny;
-            const bool oz = pz < 0 || pz >= g.nz;
-            const bool out = (oy || oz) && !outlet;
-            const int plane = out ? edge_plane<Q, i>(oy, oz, p) : i;
-            // the inlet lane reads nothing; its address is kept in bounds anyway
-            const uint32_t src = outlet ? nb : ((out || inlet) ? c : c - (uint32_t)link_offset<Q>(i, g));
-            f[i] = inlet ? 0.0f : load_plane<Q, S>(fin, plane, g.n, src, L::w(i));
-        });
-        if (outlet) {
-            // zero-gradient outlet: neighbour's fIn moments, rho relaxed
-            // toward 1 (LbmReference.cpp:275-327)
-            float nr, nu, nv, nw;
-            moments<Q>(f, nr, nu, nv, nw);
-            const float rho = nr > 1e-6f ? 1.0f + 0.999f * (nr - 1.0f) : 1.0f;
-            equilibrium_all<Q>(rho, nu, nv, nw, f);
-        } else {
-            const bool bad = collide<Q, S::kExact>(f, p.tau, p.cs);
-            if (bad && !inlet) atomicOr(diverged, 1);
-        }
-        static_for<0, Q>([&](auto I) {
-            constexpr int i = decltype(I)::value;
-            store_pop_i<Q, S, i>(fout, g.n, c, inlet ? p.feq_inlet[i] : f[i]);
-        });
-    }
-}
-
-// The bulk cells (every fluid cell without a solid neighbour, plus the fluid
-// cells of the x = 0 and x = nx-1 planes) are split by warp position into a
-// disjoint interior and shell, each its own kernel so each gets its own
-// register allocation:
-//   interior  rows with 1 <= y <= ny-2 and 1 <= z <= nz-2, 32-cell chunks
-//             1 .. wpr-2 of the row: no face, inlet or outlet cell can occur;
-//   shell     Y-face rows (all chunks), Z-face rows (all chunks), and the
-//             first and last chunk of every other row.
-// Folding the inlet/outlet planes into warps makes their accesses part of
-// coalesced requests instead of one element per 32-byte sector.
+// One bulk cell off the faces and row ends: a pure pull from the 19 (15)
+// upstream neighbours.
 template <int Q, class S>
-__global__ void __launch_bounds__(32 * kBulkRows) k_bulk_interior(const typename S::T* __restrict__ fin,
-                                                                   typename S::T* __restrict__ fout,
-                                                                   const uint32_t* __restrict__ bulk_bits, Geom g,
-                                                                   StepParams p, int z0, int* __restrict__ diverged) {
-    const int chunk = blockIdx.x + 1;
-    const int x = chunk * 32 + threadIdx.x;
-    const int y = 1 + blockIdx.y * kBulkRows + threadIdx.y;
-    const int z = z0 + blockIdx.z;
-    if (y >= g.ny - 1) return;
-    const size_t row = (size_t)z * g.ny + y;
-    const uint32_t bits = __ldg(bulk_bits + row * g.wpr + chunk);
-    if (!((bits >> threadIdx.x) & 1u)) return;
-    const uint32_t c = (uint32_t)(row * g.nx + x);
-    bulk_cell<Q, S, false>(fin, fout, g, p, x, y, z, c, diverged);
+__device__ __forceinline__ void bulk_cell(const typename S::T* __restrict__ fin, typename S::T* __restrict__ fout,
+                                          const Geom& g, const StepParams& p, uint32_t c, int* __restrict__ diverged) {
+    float f[Q];
+    static_for<0, Q>([&](auto I) {
+        constexpr int i = decltype(I)::value;
+        f[i] = load_pop_i<Q, S, i>(fin, g.ps, c - (uint32_t)link_offset<Q>(i, g));
+    });
+    if (collide<Q, S::kExact>(f, p.tau, p.cs)) atomicOr(diverged, 1);
+    static_for<0, Q>([&](auto I) {
+        constexpr int i = decltype(I)::value;
+        store_pop_i<Q, S, i>(fout, g.ps, c, f[i]);
+    });
 }
 
 // One inlet or outlet cell (x = 0 or x = nx-1, fluid): equilibrium at the
@@ -129,7 +64,7 @@ __device__ __forceinline__ void plane_cell(const typename S::T* __restrict__ fin
         const size_t nb = p.reverse ? c + 1 : c - 1;
         static_for<0, Q>([&](auto I) {
             constexpr int i = decltype(I)::value;
-            f[i] = load_pop_c<Q, S, i>(fin, g.n, nb);
+            f[i] = load_pop_c<Q, S, i>(fin, g.ps, nb);
         });
         float nr, nu, nv, nw;
         moments<Q>(f, nr, nu, nv, nw);
@@ -138,7 +73,7 @@ __device__ __forceinline__ void plane_cell(const typename S::T* __restrict__ fin
     }
     static_for<0, Q>([&](auto I) {
         constexpr int i = decltype(I)::value;
-        store_pop_c<Q, S, i>(fout, g.n, c, f[i]);
+        store_pop_c<Q, S, i>(fout, g.ps, c, f[i]);
     });
 }
 
@@ -158,7 +93,7 @@ __device__ __forceinline__ void row_end_cell(const typename S::T* __restrict__ f
     const bool mine = lane < (unsigned)Q;
     const unsigned i = mine ? lane : 0u;
     const float wi = lattice_w_rt<Q>(i);
-    typename S::T* dst = fout + (size_t)i * g.n + pc;
+    typename S::T* dst = fout + (size_t)i * g.ps + pc;
     if (px == p.inlet_x) {  // feq_inlet[i]: the equilibrium at rho 1, u = (inlet_ux, 0, 0)
         const float ux = p.inlet_ux;
         const float v = equilibrium_rt<Q>(i, 1.0f, ux, 0.0f, 0.0f, speed2(ux, 0.0f, 0.0f));
@@ -166,7 +101,7 @@ __device__ __forceinline__ void row_end_cell(const typename S::T* __restrict__ f
         return;
     }
     const size_t nb = p.reverse ? pc + 1 : pc - 1;
-    const float own = S::dec(S::ld(fin + (size_t)i * g.n + nb), wi);
+    const float own = S::dec(S::ld(fin + (size_t)i * g.ps + nb), wi);
     float f[Q];
     static_for<0, Q>([&](auto I) { f[decltype(I)::value] = __shfl_sync(0xffffffffu, own, decltype(I)::value); });
     float nr, nu, nv, nw;
@@ -191,9 +126,8 @@ __device__ __forceinline__ void row_end_cells(const typename S::T* __restrict__ 
     }
 }
 
-// Bulk cells of lattices with even nx, two x-adjacent cells per thread, every
-// row and every 64-cell chunk. A warp covers cells [64*blockIdx.x, +64) of one
-// row, so whether it touches a Y/Z domain face (`face`) or the first or last
+// Bulk cells, two x-adjacent cells per thread, every row and every 64-cell
+// chunk. A warp covers cells [64*blockIdx.x, +64) of one row, so whether it touches a Y/Z domain face (`face`) or the first or last
 // chunk of the row (`edge`) is uniform across the warp:
 //   * interior warps, and the full pairs of edge warps off the faces, run
 //     the pure pair pull (aligned 2-element loads for the e_x = 0
@@ -205,21 +139,77 @@ __device__ __forceinline__ void row_end_cells(const typename S::T* __restrict__ 
 //     are not stored;
 //   * the lane holding an x = 0 or x = nx-1 cell first updates that inlet /
 //     outlet cell.
+// Odd nx: a pair starts on an even element, so on the rows whose first cell
+// has an odd index the pairs are shifted one cell to the left (x = -1, 1,
+// 3, ...) and the first pair holds only the cell x = 0. `Par` says which
+// directions then keep the alignment (pair_aligned), at compile time, so the
+// loads need no test: of D3Q19's 19 directions 13 with nx and ny odd, 7 with
+// nx odd and ny even, 9 with nx even. The plane stride is even (plane_stride).
+// The 16-bit collision is the one-cell form (collide_regularized_fast) for
+// both cells in packed arithmetic, bit-identical to it per cell, so odd
+// lattices keep the results the one-cell kernels gave them.
+// Measured against those (one cell per thread, 2-byte loads, a second kernel
+// for the row ends and faces), 641x203x151 FP16 on a B200: 0.57 -> 0.37 ms
+// per step (34.5 -> 52 GLUPS).
+enum PairParity : int { kNxEven = 0, kNxOddNyOdd = 1, kNxOddNyEven = 2 };
+
+inline int pair_parity(const Geom& g) {
+    return g.nx % 2 == 0 ? kNxEven : (g.ny % 2 != 0 ? kNxOddNyOdd : kNxOddNyEven);
+}
+
+// Whether the upstream neighbours of an aligned pair in direction i are an
+// aligned pair: e_x + e_y nx + e_z nx ny is even.
+template <int Q>
+__host__ __device__ constexpr bool pair_aligned(int i, int par) {
+    using L = Lattice<Q>;
+    const int o = par == kNxEven ? L::ex(i) : (par == kNxOddNyOdd ? L::ex(i) + L::ey(i) + L::ez(i) : L::ex(i) + L::ey(i));
+    return o % 2 == 0;
+}
+
+// Whether stored values are collided as offsets (the 16-bit formats at even
+// nx) or as populations.
+template <class S, int Par>
+constexpr bool kOffsets = !S::kExact && Par == kNxEven;
+
+// One element / an aligned pair of a plane as the collision takes it.
+template <class S, int Par>
+__device__ __forceinline__ float pair_ld(const typename S::T* p, float w) {
+    if constexpr (kOffsets<S, Par>)
+        return S::raw(S::ld(p));
+    else
+        return S::dec(S::ld(p), w);
+}
+template <class S, int Par>
+__device__ __forceinline__ float2 pair_ld2(const typename S::T* p, float w) {
+    if constexpr (kOffsets<S, Par>)
+        return S::raw2(S::ld2(p));
+    else
+        return S::dec2(S::ld2(p), w);
+}
+
+template <int Q, class S, int Par>
+__device__ __forceinline__ unsigned pair_collide(float2 (&v)[Q], float tau, float cs) {
+    if constexpr (S::kExact || Par == kNxEven)
+        return collide_pair<Q, S>(v, tau, cs);
+    else
+        return collide_fast2<Q>(v, tau, cs);
+}
+
 // Stores the pair's post-collision values (full floats for the exact
-// format, scaled offsets otherwise): one 2-element store per plane for a full
+// format and the odd-nx kernels, scaled offsets otherwise): one 2-element store per plane for a full
 // pair, element stores for the valid cell of a partial one. The full / partial
 // test is made once for all Q planes: per plane it costs a divergence-safe
 // branch (BSSY / BSYNC) for each of the Q stores.
-template <int Q, class S>
+template <int Q, class S, int Par = kNxEven>
 __device__ __forceinline__ void store_pair(const PlanePtrs& pp, uint32_t c, const float2 (&v)[Q], unsigned pair) {
     using L = Lattice<Q>;
     using T = typename S::T;
     auto enc = [&](auto I) {
         constexpr int i = decltype(I)::value;
-        if constexpr (S::kExact)
-            return S::enc2(v[i].x, v[i].y, L::w(i));
-        else
+        if constexpr (kOffsets<S, Par>)
             return S::pack2(v[i].x, v[i].y);
+        else
+            return S::enc2(v[i].x, v[i].y, L::w(i));
     };
     if (pair == 3u) {
         static_for<0, Q>([&](auto I) {
@@ -279,7 +269,7 @@ __device__ __forceinline__ void shell_item(const PairsShell& sh, int& bx, int& b
 // block by, layer z. shell: the launch covers the shell only (interior warps
 // leave). k_bulk_pairs_tiles runs the same code for the tiles of many
 // lattices in one launch.
-template <int Q, class S>
+template <int Q, class S, int Par = kNxEven>
 __device__ __forceinline__ void pairs_tile(const typename S::T* __restrict__ fin, typename S::T* __restrict__ fout,
                                            const uint32_t* __restrict__ bulk_bits, const Geom& g,
                                            const StepParams& p, const PlanePtrs& pp, int* __restrict__ diverged,
@@ -289,20 +279,26 @@ __device__ __forceinline__ void pairs_tile(const typename S::T* __restrict__ fin
     const int y = by * kBulkRows + threadIdx.y;
     if (y >= g.ny) return;
     const size_t row = (size_t)z * g.ny + y;
-    const int k = 2 * threadIdx.x;
-    const int w = 2 * bx + (k >> 5);
-    const uint32_t bits = w < g.wpr ? __ldg(bulk_bits + row * g.wpr + w) : 0u;
-    const int x = 64 * bx + k;
-    unsigned pair = (bits >> (k & 31)) & 3u;
-    unsigned plane = 0;  // fluid inlet / outlet cells of this pair
-    if (x == 0) {
-        plane |= pair & 1u;
-        pair &= ~1u;
+    // cells of shift: with odd nx a row's first cell has the row's parity
+    const int sh = Par == kNxEven ? 0 : (int)(row & 1);
+    const int x = 64 * bx + 2 * (int)threadIdx.x - sh;
+    unsigned pair, plane = 0;  // bulk cells of this pair; its fluid inlet / outlet cells
+    if constexpr (Par == kNxEven) {
+        const int w = x >> 5;
+        const uint32_t bits = w < g.wpr ? __ldg(bulk_bits + row * g.wpr + w) : 0u;
+        pair = (bits >> (x & 31)) & 3u;
+        if (x == 0) plane |= pair & 1u;
+        if (x + 1 == g.nx - 1) plane |= pair & 2u;
+    } else {
+        const int wa = x >> 5, wb = (x + 1) >> 5;  // the two cells' words differ only on shifted rows
+        const uint32_t* words = bulk_bits + row * g.wpr;
+        const uint32_t a = x >= 0 && wa < g.wpr ? __ldg(words + wa) : 0u;
+        const uint32_t b = wb == wa ? a : (wb < g.wpr ? __ldg(words + wb) : 0u);
+        pair = ((a >> (x & 31)) & 1u) | (((b >> ((x + 1) & 31)) & 1u) << 1);
+        if (x == 0 || x == g.nx - 1) plane |= pair & 1u;
+        if (x + 1 == 0 || x + 1 == g.nx - 1) plane |= pair & 2u;
     }
-    if (x + 1 == g.nx - 1) {
-        plane |= pair & 2u;
-        pair &= ~2u;
-    }
+    pair &= ~plane;
     const uint32_t c = (uint32_t)(row * g.nx + x);
     if constexpr (!S::kExact) {  // the row-end cells by the whole warp (no interior warp holds one)
         row_end_cells<Q, S>(fin, fout, g, p, plane, x, c);
@@ -310,7 +306,7 @@ __device__ __forceinline__ void pairs_tile(const typename S::T* __restrict__ fin
     }
     if (!(pair | plane)) return;
     const bool face = (y == 0) | (y == g.ny - 1) | (z == 0) | (z == g.nz - 1);
-    const bool edge = (bx == 0) | (64 * bx + 64 >= g.nx);
+    const bool edge = (bx == 0) | (64 * bx + 64 - sh >= g.nx);
     if (shell && !face && !edge) return;  // an interior warp: done by k_bulk_tiles
 
     // FP32: the one lane of a row end that holds an inlet or outlet cell finishes it alone
@@ -319,29 +315,25 @@ __device__ __forceinline__ void pairs_tile(const typename S::T* __restrict__ fin
     float2 v[Q];
     if (!face) {
         if (pair != 3u && !edge) {  // one of the two is next to a wall (a boundary-list cell)
-            const uint32_t cc = pair == 1u ? c : c + 1u;
-            bulk_cell<Q, S, false>(fin, fout, g, p, x + (pair == 1u ? 0 : 1), y, z, cc, diverged);
+            bulk_cell<Q, S>(fin, fout, g, p, pair == 1u ? c : c + 1u, diverged);
             return;
         }
         // Full pairs, and in row-end warps every pair: the plain pull. Off the
         // Y/Z faces every source of a row lies inside the population set, also
         // for a cell that is not stored here (an inlet / outlet or wall cell
-        // next to a pair cell), so a row-end warp runs one uniform path, with
-        // the masked pair collision of the general path for its partial pairs.
+        // next to a pair cell, with odd nx the cell before or after the row),
+        // so a row-end warp runs one uniform path, with the masked pair
+        // collision of the general path for its partial pairs.
         static_for<0, Q>([&](auto I) {
             constexpr int i = decltype(I)::value;
             const T* src = static_cast<const T*>(pp.src[i]);
-            if constexpr (S::kExact) {
-                v[i] = L::ex(i) == 0 ? S::dec2(S::ld2(src + c), L::w(i))
-                                     : make_float2(S::dec(S::ld(src + c), L::w(i)),
-                                                   S::dec(S::ld(src + c + 1u), L::w(i)));
-            } else {
-                v[i] = L::ex(i) == 0 ? S::raw2(S::ld2(src + c))
-                                     : make_float2(S::raw(S::ld(src + c)), S::raw(S::ld(src + c + 1u)));
-            }
+            if constexpr (pair_aligned<Q>(i, Par))
+                v[i] = pair_ld2<S, Par>(src + c, L::w(i));
+            else
+                v[i] = make_float2(pair_ld<S, Par>(src + c, L::w(i)), pair_ld<S, Par>(src + c + 1u, L::w(i)));
         });
-        if (collide_pair<Q, S>(v, p.tau, p.cs) & pair) atomicOr(diverged, 1);
-        store_pair<Q, S>(pp, c, v, pair);
+        if (pair_collide<Q, S, Par>(v, p.tau, p.cs) & pair) atomicOr(diverged, 1);
+        store_pair<Q, S, Par>(pp, c, v, pair);
         return;
     }
     // general pair path: face rows, and partial pairs of the row-end chunks
@@ -356,18 +348,15 @@ __device__ __forceinline__ void pairs_tile(const typename S::T* __restrict__ fin
         const uint32_t off = out ? 0u : (uint32_t)link_offset<Q>(i, g);
         const uint32_t sa = va ? c - off : c;
         const uint32_t sb = vb ? c + 1u - off : c + 1u;
-        const T* base = fin + (size_t)plane * g.n;
-        if constexpr (S::kExact)
-            v[i] = make_float2(S::dec(S::ld(base + sa), L::w(i)), S::dec(S::ld(base + sb), L::w(i)));
-        else
-            v[i] = make_float2(S::raw(S::ld(base + sa)), S::raw(S::ld(base + sb)));
+        const T* base = fin + (size_t)plane * g.ps;
+        v[i] = make_float2(pair_ld<S, Par>(base + sa, L::w(i)), pair_ld<S, Par>(base + sb, L::w(i)));
     });
-    const unsigned bad = collide_pair<Q, S>(v, p.tau, p.cs) & pair;
+    const unsigned bad = pair_collide<Q, S, Par>(v, p.tau, p.cs) & pair;
     if (bad) atomicOr(diverged, 1);
-    store_pair<Q, S>(pp, c, v, pair);
+    store_pair<Q, S, Par>(pp, c, v, pair);
 }
 
-template <int Q, class S>
+template <int Q, class S, int Par>
 __global__ void __launch_bounds__(32 * kBulkRows, 4) k_bulk_pairs(const typename S::T* __restrict__ fin,
                                                                 typename S::T* __restrict__ fout,
                                                                 const uint32_t* __restrict__ bulk_bits, Geom g,
@@ -375,7 +364,7 @@ __global__ void __launch_bounds__(32 * kBulkRows, 4) k_bulk_pairs(const typename
                                                                 int* __restrict__ diverged, PairsShell sh) {
     int bx = blockIdx.x, by = blockIdx.y, z = z0 + blockIdx.z;
     if (sh.n) shell_item(sh, bx, by, z);
-    pairs_tile<Q, S>(fin, fout, bulk_bits, g, p, pp, diverged, bx, by, z, sh.n != 0);
+    pairs_tile<Q, S, Par>(fin, fout, bulk_bits, g, p, pp, diverged, bx, by, z, sh.n != 0);
 }
 
 // The bulk step of many lattices in one launch of one block per tile: the
@@ -472,7 +461,7 @@ __global__ void __launch_bounds__(32 * kBulkRows, 4) k_bulk_pairs_learned(const 
             const uint32_t off = out ? 0u : (uint32_t)link_offset<Q>(i, g);
             const uint32_t sa = va ? c - off : cs;
             const uint32_t sb = vb ? c + 1u - off : cs + 1u;
-            const T* base = fin + (size_t)pl * g.n;
+            const T* base = fin + (size_t)pl * g.ps;
             v[i] = make_float2(S::raw(S::ld(base + sa)), S::raw(S::ld(base + sb)));
         });
     }
@@ -614,7 +603,7 @@ __global__ void __launch_bounds__(32 * kBulkRows, 4) k_bulk_pairs_learned_tc(con
             const uint32_t off = out ? 0u : (uint32_t)link_offset<Q>(i, g);
             const uint32_t sa = va ? c - off : cs;
             const uint32_t sb = vb ? c + 1u - off : cs + 1u;
-            const T* base = fin + (size_t)pl * g.n;
+            const T* base = fin + (size_t)pl * g.ps;
             v[i] = make_float2(S::raw(S::ld(base + sa)), S::raw(S::ld(base + sb)));
         });
     }
@@ -824,7 +813,7 @@ __global__ void __launch_bounds__(32 * ROWS, 32 / ROWS) k_bulk_pairs_batch(const
         if (!face) {  // as k_bulk_pairs
             if (pair != 3u && !edge) {
                 const uint32_t cc = pair == 1u ? c : c + 1u;
-                bulk_cell<Q, S, false>(fin, fout, g, p, x + (pair == 1u ? 0 : 1), y, z, cc, sl.diverged);
+                bulk_cell<Q, S>(fin, fout, g, p, cc, sl.diverged);
                 continue;
             }
             static_for<0, Q>([&](auto I) {
@@ -854,7 +843,7 @@ __global__ void __launch_bounds__(32 * ROWS, 32 / ROWS) k_bulk_pairs_batch(const
             const uint32_t off = out ? 0u : (uint32_t)link_offset<Q>(i, g);
             const uint32_t sa = va ? c - off : c;
             const uint32_t sb = vb ? c + 1u - off : c + 1u;
-            const T* base = fin + (size_t)pl * g.n;
+            const T* base = fin + (size_t)pl * g.ps;
             if constexpr (S::kExact)
                 v[i] = make_float2(S::dec(S::ld(base + sa), L::w(i)), S::dec(S::ld(base + sb), L::w(i)));
             else
@@ -865,40 +854,6 @@ __global__ void __launch_bounds__(32 * ROWS, 32 / ROWS) k_bulk_pairs_batch(const
         store_pair<Q, S>(pp, c, v, pair);
     }
     }
-}
-
-template <int Q, class S>
-__global__ void __launch_bounds__(32 * kBulkRows) k_bulk_shell(const typename S::T* __restrict__ fin,
-                                                                typename S::T* __restrict__ fout,
-                                                                const uint32_t* __restrict__ bulk_bits, Geom g,
-                                                                StepParams p, ShellPlan sp, int* __restrict__ diverged) {
-    // one warp per (row, chunk) item of the shell
-    unsigned long long item = (unsigned long long)blockIdx.x * kBulkRows + threadIdx.y;
-    int chunk, y, z;
-    if (item < sp.n_a) {  // Y-face rows, every chunk
-        chunk = (int)(item % g.wpr);
-        const unsigned long long r = item / g.wpr;
-        y = sp.yf[(int)(r % sp.nyf)];
-        z = sp.z0 + (int)(r / sp.nyf);
-    } else if ((item -= sp.n_a) < sp.n_b) {  // Z-face rows off the Y faces, every chunk
-        chunk = (int)(item % g.wpr);
-        const unsigned long long r = item / g.wpr;
-        y = 1 + (int)(r % sp.nyi);
-        z = sp.zf[(int)(r / sp.nyi)];
-    } else if ((item -= sp.n_b) < sp.n_c) {  // end chunks of interior rows
-        chunk = sp.cend[(int)(item % sp.ncend)];
-        const unsigned long long r = item / sp.ncend;
-        y = 1 + (int)(r % sp.nyi);
-        z = sp.zi0 + (int)(r / sp.nyi);
-    } else {
-        return;
-    }
-    const size_t row = (size_t)z * g.ny + y;
-    const uint32_t bits = __ldg(bulk_bits + row * g.wpr + chunk);
-    if (!((bits >> threadIdx.x) & 1u)) return;
-    const int x = chunk * 32 + threadIdx.x;
-    const uint32_t c = (uint32_t)(row * g.nx + x);
-    bulk_cell<Q, S, true>(fin, fout, g, p, x, y, z, c, diverged);
 }
 
 // Boundary-list entries: fluid cells with a solid neighbour (off the
@@ -921,7 +876,7 @@ __device__ __forceinline__ void boundary_entry(const typename S::T* __restrict__
     if (cls == kCellSolidFill) {  // solid cell: f_i = w_i (LbmReference.cpp:264-267)
         static_for<0, Q>([&](auto I) {
             constexpr int i = decltype(I)::value;
-            store_pop_c<Q, S, i>(fout, g.n, c, L::w(i));
+            store_pop_c<Q, S, i>(fout, g.ps, c, L::w(i));
         });
         return;
     }
@@ -945,13 +900,13 @@ __device__ __forceinline__ void boundary_entry(const typename S::T* __restrict__
             const int py = (int)y - L::ey(i), pz = (int)z - L::ez(i);
             pa = edge_plane<Q, i>(py < 0 || py >= g.ny, pz < 0 || pz >= g.nz, p);
         }
-        const float va = load_plane<Q, S>(fin, pa, g.n, sa, L::w(i));
+        const float va = load_plane<Q, S>(fin, pa, g.ps, sa, L::w(i));
         float v = va;
         if (kind == kLinkBzNear || kind == kLinkBzFar) {
             const float2 k = __ldg(bl.coef + co0 + __popc(bzmask & ((1u << i) - 1u)));
             const int pb = kind == kLinkBzNear ? op : i;
             const size_t sb = kind == kLinkBzNear ? (size_t)c + link_offset<Q>(i, g) : (size_t)c;
-            const float vb = load_plane<Q, S>(fin, pb, g.n, sb, L::w(i));
+            const float vb = load_plane<Q, S>(fin, pb, g.ps, sb, L::w(i));
             v = k.x * va + k.y * vb;
         }
         f[i] = v;
@@ -959,7 +914,7 @@ __device__ __forceinline__ void boundary_entry(const typename S::T* __restrict__
     if (collide<Q, S::kExact>(f, p.tau, p.cs)) atomicOr(diverged, 1);
     static_for<0, Q>([&](auto I) {
         constexpr int i = decltype(I)::value;
-        store_pop_c<Q, S, i>(fout, g.n, c, f[i]);
+        store_pop_c<Q, S, i>(fout, g.ps, c, f[i]);
     });
 }
 
@@ -1016,7 +971,7 @@ __global__ void __launch_bounds__(128) k_boundary_pull_learned(const typename S:
     if (live && !fluid) {  // solid cell: f_i = w_i (LbmReference.cpp:264-267)
         static_for<0, Q>([&](auto I) {
             constexpr int i = decltype(I)::value;
-            store_pop_c<Q, S, i>(fout, g.n, c, L::w(i));
+            store_pop_c<Q, S, i>(fout, g.ps, c, L::w(i));
         });
     }
     const uint32_t nxy = (uint32_t)g.nxy;
@@ -1044,13 +999,13 @@ __global__ void __launch_bounds__(128) k_boundary_pull_learned(const typename S:
                 const int py = (int)y - L::ey(i), pz = (int)z - L::ez(i);
                 pa = edge_plane<Q, i>(py < 0 || py >= g.ny, pz < 0 || pz >= g.nz, p);
             }
-            const float va = load_plane<Q, S>(fin, pa, g.n, sa, L::w(i));
+            const float va = load_plane<Q, S>(fin, pa, g.ps, sa, L::w(i));
             float v = va;
             if (kind == kLinkBzNear || kind == kLinkBzFar) {
                 const float2 kk = __ldg(bl.coef + co0 + __popc(bzmask & ((1u << i) - 1u)));
                 const int pb = kind == kLinkBzNear ? op : i;
                 const size_t sb = kind == kLinkBzNear ? (size_t)c + link_offset<Q>(i, g) : (size_t)c;
-                const float vb = load_plane<Q, S>(fin, pb, g.n, sb, L::w(i));
+                const float vb = load_plane<Q, S>(fin, pb, g.ps, sb, L::w(i));
                 v = kk.x * va + kk.y * vb;
             }
             h[i] = make_float2((v - L::w(i)) * 256.0f, 0.0f);
@@ -1079,7 +1034,7 @@ __global__ void __launch_bounds__(128) k_boundary_pull_learned(const typename S:
     if (bad) atomicOr(diverged, 1);
     static_for<0, Q>([&](auto I) {
         constexpr int i = decltype(I)::value;
-        store_pop_c<Q, S, i>(fout, g.n, c, L::w(i) + h[i].x * (1.0f / 256.0f));
+        store_pop_c<Q, S, i>(fout, g.ps, c, L::w(i) + h[i].x * (1.0f / 256.0f));
     });
 }
 
@@ -1090,8 +1045,8 @@ static PlanePtrs pp_of(const void* fin, void* fout, const Geom& g) {
     for (int i = 0; i < Q; ++i) {
         const long long off = (long long)Lattice<Q>::ex(i) + (long long)Lattice<Q>::ey(i) * g.nx +
                               (long long)Lattice<Q>::ez(i) * g.nxy;
-        pp.src[i] = (const typename S::T*)fin + ((long long)i * (long long)g.n - off);
-        pp.dst[i] = (typename S::T*)fout + (size_t)i * g.n;
+        pp.src[i] = (const typename S::T*)fin + ((long long)i * (long long)g.ps - off);
+        pp.dst[i] = (typename S::T*)fout + (size_t)i * g.ps;
     }
     return pp;
 }
@@ -1103,69 +1058,46 @@ static cudaError_t bulk_t(const void* fin, void* fout, const uint32_t* bits, con
     if (zc <= 0) return cudaSuccess;
     const int z1 = z0 + zc;
     dim3 block(32, kBulkRows, 1);
-    if (g.nx % 2 == 0) {  // pairs start on even cells: every row through k_bulk_pairs
-        PairsShell sh{};
-        if (staged) {  // the interior warps' rows staged in shared memory by TMA
-            int nl = 0;
-            cudaError_t e = launch_bulk_staged(Q, storage_code<S>(), fin, fout, bits, g, p, z0, zc, dv, s, &nl);
-            if (e != cudaSuccess) return e;
-            *launched += nl;
-            sh.gx = (g.nx + 63) / 64;
-            sh.nyb = (g.ny + kBulkRows - 1) / kBulkRows;
-            sh.z0 = z0;
-            sh.zi0 = z0 > 1 ? z0 : 1;
-            const int zi1 = z1 < g.nz - 1 ? z1 : g.nz - 1;
-            sh.nyf = sh.nyb >= 2 ? 2 : 1;
-            sh.nzf = 0;
-            if (z0 <= 0 && 0 < z1) sh.zf[sh.nzf++] = 0;
-            if (g.nz > 1 && z0 <= g.nz - 1 && g.nz - 1 < z1) sh.zf[sh.nzf++] = g.nz - 1;
-            sh.ne = 2ull * sh.nyb * zc;
-            sh.nf = zi1 > sh.zi0 ? (unsigned long long)(sh.gx - 2) * sh.nyf * (zi1 - sh.zi0) : 0ull;
-            const unsigned long long ng = (unsigned long long)(sh.gx - 2) * sh.nyb * sh.nzf;
-            sh.n = sh.ne + sh.nf + ng;
-            if (sh.n == 0) return cudaSuccess;
-            k_bulk_pairs<Q, S><<<(unsigned)sh.n, block, 0, s>>>((const typename S::T*)fin, (typename S::T*)fout, bits, g,
-                                                                p, pp_of<Q, S>(fin, fout, g), z0, dv, sh);
-            ++*launched;
-            return cudaGetLastError();
-        }
-        dim3 grid((unsigned)((g.nx + 63) / 64), (unsigned)((g.ny + kBulkRows - 1) / kBulkRows), (unsigned)zc);
-        k_bulk_pairs<Q, S><<<grid, block, 0, s>>>((const typename S::T*)fin, (typename S::T*)fout, bits, g, p,
-                                                  pp_of<Q, S>(fin, fout, g), z0, dv, sh);
+    const PlanePtrs pp = pp_of<Q, S>(fin, fout, g);
+    PairsShell sh{};
+    if (staged) {  // the interior warps' rows staged in shared memory by TMA (even nx)
+        int nl = 0;
+        cudaError_t e = launch_bulk_staged(Q, storage_code<S>(), fin, fout, bits, g, p, z0, zc, dv, s, &nl);
+        if (e != cudaSuccess) return e;
+        *launched += nl;
+        sh.gx = (g.nx + 63) / 64;
+        sh.nyb = (g.ny + kBulkRows - 1) / kBulkRows;
+        sh.z0 = z0;
+        sh.zi0 = z0 > 1 ? z0 : 1;
+        const int zi1 = z1 < g.nz - 1 ? z1 : g.nz - 1;
+        sh.nyf = sh.nyb >= 2 ? 2 : 1;
+        sh.nzf = 0;
+        if (z0 <= 0 && 0 < z1) sh.zf[sh.nzf++] = 0;
+        if (g.nz > 1 && z0 <= g.nz - 1 && g.nz - 1 < z1) sh.zf[sh.nzf++] = g.nz - 1;
+        sh.ne = 2ull * sh.nyb * zc;
+        sh.nf = zi1 > sh.zi0 ? (unsigned long long)(sh.gx - 2) * sh.nyf * (zi1 - sh.zi0) : 0ull;
+        const unsigned long long ng = (unsigned long long)(sh.gx - 2) * sh.nyb * sh.nzf;
+        sh.n = sh.ne + sh.nf + ng;
+        if (sh.n == 0) return cudaSuccess;
+        k_bulk_pairs<Q, S, kNxEven><<<(unsigned)sh.n, block, 0, s>>>((const typename S::T*)fin, (typename S::T*)fout,
+                                                                     bits, g, p, pp, z0, dv, sh);
         ++*launched;
         return cudaGetLastError();
     }
-    // odd nx: one-cell interior kernel + shell kernel (planes ride in the shell's row-end warps)
-    const int zi0 = z0 > 1 ? z0 : 1, zi1 = z1 < g.nz - 1 ? z1 : g.nz - 1;
-    if (g.wpr > 2 && g.ny > 2 && zi1 > zi0) {
-        const unsigned gy = (unsigned)((g.ny - 2 + kBulkRows - 1) / kBulkRows);
-        dim3 grid((unsigned)(g.wpr - 2), gy, (unsigned)(zi1 - zi0));
-        k_bulk_interior<Q, S><<<grid, block, 0, s>>>((const typename S::T*)fin, (typename S::T*)fout, bits, g, p, zi0,
-                                                     dv);
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
-        ++*launched;
-    }
-    ShellPlan sp{};
-    sp.z0 = z0;
-    sp.nyf = 0;
-    sp.yf[sp.nyf++] = 0;
-    if (g.ny > 1) sp.yf[sp.nyf++] = g.ny - 1;
-    sp.nyi = g.ny > 2 ? g.ny - 2 : 0;
-    sp.nzf = 0;
-    if (z0 <= 0 && 0 < z1) sp.zf[sp.nzf++] = 0;
-    if (g.nz > 1 && z0 <= g.nz - 1 && g.nz - 1 < z1) sp.zf[sp.nzf++] = g.nz - 1;
-    sp.zi0 = zi0;
-    sp.ncend = 0;
-    sp.cend[sp.ncend++] = 0;
-    if (g.wpr > 1) sp.cend[sp.ncend++] = g.wpr - 1;
-    sp.n_a = (unsigned long long)sp.nyf * zc * g.wpr;
-    sp.n_b = (unsigned long long)sp.nzf * sp.nyi * g.wpr;
-    sp.n_c = zi1 > zi0 ? (unsigned long long)(zi1 - zi0) * sp.nyi * sp.ncend : 0ull;
-    const unsigned long long items = sp.n_a + sp.n_b + sp.n_c;
-    if (items == 0) return cudaSuccess;
-    const unsigned blocks = (unsigned)((items + kBulkRows - 1) / kBulkRows);
-    k_bulk_shell<Q, S><<<blocks, block, 0, s>>>((const typename S::T*)fin, (typename S::T*)fout, bits, g, p, sp, dv);
+    // odd nx: one cell more, for the rows shifted to the left
+    const int par = pair_parity(g);
+    dim3 grid((unsigned)((g.nx + (par == kNxEven ? 0 : 1) + 63) / 64),
+              (unsigned)((g.ny + kBulkRows - 1) / kBulkRows), (unsigned)zc);
+    auto launch = [&](auto P) {
+        k_bulk_pairs<Q, S, decltype(P)::value><<<grid, block, 0, s>>>((const typename S::T*)fin,
+                                                                     (typename S::T*)fout, bits, g, p, pp, z0, dv, sh);
+    };
+    if (par == kNxEven)
+        launch(std::integral_constant<int, kNxEven>{});
+    else if (par == kNxOddNyOdd)
+        launch(std::integral_constant<int, kNxOddNyOdd>{});
+    else
+        launch(std::integral_constant<int, kNxOddNyEven>{});
     ++*launched;
     return cudaGetLastError();
 }
@@ -1195,8 +1127,8 @@ static cudaError_t bulk_learned_t(const void* fin, void* fout, const uint32_t* b
         for (int i = 0; i < Q; ++i) {
             const long long off = (long long)Lattice<Q>::ex(i) + (long long)Lattice<Q>::ey(i) * g.nx +
                                   (long long)Lattice<Q>::ez(i) * g.nxy;
-            pp.src[i] = (const typename S::T*)fin + ((long long)i * (long long)g.n - off);
-            pp.dst[i] = (typename S::T*)fout + (size_t)i * g.n;
+            pp.src[i] = (const typename S::T*)fin + ((long long)i * (long long)g.ps - off);
+            pp.dst[i] = (typename S::T*)fout + (size_t)i * g.ps;
         }
         dim3 block(32, kBulkRows, 1);
         dim3 grid((unsigned)((g.nx + 63) / 64), (unsigned)((g.ny + kBulkRows - 1) / kBulkRows), (unsigned)zc);

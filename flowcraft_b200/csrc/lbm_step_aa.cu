@@ -100,9 +100,9 @@ __device__ __forceinline__ size_t out_slot(uint32_t c, int x, int y, int z, cons
     if constexpr (Odd) {
         const int tx = x + L::ex(I), ty = y + L::ey(I), tz = z + L::ez(I);
         if (tx >= 0 && ty >= 0 && tz >= 0 && tx < g.nx && ty < g.ny && tz < g.nz)
-            return (size_t)I * g.n + (size_t)((long long)c + link_offset<Q>(I, g));
+            return (size_t)I * g.ps + (size_t)((long long)c + link_offset<Q>(I, g));
     }
-    return (size_t)L::opp(I) * g.n + c;
+    return (size_t)L::opp(I) * g.ps + c;
 }
 
 // One interior bulk cell (the one-cell path of k_bulk_pairs).
@@ -113,15 +113,15 @@ __device__ __forceinline__ void aa_interior_cell(typename S::T* f, const Geom& g
     float v[Q];
     static_for<0, Q>([&](auto I) {
         constexpr int i = decltype(I)::value;
-        const size_t s = Odd ? (size_t)L::opp(i) * g.n + (size_t)((long long)c - link_offset<Q>(i, g))
-                             : (size_t)i * g.n + c;
+        const size_t s = Odd ? (size_t)L::opp(i) * g.ps + (size_t)((long long)c - link_offset<Q>(i, g))
+                             : (size_t)i * g.ps + c;
         v[i] = S::dec(ld_plain<S>(f + s), L::w(i));
     });
     if (collide<Q, S::kExact>(v, p.tau, p.cs)) atomicOr(diverged, 1);
     static_for<0, Q>([&](auto I) {
         constexpr int i = decltype(I)::value;
-        const size_t d = Odd ? (size_t)i * g.n + (size_t)((long long)c + link_offset<Q>(i, g))
-                             : (size_t)L::opp(i) * g.n + c;
+        const size_t d = Odd ? (size_t)i * g.ps + (size_t)((long long)c + link_offset<Q>(i, g))
+                             : (size_t)L::opp(i) * g.ps + c;
         f[d] = S::enc(v[i], L::w(i));
     });
 }
@@ -170,12 +170,12 @@ __device__ __forceinline__ void aa_row_end_cell(typename S::T* f, const Geom& g,
     }
     // the slot out_slot<Q, i, Odd> names, for the run-time direction
     const unsigned opp = i == 0 ? 0u : ((i - 1u) ^ 1u) + 1u;
-    size_t slot = (size_t)opp * g.n + pc;
+    size_t slot = (size_t)opp * g.ps + pc;
     if constexpr (Odd) {
         const int ex = (int)lattice_e_rt<Q, 0>(i), ey = (int)lattice_e_rt<Q, 1>(i), ez = (int)lattice_e_rt<Q, 2>(i);
         const int tx = px + ex, ty = y + ey, tz = z + ez;
         if (tx >= 0 && ty >= 0 && tz >= 0 && tx < g.nx && ty < g.ny && tz < g.nz)
-            slot = (size_t)i * g.n + (size_t)((long long)pc + ex + (long long)ey * g.nx + (long long)ez * g.nxy);
+            slot = (size_t)i * g.ps + (size_t)((long long)pc + ex + (long long)ey * g.nx + (long long)ez * g.nxy);
     }
     if (mine) f[slot] = S::enc(v, lattice_w_rt<Q>(i));
 }
@@ -329,7 +329,7 @@ __global__ void __launch_bounds__(32 * kBulkRows, 4) k_bulk_pairs_aa(typename S:
         const uint32_t off = (out || !Odd) ? 0u : (uint32_t)link_offset<Q>(i, g);
         const uint32_t sa = va ? c - off : c;
         const uint32_t sb = vb ? c + 1u - off : c + 1u;
-        const T* base = f + (size_t)rplane * g.n;
+        const T* base = f + (size_t)rplane * g.ps;
         const T ha = ld_plain<S>(base + sa), hb = ld_plain<S>(base + sb);
         if constexpr (S::kExact)
             v[i] = make_float2(S::dec(ha, L::w(i)), S::dec(hb, L::w(i)));
@@ -349,8 +349,8 @@ __global__ void __launch_bounds__(32 * kBulkRows, 4) k_bulk_pairs_aa(typename S:
         const int ty = y + L::ey(i), tz = z + L::ez(i);
         const bool inside = ty >= 0 && ty < g.ny && tz >= 0 && tz < g.nz;
         const bool push = Odd && inside;
-        T* dst = f + (push ? (size_t)i * g.n + (size_t)((long long)c + link_offset<Q>(i, g))
-                           : (size_t)L::opp(i) * g.n + c);
+        T* dst = f + (push ? (size_t)i * g.ps + (size_t)((long long)c + link_offset<Q>(i, g))
+                           : (size_t)L::opp(i) * g.ps + c);
         if (pair == 3u && (!push || L::ex(i) == 0)) {
             *reinterpret_cast<T2*>(dst) = h;
         } else {
@@ -416,13 +416,13 @@ __global__ void __launch_bounds__(128) k_boundary_aa(typename S::T* f, BoundaryL
         const size_t off = (size_t)link_offset<Q>(i, g);
         size_t sa;
         if (kind == kLinkStream) {  // f*_i(c - e_i)
-            sa = Odd ? (size_t)op * g.n + (c - off) : (size_t)i * g.n + c;
+            sa = Odd ? (size_t)op * g.ps + (c - off) : (size_t)i * g.ps + c;
         } else if (kind == kLinkEdge) {  // f*_m(c) for the mirrored / bounced m
             const int py = y - L::ey(i), pz = z - L::ez(i);
             const int m = edge_plane<Q, i>(py < 0 || py >= g.ny, pz < 0 || pz >= g.nz, p);
-            sa = (size_t)L::opp(m) * g.n + c;
+            sa = (size_t)L::opp(m) * g.ps + c;
         } else {  // f*_op(c); before an even step it sits in the solid neighbour c - e_i
-            sa = Odd ? (size_t)i * g.n + c : (size_t)op * g.n + (c - off);
+            sa = Odd ? (size_t)i * g.ps + c : (size_t)op * g.ps + (c - off);
         }
         const float va = S::dec(ld_plain<S>(f + sa), L::w(i));
         float r = va;
@@ -431,7 +431,7 @@ __global__ void __launch_bounds__(128) k_boundary_aa(typename S::T* f, BoundaryL
             const float2 kc = __ldg(bl.coef + slot);
             float vb;
             if (kind == kLinkBzNear) {  // f*_op(c + e_i)
-                const size_t sb = Odd ? (size_t)i * g.n + (c + off) : (size_t)op * g.n + c;
+                const size_t sb = Odd ? (size_t)i * g.ps + (c + off) : (size_t)op * g.ps + c;
                 vb = S::dec(ld_plain<S>(f + sb), L::w(i));
             } else {  // f*_i(c), kept from the previous step
                 vb = S::dec(bz[slot], L::w(i));
@@ -484,8 +484,8 @@ __device__ __forceinline__ void aa_store_pair(typename S::T* f, const PlanePtrs&
         const int ty = y + L::ey(i), tz = z + L::ez(i);
         const bool inside = ty >= 0 && ty < g.ny && tz >= 0 && tz < g.nz;
         const bool push = Odd && inside;
-        T* dst = f + (push ? (size_t)i * g.n + (size_t)((long long)c + link_offset<Q>(i, g))
-                           : (size_t)L::opp(i) * g.n + c);
+        T* dst = f + (push ? (size_t)i * g.ps + (size_t)((long long)c + link_offset<Q>(i, g))
+                           : (size_t)L::opp(i) * g.ps + c);
         if (pair == 3u && (!push || L::ex(i) == 0)) {
             *reinterpret_cast<T2*>(dst) = h;
         } else {
@@ -570,7 +570,7 @@ __global__ void __launch_bounds__(32 * kBulkRows, 4) k_bulk_pairs_aa_learned(typ
             const uint32_t off = (out || !Odd) ? 0u : (uint32_t)link_offset<Q>(i, g);
             const uint32_t sa = va ? c - off : cs;
             const uint32_t sb = vb ? c + 1u - off : cs + 1u;
-            const T* base = f + (size_t)rplane * g.n;
+            const T* base = f + (size_t)rplane * g.ps;
             v[i] = make_float2(S::raw(ld_plain<S>(base + sa)), S::raw(ld_plain<S>(base + sb)));
         });
     }
@@ -682,13 +682,13 @@ __global__ void __launch_bounds__(128) k_boundary_aa_learned(typename S::T* f, B
             const size_t off = (size_t)link_offset<Q>(i, g);
             size_t sa;
             if (kind == kLinkStream) {  // f*_i(c - e_i)
-                sa = Odd ? (size_t)op * g.n + (c - off) : (size_t)i * g.n + c;
+                sa = Odd ? (size_t)op * g.ps + (c - off) : (size_t)i * g.ps + c;
             } else if (kind == kLinkEdge) {  // f*_m(c) for the mirrored / bounced m
                 const int py = y - L::ey(i), pz = z - L::ez(i);
                 const int m = edge_plane<Q, i>(py < 0 || py >= g.ny, pz < 0 || pz >= g.nz, p);
-                sa = (size_t)L::opp(m) * g.n + c;
+                sa = (size_t)L::opp(m) * g.ps + c;
             } else {  // f*_op(c); before an even step it sits in the solid neighbour c - e_i
-                sa = Odd ? (size_t)i * g.n + c : (size_t)op * g.n + (c - off);
+                sa = Odd ? (size_t)i * g.ps + c : (size_t)op * g.ps + (c - off);
             }
             const float va = S::dec(ld_plain<S>(f + sa), L::w(i));
             float r = va;
@@ -697,7 +697,7 @@ __global__ void __launch_bounds__(128) k_boundary_aa_learned(typename S::T* f, B
                 const float2 kc = __ldg(bl.coef + slot);
                 float vb;
                 if (kind == kLinkBzNear) {  // f*_op(c + e_i)
-                    const size_t sb = Odd ? (size_t)i * g.n + (c + off) : (size_t)op * g.n + c;
+                    const size_t sb = Odd ? (size_t)i * g.ps + (c + off) : (size_t)op * g.ps + c;
                     vb = S::dec(ld_plain<S>(f + sb), L::w(i));
                 } else {  // f*_i(c), kept from the previous step
                     vb = S::dec(bz[slot], L::w(i));
@@ -799,7 +799,7 @@ static cudaError_t bulk_aa_t(void* f, const uint32_t* bits, const Geom& g, const
     for (int i = 0; i < Q; ++i) {
         const long long off = (long long)Lattice<Q>::ex(i) + (long long)Lattice<Q>::ey(i) * g.nx +
                               (long long)Lattice<Q>::ez(i) * g.nxy;
-        const long long pi = (long long)i * (long long)g.n, po = (long long)Lattice<Q>::opp(i) * (long long)g.n;
+        const long long pi = (long long)i * (long long)g.ps, po = (long long)Lattice<Q>::opp(i) * (long long)g.ps;
         pp.src[i] = base + (odd ? po - off : pi);
         pp.dst[i] = base + (odd ? pi + off : po);
     }
@@ -842,7 +842,7 @@ static cudaError_t bulk_aa_learned_t(void* f, const uint32_t* bits, const Geom& 
         for (int i = 0; i < Q; ++i) {
             const long long off = (long long)Lattice<Q>::ex(i) + (long long)Lattice<Q>::ey(i) * g.nx +
                                   (long long)Lattice<Q>::ez(i) * g.nxy;
-            const long long pi = (long long)i * (long long)g.n, po = (long long)Lattice<Q>::opp(i) * (long long)g.n;
+            const long long pi = (long long)i * (long long)g.ps, po = (long long)Lattice<Q>::opp(i) * (long long)g.ps;
             pp.src[i] = base + (odd ? po - off : pi);
             pp.dst[i] = base + (odd ? pi + off : po);
         }

@@ -283,7 +283,7 @@ __global__ void __launch_bounds__(kTileThreads, kTileBlocksPerSm) k_bulk_tiles(c
                 if (collide<Q, S::kExact>(f, p.tau, p.cs)) atomicOr(diverged, 1);
                 static_for<0, Q>([&](auto I) {
                     constexpr int i = decltype(I)::value;
-                    store_pop_i<Q, S, i>(fout, g.n, c + (uint32_t)b, f[i]);
+                    store_pop_i<Q, S, i>(fout, g.ps, c + (uint32_t)b, f[i]);
                 });
             }
         }
@@ -347,7 +347,7 @@ static cudaError_t tiles_t(const void* fin, void* fout, const uint32_t* bits, co
         PlanePtrs pp{};
         for (int i = 0; i < Q; ++i) {
             pp.src[i] = nullptr;
-            pp.dst[i] = (typename S::T*)fout + (size_t)i * g.n;
+            pp.dst[i] = (typename S::T*)fout + (size_t)i * g.ps;
         }
         // per instantiation and device: the shared-memory opt-in and the grid
         constexpr int kMaxDev = 64;
