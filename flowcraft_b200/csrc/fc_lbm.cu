@@ -387,36 +387,23 @@ int guard_snapshot(fc_lbm* h, cudaStream_t s, int set) {
     return FC_LBM_OK;
 }
 
-// The two step kernels, with or without the learned closure, ping-pong or in place.
-cudaError_t launch_bulk(fc_lbm* h, const fc::StepParams& p, const void* fin, void* fout, int z0, int zc,
-                        cudaStream_t s, int* nl) {
+// One step of the bulk cells of layers [z0, z0 + zc) and the boundary-list
+// entries [b, e), with or without the learned closure, ping-pong or in place.
+cudaError_t launch_step(fc_lbm* h, const fc::StepParams& p, const void* fin, void* fout, int z0, int zc, uint32_t b,
+                        uint32_t e, cudaStream_t s, int* nl) {
+    const fc::BoundarySpan bnd{boundary_list(h), b, e, 0};
     if (in_place(h) && h->closure_on)
         return fc::launch_bulk_aa_learned(h->q, h->storage, h->pop[0], h->d_bulk_bits, h->g, p, z0, zc,
-                                          h->d_diverged, s, nl, h->cur, aa_side(h), h->closure);
+                                          h->d_diverged, s, nl, h->cur, aa_side(h), h->closure, bnd);
     if (in_place(h))
         return fc::launch_bulk_aa(h->q, h->storage, h->pop[0], h->d_bulk_bits, h->g, p, z0, zc, h->d_diverged, s, nl,
-                                  h->cur, aa_side(h));
+                                  h->cur, aa_side(h), bnd);
     if (h->closure_on)
         return fc::launch_bulk_pull_learned(h->q, h->storage, fin, fout, h->d_bulk_bits, h->g, p, z0, zc,
-                                            h->d_diverged, s, nl, h->closure,
+                                            h->d_diverged, s, nl, h->closure, bnd,
                                             (h->flags & FC_OPTION_TC_CLOSURE) ? 1 : 0);
     return fc::launch_bulk_pull(h->q, h->storage, fin, fout, h->d_bulk_bits, h->g, p, z0, zc, h->d_diverged, s, nl,
-                                (h->flags & FC_OPTION_TMA_STAGING) ? 1 : 0);
-}
-
-cudaError_t launch_boundary(fc_lbm* h, const fc::StepParams& p, const void* fin, void* fout, uint32_t b, uint32_t e,
-                            cudaStream_t s) {
-    const fc::BoundaryList bl = boundary_list(h);
-    if (in_place(h) && h->closure_on)
-        return fc::launch_boundary_aa_learned(h->q, h->storage, h->pop[0], bl, b, e, h->g, p, h->d_diverged, s,
-                                              h->cur, aa_side(h), h->closure);
-    if (in_place(h))
-        return fc::launch_boundary_aa(h->q, h->storage, h->pop[0], bl, b, e, h->g, p, h->d_diverged, s, h->cur,
-                                      aa_side(h));
-    if (h->closure_on)
-        return fc::launch_boundary_pull_learned(h->q, h->storage, fin, fout, bl, b, e, h->g, p, h->d_diverged, s,
-                                                h->closure);
-    return fc::launch_boundary_pull(h->q, h->storage, fin, fout, bl, b, e, h->g, p, h->d_diverged, s);
+                                bnd, (h->flags & FC_OPTION_TMA_STAGING) ? 1 : 0);
 }
 
 int step_range_on(fc_lbm* h, cudaStream_t s, int z0, int zc) {
@@ -427,16 +414,11 @@ int step_range_on(fc_lbm* h, cudaStream_t s, int z0, int zc) {
     const void* fin = h->pop[h->cur];
     void* fout = h->pop[1 - h->cur];
     FC_RC(guard_snapshot(h, s, 1 - h->cur));
-    if (h->n_bulk > 0) {
-        int nl = 0;
-        FC_TRY(h, launch_bulk(h, p, fin, fout, z0, z1 - z0, s, &nl), "bulk step");
-        h->launches += nl;
-    }
-    const uint32_t b = h->z_begin[(size_t)z0], e = h->z_begin[(size_t)z1];
-    if (e > b) {
-        FC_TRY(h, launch_boundary(h, p, fin, fout, b, e, s), "boundary step");
-        h->launches++;
-    }
+    int nl = 0;
+    FC_TRY(h, launch_step(h, p, fin, fout, z0, h->n_bulk > 0 ? z1 - z0 : 0, h->z_begin[(size_t)z0],
+                          h->z_begin[(size_t)z1], s, &nl),
+           "step");
+    h->launches += nl;
     return FC_LBM_OK;
 }
 
@@ -1105,14 +1087,15 @@ int fc_lbm_step_timed(fc_lbm* h, int32_t n, float* total_ms, float* bulk_ms, flo
         cudaError_t ce = cudaSuccess;
         if (h->n_bulk > 0) {
             int nl = 0;
-            ce = launch_bulk(h, p, fin, fout, 0, h->g.nz, h->stream, &nl);
+            ce = launch_step(h, p, fin, fout, 0, h->g.nz, 0, 0, h->stream, &nl);
             h->launches += nl;
         }
         cudaEventRecord(ev[3 + 4 * k], h->stream);
         cudaEventRecord(ev[4 + 4 * k], h->stream);
         if (ce == cudaSuccess && e > b) {
-            ce = launch_boundary(h, p, fin, fout, b, e, h->stream);
-            h->launches++;
+            int nl = 0;
+            ce = launch_step(h, p, fin, fout, 0, 0, b, e, h->stream, &nl);
+            h->launches += nl;
         }
         cudaEventRecord(ev[5 + 4 * k], h->stream);
         if (ce != cudaSuccess) rc = cuda_fail(h, ce, "timed step");
@@ -1543,7 +1526,7 @@ int batch_bulk_members(fc_lbm_batch* b, int parity) {
         if (h->n_bulk == 0) continue;
         const int side = h->cur ^ parity;
         int nl = 0;
-        e = launch_bulk(h, step_params(h), h->pop[side], h->pop[1 - side], 0, h->g.nz, b->fork[k % nf], &nl);
+        e = launch_step(h, step_params(h), h->pop[side], h->pop[1 - side], 0, h->g.nz, 0, 0, b->fork[k % nf], &nl);
     }
     if (e == cudaSuccess)
         e = fc::launch_boundary_batch(b->q, b->storage, b->d_lat, (int)b->m.size(), b->btotal, parity, b->stream);

@@ -72,10 +72,25 @@ struct BoundaryList {
     const float2* coef;
 };
 
+// The boundary-list entries [begin, end) that a step kernel updates beside
+// its bulk cells. The launch's first `slabs` z slabs of blocks take them, one
+// entry per thread: an entry is a long chain of dependent loads, so its
+// blocks start first and run under the bulk blocks instead of after them.
+// Against a kernel of their own behind the bulk kernel (10-25 us per step on a
+// B200): 48x24x24 FP32, 20 steps and a field, 562 -> 381 us; 256x128x128 FP32
+// with smoke, 20 frames of 2 steps, 7.31 -> 6.63 ms; 384x192x192 with the
+// learned closure, 50 steps, 24.85 -> 24.26 ms; no change at 268M cells.
+struct BoundarySpan {
+    BoundaryList list;
+    uint32_t begin, end;
+    unsigned slabs;  // set by the launcher
+};
+
 // ---- launchers (defined in the .cu files) ----
 // storage: 0 fp32, 1 fp16 offset, 2 bf16 offset; q: 15 or 19.
-// Bulk cells of z range [z0, z0+zc). *launched receives the number of kernels
-// enqueued.
+// The step launchers (launch_bulk_*) update the bulk cells of z range [z0,
+// z0+zc) and the boundary-list entries of `bnd`, in one kernel (either part
+// may be empty); *launched receives the number of kernels enqueued.
 // Learned closure (closure.cuh): fragment-ordered weights, the per-cell wall
 // distance and the input normalization, passed to the kernels by value.
 constexpr int kClosureIn = 5;
@@ -133,7 +148,8 @@ int closure_samples(int q, int storage, const void* f, const uint8_t* solid, con
 // instead of the warp-level mma.sync MLP.
 cudaError_t launch_bulk_pull_learned(int q, int storage, const void* fin, void* fout, const uint32_t* bulk_bits,
                                      const Geom& g, const StepParams& p, int z0, int zc, int* diverged,
-                                     cudaStream_t s, int* launched, const ClosureDev& cl, int tc = 0);
+                                     cudaStream_t s, int* launched, const ClosureDev& cl, const BoundarySpan& bnd,
+                                     int tc = 0);
 cudaError_t launch_closure_probe(int q, int storage, const void* f, const uint8_t* solid, const Geom& g,
                                  const ClosureDev& cl, float* out, uint8_t* in_range, unsigned long long* counts,
                                  int layout, cudaStream_t s);
@@ -205,20 +221,15 @@ struct AaSide {
     float4* outm;
     size_t rows;
 };
-// One in-place step's bulk and boundary kernels; `odd` is the step's parity
+// One in-place step's kernel; `odd` is the step's parity
 // (0: reads the kLayoutAAEven state, 1: kLayoutAAOdd). Even nx >= 4 only.
 cudaError_t launch_bulk_aa(int q, int storage, void* f, const uint32_t* bulk_bits, const Geom& g, const StepParams& p,
-                           int z0, int zc, int* diverged, cudaStream_t s, int* launched, int odd, const AaSide& sd);
-cudaError_t launch_boundary_aa(int q, int storage, void* f, const BoundaryList& bl, uint32_t begin, uint32_t end,
-                               const Geom& g, const StepParams& p, int* diverged, cudaStream_t s, int odd,
-                               const AaSide& sd);
+                           int z0, int zc, int* diverged, cudaStream_t s, int* launched, int odd, const AaSide& sd,
+                           const BoundarySpan& bnd);
 // The same with the learned closure (16-bit offset formats).
 cudaError_t launch_bulk_aa_learned(int q, int storage, void* f, const uint32_t* bulk_bits, const Geom& g,
                                    const StepParams& p, int z0, int zc, int* diverged, cudaStream_t s, int* launched,
-                                   int odd, const AaSide& sd, const ClosureDev& cl);
-cudaError_t launch_boundary_aa_learned(int q, int storage, void* f, const BoundaryList& bl, uint32_t begin,
-                                       uint32_t end, const Geom& g, const StepParams& p, int* diverged,
-                                       cudaStream_t s, int odd, const AaSide& sd, const ClosureDev& cl);
+                                   int odd, const AaSide& sd, const ClosureDev& cl, const BoundarySpan& bnd);
 // Fills the side buffers from the state a step of parity `par` reads (after a
 // seed or a population load); `count` = boundary-list length.
 cudaError_t launch_aa_prime(int q, int storage, const void* f, const BoundaryList& bl, uint32_t count, const Geom& g,
@@ -229,7 +240,7 @@ cudaError_t launch_aa_prime(int q, int storage, const void* f, const BoundaryLis
 // (staged_eligible), the rest through k_bulk_pairs.
 cudaError_t launch_bulk_pull(int q, int storage, const void* fin, void* fout, const uint32_t* bulk_bits,
                              const Geom& g, const StepParams& p, int z0, int zc, int* diverged, cudaStream_t s,
-                             int* launched, int staged = 0);
+                             int* launched, const BoundarySpan& bnd, int staged = 0);
 // The interior rows only (lbm_step_staged.cu): rows off the Y/Z faces,
 // 64-cell chunks off the row ends.
 cudaError_t launch_bulk_staged(int q, int storage, const void* fin, void* fout, const uint32_t* bulk_bits,
@@ -237,12 +248,6 @@ cudaError_t launch_bulk_staged(int q, int storage, const void* fin, void* fout, 
                                int* launched);
 // nx a multiple of 16 bytes' worth of elements, nx > 128, ny, nz >= 3.
 bool staged_eligible(int storage, const Geom& g);
-cudaError_t launch_boundary_pull_learned(int q, int storage, const void* fin, void* fout, const BoundaryList& bl,
-                                         uint32_t begin, uint32_t end, const Geom& g, const StepParams& p,
-                                         int* diverged, cudaStream_t s, const ClosureDev& cl);
-cudaError_t launch_boundary_pull(int q, int storage, const void* fin, void* fout, const BoundaryList& bl,
-                                 uint32_t begin, uint32_t end, const Geom& g, const StepParams& p, int* diverged,
-                                 cudaStream_t s);
 
 // `layout` (every launcher that reads or writes a whole state): where the
 // populations sit between steps, a PopLayout of aa.cuh: 0 plane-major

@@ -1,9 +1,9 @@
 // The LBM step on B200: one fused pull-stream + boundary + regularized
 // collision update per cell (FlowCraft/LbmReference.cpp:241-469, the GPU
-// twin shaders/lbm_step.comp.glsl:98-364), split into two kernels so the
-// kernel that touches >99% of the cells never branches on geometry:
+// twin shaders/lbm_step.comp.glsl:98-364), split into two parts so the part
+// that touches >99% of the cells never branches on geometry:
 //
-//   k_bulk_pairs     two x-adjacent cells per thread; a warp covers 64 cells of
+//   pairs_tile       two x-adjacent cells per thread; a warp covers 64 cells of
 //                    one row, reads their bits of the bit-packed bulk mask,
 //                    gathers Q populations per cell from the upstream
 //                    neighbours (aligned 2-element loads where a direction's
@@ -11,14 +11,15 @@
 //                    Q pairs. Boundary and solid cells are masked out. Warps
 //                    on a Y/Z face take mirror / bounce-back sources, warps at
 //                    a row end also update the inlet / outlet cell.
-//   k_boundary_pull  one thread per entry of the compacted boundary list:
+//   boundary_entry   one thread per entry of the compacted boundary list:
 //                    fluid cells with a solid neighbour (halfway or Bouzidi
 //                    links) and the solid cells an outlet may read. Link kinds and
 //                    Bouzidi coefficients were precomputed at init from the
 //                    solid mask and SDF with the reference's float operations.
 //
-// Both kernels read one population set and write the other (ping-pong), so
-// they are independent and touch disjoint cells.
+// Both read one population set and write the other (ping-pong), so they are
+// independent and touch disjoint cells: one kernel runs both, the entries in
+// its first blocks (BoundarySpan).
 #include "aa.cuh"
 #include "closure.cuh"
 #include "closure_tc.cuh"
@@ -226,6 +227,155 @@ __device__ __forceinline__ void store_pair(const PlanePtrs& pp, uint32_t c, cons
     }
 }
 
+// Boundary-list entries: fluid cells with a solid neighbour (off the
+// inlet/outlet planes) and the solid cells an outlet reads. Every link's source
+// address is formed with selects first and all loads issue together.
+template <int Q, class S>
+__device__ __forceinline__ void boundary_entry(const typename S::T* __restrict__ fin,
+                                               typename S::T* __restrict__ fout, const BoundaryList& bl, uint32_t e,
+                                               const Geom& g, const StepParams& p, int* __restrict__ diverged) {
+    using L = Lattice<Q>;
+    const uint32_t c = __ldg(bl.cells + e);
+    const unsigned long long lk = __ldg(bl.links + e);
+    const unsigned cls = (unsigned)(lk >> kClassShift) & 7u;
+    const uint32_t nxy = (uint32_t)g.nxy;
+    const uint32_t z = c / nxy;
+    const uint32_t rem = c - z * nxy;
+    const uint32_t y = rem / (uint32_t)g.nx;
+
+    float f[Q];
+    if (cls == kCellSolidFill) {  // solid cell: f_i = w_i (LbmReference.cpp:264-267)
+        static_for<0, Q>([&](auto I) {
+            constexpr int i = decltype(I)::value;
+            store_pop_c<Q, S, i>(fout, g.ps, c, L::w(i));
+        });
+        return;
+    }
+    // Fluid cell next to a wall (LbmReference.cpp:329-383).
+    const uint32_t co0 = __ldg(bl.coef_off + e);
+    uint32_t bzmask = 0;  // directions that carry a Bouzidi coefficient pair
+    static_for<0, Q>([&](auto I) {
+        constexpr int i = decltype(I)::value;
+        if ((((unsigned)(lk >> (3 * i))) & 6u) == 2u) bzmask |= 1u << i;
+    });
+    static_for<0, Q>([&](auto I) {
+        constexpr int i = decltype(I)::value;
+        constexpr int op = L::opp(i);
+        const unsigned kind = (unsigned)(lk >> (3 * i)) & 7u;
+        int pa = op;
+        size_t sa = c;
+        if (kind == kLinkStream) {
+            pa = i;
+            sa = (size_t)c - link_offset<Q>(i, g);
+        } else if (kind == kLinkEdge) {
+            const int py = (int)y - L::ey(i), pz = (int)z - L::ez(i);
+            pa = edge_plane<Q, i>(py < 0 || py >= g.ny, pz < 0 || pz >= g.nz, p);
+        }
+        const float va = load_plane<Q, S>(fin, pa, g.ps, sa, L::w(i));
+        float v = va;
+        if (kind == kLinkBzNear || kind == kLinkBzFar) {
+            const float2 k = __ldg(bl.coef + co0 + __popc(bzmask & ((1u << i) - 1u)));
+            const int pb = kind == kLinkBzNear ? op : i;
+            const size_t sb = kind == kLinkBzNear ? (size_t)c + link_offset<Q>(i, g) : (size_t)c;
+            const float vb = load_plane<Q, S>(fin, pb, g.ps, sb, L::w(i));
+            v = k.x * va + k.y * vb;
+        }
+        f[i] = v;
+    });
+    if (collide<Q, S::kExact>(f, p.tau, p.cs)) atomicOr(diverged, 1);
+    static_for<0, Q>([&](auto I) {
+        constexpr int i = decltype(I)::value;
+        store_pop_c<Q, S, i>(fout, g.ps, c, f[i]);
+    });
+}
+
+// boundary_entry with the learned closure (16-bit offset storage): the same
+// link handling in float populations, then the two-phase collision on
+// offsets (f - w) * 2^8 with the warp-wide closure. Every lane of a warp runs
+// the closure (e == end: no entry); only live fluid entries store. `in` and
+// `out` are the warp's closure buffers.
+template <int Q, class S>
+__device__ __forceinline__ void boundary_entry_learned(const typename S::T* __restrict__ fin,
+                                                       typename S::T* __restrict__ fout, const BoundaryList& bl,
+                                                       uint32_t e, uint32_t end, const Geom& g, const StepParams& p,
+                                                       int* __restrict__ diverged, const ClosureDev& cl,
+                                                       uint32_t* s_in, float2* s_out) {
+    static_assert(!S::kExact, "the learned closure runs on the 16-bit offset formats");
+    using L = Lattice<Q>;
+    const bool live = e < end;
+    const uint32_t c = live ? __ldg(bl.cells + e) : 0u;
+    const unsigned long long lk = live ? __ldg(bl.links + e) : 0ull;
+    const unsigned cls = (unsigned)(lk >> kClassShift) & 7u;
+    const bool fluid = live && cls != kCellSolidFill;
+    if (live && !fluid) {  // solid cell: f_i = w_i (LbmReference.cpp:264-267)
+        static_for<0, Q>([&](auto I) {
+            constexpr int i = decltype(I)::value;
+            store_pop_c<Q, S, i>(fout, g.ps, c, L::w(i));
+        });
+    }
+    const uint32_t nxy = (uint32_t)g.nxy;
+    const uint32_t z = c / nxy;
+    const uint32_t rem = c - z * nxy;
+    const uint32_t y = rem / (uint32_t)g.nx;
+    float2 h[Q];
+    if (fluid) {
+        const uint32_t co0 = __ldg(bl.coef_off + e);
+        uint32_t bzmask = 0;
+        static_for<0, Q>([&](auto I) {
+            constexpr int i = decltype(I)::value;
+            if ((((unsigned)(lk >> (3 * i))) & 6u) == 2u) bzmask |= 1u << i;
+        });
+        static_for<0, Q>([&](auto I) {
+            constexpr int i = decltype(I)::value;
+            constexpr int op = L::opp(i);
+            const unsigned kind = (unsigned)(lk >> (3 * i)) & 7u;
+            int pa = op;
+            size_t sa = c;
+            if (kind == kLinkStream) {
+                pa = i;
+                sa = (size_t)c - link_offset<Q>(i, g);
+            } else if (kind == kLinkEdge) {
+                const int py = (int)y - L::ey(i), pz = (int)z - L::ez(i);
+                pa = edge_plane<Q, i>(py < 0 || py >= g.ny, pz < 0 || pz >= g.nz, p);
+            }
+            const float va = load_plane<Q, S>(fin, pa, g.ps, sa, L::w(i));
+            float v = va;
+            if (kind == kLinkBzNear || kind == kLinkBzFar) {
+                const float2 kk = __ldg(bl.coef + co0 + __popc(bzmask & ((1u << i) - 1u)));
+                const int pb = kind == kLinkBzNear ? op : i;
+                const size_t sb = kind == kLinkBzNear ? (size_t)c + link_offset<Q>(i, g) : (size_t)c;
+                const float vb = load_plane<Q, S>(fin, pb, g.ps, sb, L::w(i));
+                v = kk.x * va + kk.y * vb;
+            }
+            h[i] = make_float2((v - L::w(i)) * 256.0f, 0.0f);
+        });
+    } else {
+        static_for<0, Q>([&](auto I) { h[decltype(I)::value] = make_float2(0.0f, 0.0f); });
+    }
+    Mom2 mo;
+    const unsigned bad = moments2<Q>(h, mo) & (fluid ? 1u : 0u);
+    float x0, x1, x2;
+    closure_invariants(mo.pxx.x, mo.pyy.x, mo.pzz.x, mo.pxy.x, mo.pxz.x, mo.pyz.x, mo.pp.x, mo.inv.x, x0, x1, x2);
+    const float x3 = fluid ? (float)__ldg(cl.wall + c) * 0.0625f : 0.0f;
+    const bool lin = fluid && closure_wall_ok(cl, __ldg(cl.wall + c)) && closure_in_range(cl, x0, x1, x2);
+    const float sg = smagorinsky_g(mo.pp.x, mo.rho.x, mo.inv.x, p.tau, p.cs);
+    const float ds = closure_anchored(cl) ? smagorinsky_d3(mo.pp.x, mo.rho.x, mo.inv.x, p.tau, p.cs) : 0.0f;
+    uint32_t* in = s_in + (threadIdx.x & 31) * 8;
+    closure_pack_inputs(cl, x0, x1, x2, x3, in);
+    closure_pack_inputs(cl, 0.0f, 0.0f, 0.0f, 0.0f, in + 4);
+    __syncwarp();
+    float2 nu = make_float2(0.0f, 0.0f);  // warps with no cell in range skip the MLP
+    if (__any_sync(0xffffffffu, lin)) nu = closure_warp_mlp(cl.frag, s_in, s_out);
+    if (!fluid) return;
+    const float gx = lin ? closure_g(cl, nu.x, p.tau, ds) : sg;
+    relax2<Q>(h, mo, make_float2(gx, gx));
+    if (bad) atomicOr(diverged, 1);
+    static_for<0, Q>([&](auto I) {
+        constexpr int i = decltype(I)::value;
+        store_pop_c<Q, S, i>(fout, g.ps, c, L::w(i) + h[i].x * (1.0f / 256.0f));
+    });
+}
+
 // Blocks of k_bulk_pairs when its interior warps run in k_bulk_tiles: the
 // shell as a 1D list of (chunk, 8-row block, z) items in three regions,
 //   E  the first and last chunk of every row block of every layer,
@@ -361,8 +511,14 @@ __global__ void __launch_bounds__(32 * kBulkRows, 4) k_bulk_pairs(const typename
                                                                 typename S::T* __restrict__ fout,
                                                                 const uint32_t* __restrict__ bulk_bits, Geom g,
                                                                 StepParams p, PlanePtrs pp, int z0,
-                                                                int* __restrict__ diverged, PairsShell sh) {
-    int bx = blockIdx.x, by = blockIdx.y, z = z0 + blockIdx.z;
+                                                                int* __restrict__ diverged, PairsShell sh,
+                                                                BoundarySpan bnd) {
+    uint32_t e;
+    if (boundary_block(bnd, e)) {
+        if (e < bnd.end) boundary_entry<Q, S>(fin, fout, bnd.list, e, g, p, diverged);
+        return;
+    }
+    int bx = blockIdx.x, by = blockIdx.y, z = z0 + (int)(blockIdx.z - bnd.slabs);
     if (sh.n) shell_item(sh, bx, by, z);
     pairs_tile<Q, S, Par>(fin, fout, bulk_bits, g, p, pp, diverged, bx, by, z, sh.n != 0);
 }
@@ -405,15 +561,22 @@ __global__ void __launch_bounds__(32 * kBulkRows, 4) k_bulk_pairs_learned(const 
                                                                         typename S::T* __restrict__ fout,
                                                                         const uint32_t* __restrict__ bulk_bits,
                                                                         Geom g, StepParams p, PlanePtrs pp, int z0,
-                                                                        int* __restrict__ diverged, ClosureDev cl) {
+                                                                        int* __restrict__ diverged, ClosureDev cl,
+                                                                        BoundarySpan bnd) {
     static_assert(!S::kExact, "the learned closure runs on the 16-bit offset formats");
     using L = Lattice<Q>;
     using T = typename S::T;
     __shared__ uint32_t s_in[kBulkRows][32 * 8];
     __shared__ float2 s_out[kBulkRows][32];
     __shared__ float2 s_mo[kBulkRows][12][32];  // the relaxation's moments while the MLP runs
+    uint32_t e;
+    if (boundary_block(bnd, e)) {
+        boundary_entry_learned<Q, S>(fin, fout, bnd.list, e, bnd.end, g, p, diverged, cl, s_in[threadIdx.y],
+                                     s_out[threadIdx.y]);
+        return;
+    }
     const int y = blockIdx.y * kBulkRows + threadIdx.y;
-    const int z = z0 + blockIdx.z;
+    const int z = z0 + (int)(blockIdx.z - bnd.slabs);
     if (y >= g.ny) return;  // the whole warp: one row
     const size_t row = (size_t)z * g.ny + y;
     const int k = 2 * threadIdx.x;
@@ -548,13 +711,24 @@ __global__ void __launch_bounds__(32 * kBulkRows, 4) k_bulk_pairs_learned_tc(con
                                                                            typename S::T* __restrict__ fout,
                                                                            const uint32_t* __restrict__ bulk_bits,
                                                                            Geom g, StepParams p, PlanePtrs pp, int z0,
-                                                                           int* __restrict__ diverged, ClosureDev cl) {
+                                                                           int* __restrict__ diverged, ClosureDev cl,
+                                                                           BoundarySpan bnd) {
     static_assert(!S::kExact, "the learned closure runs on the 16-bit offset formats");
     using L = Lattice<Q>;
     using T = typename S::T;
     __shared__ TcSmem tsm;
+    uint32_t e;
+    if (boundary_block(bnd, e)) {
+        // the warps' closure buffers in the space of the block's MLP
+        static_assert(sizeof(TcSmem) >= kBulkRows * 32 * (8 * sizeof(uint32_t) + sizeof(float2)), "closure buffers");
+        uint32_t* s_in = reinterpret_cast<uint32_t*>(&tsm);
+        float2* s_out = reinterpret_cast<float2*>(s_in + kBulkRows * 32 * 8);
+        boundary_entry_learned<Q, S>(fin, fout, bnd.list, e, bnd.end, g, p, diverged, cl, s_in + threadIdx.y * 32 * 8,
+                                     s_out + threadIdx.y * 32);
+        return;
+    }
     const int y = blockIdx.y * kBulkRows + threadIdx.y;
-    const int z = z0 + blockIdx.z;
+    const int z = z0 + (int)(blockIdx.z - bnd.slabs);
     const bool row_ok = y < g.ny;  // the whole warp: one row
     const size_t row = (size_t)z * g.ny + (row_ok ? y : 0);
     const int k = 2 * threadIdx.x;
@@ -856,78 +1030,6 @@ __global__ void __launch_bounds__(32 * ROWS, 32 / ROWS) k_bulk_pairs_batch(const
     }
 }
 
-// Boundary-list entries: fluid cells with a solid neighbour (off the
-// inlet/outlet planes) and the solid cells an outlet reads. Every link's source
-// address is formed with selects first and all loads issue together.
-template <int Q, class S>
-__device__ __forceinline__ void boundary_entry(const typename S::T* __restrict__ fin,
-                                               typename S::T* __restrict__ fout, const BoundaryList& bl, uint32_t e,
-                                               const Geom& g, const StepParams& p, int* __restrict__ diverged) {
-    using L = Lattice<Q>;
-    const uint32_t c = __ldg(bl.cells + e);
-    const unsigned long long lk = __ldg(bl.links + e);
-    const unsigned cls = (unsigned)(lk >> kClassShift) & 7u;
-    const uint32_t nxy = (uint32_t)g.nxy;
-    const uint32_t z = c / nxy;
-    const uint32_t rem = c - z * nxy;
-    const uint32_t y = rem / (uint32_t)g.nx;
-
-    float f[Q];
-    if (cls == kCellSolidFill) {  // solid cell: f_i = w_i (LbmReference.cpp:264-267)
-        static_for<0, Q>([&](auto I) {
-            constexpr int i = decltype(I)::value;
-            store_pop_c<Q, S, i>(fout, g.ps, c, L::w(i));
-        });
-        return;
-    }
-    // Fluid cell next to a wall (LbmReference.cpp:329-383).
-    const uint32_t co0 = __ldg(bl.coef_off + e);
-    uint32_t bzmask = 0;  // directions that carry a Bouzidi coefficient pair
-    static_for<0, Q>([&](auto I) {
-        constexpr int i = decltype(I)::value;
-        if ((((unsigned)(lk >> (3 * i))) & 6u) == 2u) bzmask |= 1u << i;
-    });
-    static_for<0, Q>([&](auto I) {
-        constexpr int i = decltype(I)::value;
-        constexpr int op = L::opp(i);
-        const unsigned kind = (unsigned)(lk >> (3 * i)) & 7u;
-        int pa = op;
-        size_t sa = c;
-        if (kind == kLinkStream) {
-            pa = i;
-            sa = (size_t)c - link_offset<Q>(i, g);
-        } else if (kind == kLinkEdge) {
-            const int py = (int)y - L::ey(i), pz = (int)z - L::ez(i);
-            pa = edge_plane<Q, i>(py < 0 || py >= g.ny, pz < 0 || pz >= g.nz, p);
-        }
-        const float va = load_plane<Q, S>(fin, pa, g.ps, sa, L::w(i));
-        float v = va;
-        if (kind == kLinkBzNear || kind == kLinkBzFar) {
-            const float2 k = __ldg(bl.coef + co0 + __popc(bzmask & ((1u << i) - 1u)));
-            const int pb = kind == kLinkBzNear ? op : i;
-            const size_t sb = kind == kLinkBzNear ? (size_t)c + link_offset<Q>(i, g) : (size_t)c;
-            const float vb = load_plane<Q, S>(fin, pb, g.ps, sb, L::w(i));
-            v = k.x * va + k.y * vb;
-        }
-        f[i] = v;
-    });
-    if (collide<Q, S::kExact>(f, p.tau, p.cs)) atomicOr(diverged, 1);
-    static_for<0, Q>([&](auto I) {
-        constexpr int i = decltype(I)::value;
-        store_pop_c<Q, S, i>(fout, g.ps, c, f[i]);
-    });
-}
-
-template <int Q, class S>
-__global__ void __launch_bounds__(128) k_boundary_pull(const typename S::T* __restrict__ fin,
-                                                        typename S::T* __restrict__ fout, BoundaryList bl,
-                                                        uint32_t begin, uint32_t end, Geom g, StepParams p,
-                                                        int* __restrict__ diverged) {
-    const uint32_t e = begin + blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= end) return;
-    boundary_entry<Q, S>(fin, fout, bl, e, g, p, diverged);
-}
-
 // The boundary-list entries of every lattice of a batch in one launch: a
 // thread takes one entry of the concatenated lists and finds its lattice by
 // binary search over the lattices' first entries.
@@ -949,95 +1051,6 @@ __global__ void __launch_bounds__(128) k_boundary_pull_batch(const BatchLattice*
                          (uint32_t)(w - L.bnd_first), L.g, L.p, L.diverged);
 }
 
-// k_boundary_pull with the learned closure (16-bit offset storage): the same
-// link handling in float populations, then the two-phase collision on
-// offsets (f - w) * 2^8 with the warp-wide closure. Every lane of a warp runs
-// the closure; only live fluid entries store.
-template <int Q, class S>
-__global__ void __launch_bounds__(128) k_boundary_pull_learned(const typename S::T* __restrict__ fin,
-                                                                typename S::T* __restrict__ fout, BoundaryList bl,
-                                                                uint32_t begin, uint32_t end, Geom g, StepParams p,
-                                                                int* __restrict__ diverged, ClosureDev cl) {
-    static_assert(!S::kExact, "the learned closure runs on the 16-bit offset formats");
-    using L = Lattice<Q>;
-    __shared__ uint32_t s_in[4][32 * 8];
-    __shared__ float2 s_out[4][32];
-    const uint32_t e = begin + blockIdx.x * blockDim.x + threadIdx.x;
-    const bool live = e < end;
-    const uint32_t c = live ? __ldg(bl.cells + e) : 0u;
-    const unsigned long long lk = live ? __ldg(bl.links + e) : 0ull;
-    const unsigned cls = (unsigned)(lk >> kClassShift) & 7u;
-    const bool fluid = live && cls != kCellSolidFill;
-    if (live && !fluid) {  // solid cell: f_i = w_i (LbmReference.cpp:264-267)
-        static_for<0, Q>([&](auto I) {
-            constexpr int i = decltype(I)::value;
-            store_pop_c<Q, S, i>(fout, g.ps, c, L::w(i));
-        });
-    }
-    const uint32_t nxy = (uint32_t)g.nxy;
-    const uint32_t z = c / nxy;
-    const uint32_t rem = c - z * nxy;
-    const uint32_t y = rem / (uint32_t)g.nx;
-    float2 h[Q];
-    if (fluid) {
-        const uint32_t co0 = __ldg(bl.coef_off + e);
-        uint32_t bzmask = 0;
-        static_for<0, Q>([&](auto I) {
-            constexpr int i = decltype(I)::value;
-            if ((((unsigned)(lk >> (3 * i))) & 6u) == 2u) bzmask |= 1u << i;
-        });
-        static_for<0, Q>([&](auto I) {
-            constexpr int i = decltype(I)::value;
-            constexpr int op = L::opp(i);
-            const unsigned kind = (unsigned)(lk >> (3 * i)) & 7u;
-            int pa = op;
-            size_t sa = c;
-            if (kind == kLinkStream) {
-                pa = i;
-                sa = (size_t)c - link_offset<Q>(i, g);
-            } else if (kind == kLinkEdge) {
-                const int py = (int)y - L::ey(i), pz = (int)z - L::ez(i);
-                pa = edge_plane<Q, i>(py < 0 || py >= g.ny, pz < 0 || pz >= g.nz, p);
-            }
-            const float va = load_plane<Q, S>(fin, pa, g.ps, sa, L::w(i));
-            float v = va;
-            if (kind == kLinkBzNear || kind == kLinkBzFar) {
-                const float2 kk = __ldg(bl.coef + co0 + __popc(bzmask & ((1u << i) - 1u)));
-                const int pb = kind == kLinkBzNear ? op : i;
-                const size_t sb = kind == kLinkBzNear ? (size_t)c + link_offset<Q>(i, g) : (size_t)c;
-                const float vb = load_plane<Q, S>(fin, pb, g.ps, sb, L::w(i));
-                v = kk.x * va + kk.y * vb;
-            }
-            h[i] = make_float2((v - L::w(i)) * 256.0f, 0.0f);
-        });
-    } else {
-        static_for<0, Q>([&](auto I) { h[decltype(I)::value] = make_float2(0.0f, 0.0f); });
-    }
-    Mom2 mo;
-    const unsigned bad = moments2<Q>(h, mo) & (fluid ? 1u : 0u);
-    float x0, x1, x2;
-    closure_invariants(mo.pxx.x, mo.pyy.x, mo.pzz.x, mo.pxy.x, mo.pxz.x, mo.pyz.x, mo.pp.x, mo.inv.x, x0, x1, x2);
-    const float x3 = fluid ? (float)__ldg(cl.wall + c) * 0.0625f : 0.0f;
-    const bool lin = fluid && closure_wall_ok(cl, __ldg(cl.wall + c)) && closure_in_range(cl, x0, x1, x2);
-    const float sg = smagorinsky_g(mo.pp.x, mo.rho.x, mo.inv.x, p.tau, p.cs);
-    const float ds = closure_anchored(cl) ? smagorinsky_d3(mo.pp.x, mo.rho.x, mo.inv.x, p.tau, p.cs) : 0.0f;
-    const int warp = threadIdx.x >> 5;
-    uint32_t* in = &s_in[warp][(threadIdx.x & 31) * 8];
-    closure_pack_inputs(cl, x0, x1, x2, x3, in);
-    closure_pack_inputs(cl, 0.0f, 0.0f, 0.0f, 0.0f, in + 4);
-    __syncwarp();
-    float2 nu = make_float2(0.0f, 0.0f);  // warps with no cell in range skip the MLP
-    if (__any_sync(0xffffffffu, lin)) nu = closure_warp_mlp(cl.frag, s_in[warp], s_out[warp]);
-    if (!fluid) return;
-    const float gx = lin ? closure_g(cl, nu.x, p.tau, ds) : sg;
-    relax2<Q>(h, mo, make_float2(gx, gx));
-    if (bad) atomicOr(diverged, 1);
-    static_for<0, Q>([&](auto I) {
-        constexpr int i = decltype(I)::value;
-        store_pop_c<Q, S, i>(fout, g.ps, c, L::w(i) + h[i].x * (1.0f / 256.0f));
-    });
-}
-
 // Plane pointers of a ping-pong step (PlanePtrs in lbm_internal.h).
 template <int Q, class S>
 static PlanePtrs pp_of(const void* fin, void* fout, const Geom& g) {
@@ -1053,14 +1066,15 @@ static PlanePtrs pp_of(const void* fin, void* fout, const Geom& g) {
 
 template <int Q, class S>
 static cudaError_t bulk_t(const void* fin, void* fout, const uint32_t* bits, const Geom& g, const StepParams& p,
-                          int z0, int zc, int* dv, cudaStream_t s, int* launched, int staged) {
+                          int z0, int zc, int* dv, cudaStream_t s, int* launched, const BoundarySpan& bnd,
+                          int staged) {
     *launched = 0;
-    if (zc <= 0) return cudaSuccess;
+    if (zc <= 0 && bnd.end <= bnd.begin) return cudaSuccess;
     const int z1 = z0 + zc;
     dim3 block(32, kBulkRows, 1);
     const PlanePtrs pp = pp_of<Q, S>(fin, fout, g);
     PairsShell sh{};
-    if (staged) {  // the interior warps' rows staged in shared memory by TMA (even nx)
+    if (staged && zc > 0) {  // the interior warps' rows staged in shared memory by TMA (even nx)
         int nl = 0;
         cudaError_t e = launch_bulk_staged(Q, storage_code<S>(), fin, fout, bits, g, p, z0, zc, dv, s, &nl);
         if (e != cudaSuccess) return e;
@@ -1078,19 +1092,21 @@ static cudaError_t bulk_t(const void* fin, void* fout, const uint32_t* bits, con
         sh.nf = zi1 > sh.zi0 ? (unsigned long long)(sh.gx - 2) * sh.nyf * (zi1 - sh.zi0) : 0ull;
         const unsigned long long ng = (unsigned long long)(sh.gx - 2) * sh.nyb * sh.nzf;
         sh.n = sh.ne + sh.nf + ng;
-        if (sh.n == 0) return cudaSuccess;
-        k_bulk_pairs<Q, S, kNxEven><<<(unsigned)sh.n, block, 0, s>>>((const typename S::T*)fin, (typename S::T*)fout,
-                                                                     bits, g, p, pp, z0, dv, sh);
+        const BoundarySpan bs = with_slabs(bnd, (unsigned)sh.n, 1);
+        k_bulk_pairs<Q, S, kNxEven><<<dim3((unsigned)sh.n, 1, 1 + bs.slabs), block, 0, s>>>(
+            (const typename S::T*)fin, (typename S::T*)fout, bits, g, p, pp, z0, dv, sh, bs);
         ++*launched;
         return cudaGetLastError();
     }
     // odd nx: one cell more, for the rows shifted to the left
     const int par = pair_parity(g);
     dim3 grid((unsigned)((g.nx + (par == kNxEven ? 0 : 1) + 63) / 64),
-              (unsigned)((g.ny + kBulkRows - 1) / kBulkRows), (unsigned)zc);
+              (unsigned)((g.ny + kBulkRows - 1) / kBulkRows), 1);
+    const BoundarySpan bs = with_slabs(bnd, grid.x, grid.y);
+    grid.z = (unsigned)(zc > 0 ? zc : 0) + bs.slabs;
     auto launch = [&](auto P) {
-        k_bulk_pairs<Q, S, decltype(P)::value><<<grid, block, 0, s>>>((const typename S::T*)fin,
-                                                                     (typename S::T*)fout, bits, g, p, pp, z0, dv, sh);
+        k_bulk_pairs<Q, S, decltype(P)::value><<<grid, block, 0, s>>>(
+            (const typename S::T*)fin, (typename S::T*)fout, bits, g, p, pp, z0, dv, sh, bs);
     };
     if (par == kNxEven)
         launch(std::integral_constant<int, kNxEven>{});
@@ -1103,58 +1119,27 @@ static cudaError_t bulk_t(const void* fin, void* fout, const uint32_t* bits, con
 }
 
 template <int Q, class S>
-static cudaError_t boundary_t(const void* fin, void* fout, const BoundaryList& bl, uint32_t b, uint32_t e,
-                              const Geom& g, const StepParams& p, int* dv, cudaStream_t s) {
-    if (e <= b) return cudaSuccess;
-    const unsigned threads = 128;
-    const unsigned blocks = (e - b + threads - 1) / threads;
-    k_boundary_pull<Q, S><<<blocks, threads, 0, s>>>((const typename S::T*)fin, (typename S::T*)fout, bl, b, e, g, p,
-                                                     dv);
-    return cudaGetLastError();
-}
-
-template <int Q, class S>
 static cudaError_t bulk_learned_t(const void* fin, void* fout, const uint32_t* bits, const Geom& g,
                                   const StepParams& p, int z0, int zc, int* dv, cudaStream_t s, int* launched,
-                                  const ClosureDev& cl, int tc) {
+                                  const ClosureDev& cl, const BoundarySpan& bnd, int tc) {
     *launched = 0;
     if constexpr (S::kExact) {
         return cudaErrorNotSupported;
     } else {
-        if (zc <= 0) return cudaSuccess;
+        if (zc <= 0 && bnd.end <= bnd.begin) return cudaSuccess;
         if (g.nx % 2 != 0) return cudaErrorNotSupported;
-        PlanePtrs pp{};
-        for (int i = 0; i < Q; ++i) {
-            const long long off = (long long)Lattice<Q>::ex(i) + (long long)Lattice<Q>::ey(i) * g.nx +
-                                  (long long)Lattice<Q>::ez(i) * g.nxy;
-            pp.src[i] = (const typename S::T*)fin + ((long long)i * (long long)g.ps - off);
-            pp.dst[i] = (typename S::T*)fout + (size_t)i * g.ps;
-        }
+        const PlanePtrs pp = pp_of<Q, S>(fin, fout, g);
         dim3 block(32, kBulkRows, 1);
-        dim3 grid((unsigned)((g.nx + 63) / 64), (unsigned)((g.ny + kBulkRows - 1) / kBulkRows), (unsigned)zc);
+        dim3 grid((unsigned)((g.nx + 63) / 64), (unsigned)((g.ny + kBulkRows - 1) / kBulkRows), 1);
+        const BoundarySpan bs = with_slabs(bnd, grid.x, grid.y);
+        grid.z = (unsigned)(zc > 0 ? zc : 0) + bs.slabs;
         if (tc)
             k_bulk_pairs_learned_tc<Q, S><<<grid, block, 0, s>>>((const typename S::T*)fin, (typename S::T*)fout,
-                                                                 bits, g, p, pp, z0, dv, cl);
+                                                                 bits, g, p, pp, z0, dv, cl, bs);
         else
             k_bulk_pairs_learned<Q, S><<<grid, block, 0, s>>>((const typename S::T*)fin, (typename S::T*)fout, bits,
-                                                              g, p, pp, z0, dv, cl);
+                                                              g, p, pp, z0, dv, cl, bs);
         ++*launched;
-        return cudaGetLastError();
-    }
-}
-
-template <int Q, class S>
-static cudaError_t boundary_learned_t(const void* fin, void* fout, const BoundaryList& bl, uint32_t b, uint32_t e,
-                                      const Geom& g, const StepParams& p, int* dv, cudaStream_t s,
-                                      const ClosureDev& cl) {
-    if constexpr (S::kExact) {
-        return cudaErrorNotSupported;
-    } else {
-        if (e <= b) return cudaSuccess;
-        const unsigned threads = 128;
-        const unsigned blocks = (e - b + threads - 1) / threads;
-        k_boundary_pull_learned<Q, S><<<blocks, threads, 0, s>>>((const typename S::T*)fin, (typename S::T*)fout, bl,
-                                                                 b, e, g, p, dv, cl);
         return cudaGetLastError();
     }
 }
@@ -1189,27 +1174,16 @@ static cudaError_t closure_probe_t(const void* f, const uint8_t* solid, const Ge
 
 cudaError_t launch_bulk_pull(int q, int storage, const void* fin, void* fout, const uint32_t* bulk_bits,
                              const Geom& g, const StepParams& p, int z0, int zc, int* diverged, cudaStream_t s,
-                             int* launched, int staged) {
+                             int* launched, const BoundarySpan& bnd, int staged) {
     const int st = staged && g.nx % 2 == 0 && staged_eligible(storage, g) ? 1 : 0;
-    FC_DISPATCH(q, storage, bulk_t, fin, fout, bulk_bits, g, p, z0, zc, diverged, s, launched, st);
-}
-
-cudaError_t launch_boundary_pull(int q, int storage, const void* fin, void* fout, const BoundaryList& bl,
-                                 uint32_t begin, uint32_t end, const Geom& g, const StepParams& p, int* diverged,
-                                 cudaStream_t s) {
-    FC_DISPATCH(q, storage, boundary_t, fin, fout, bl, begin, end, g, p, diverged, s);
+    FC_DISPATCH(q, storage, bulk_t, fin, fout, bulk_bits, g, p, z0, zc, diverged, s, launched, bnd, st);
 }
 
 cudaError_t launch_bulk_pull_learned(int q, int storage, const void* fin, void* fout, const uint32_t* bulk_bits,
                                      const Geom& g, const StepParams& p, int z0, int zc, int* diverged,
-                                     cudaStream_t s, int* launched, const ClosureDev& cl, int tc) {
-    FC_DISPATCH(q, storage, bulk_learned_t, fin, fout, bulk_bits, g, p, z0, zc, diverged, s, launched, cl, tc);
-}
-
-cudaError_t launch_boundary_pull_learned(int q, int storage, const void* fin, void* fout, const BoundaryList& bl,
-                                         uint32_t begin, uint32_t end, const Geom& g, const StepParams& p,
-                                         int* diverged, cudaStream_t s, const ClosureDev& cl) {
-    FC_DISPATCH(q, storage, boundary_learned_t, fin, fout, bl, begin, end, g, p, diverged, s, cl);
+                                     cudaStream_t s, int* launched, const ClosureDev& cl, const BoundarySpan& bnd,
+                                     int tc) {
+    FC_DISPATCH(q, storage, bulk_learned_t, fin, fout, bulk_bits, g, p, z0, zc, diverged, s, launched, cl, bnd, tc);
 }
 
 template <int Q, class S>

@@ -196,6 +196,191 @@ __device__ __forceinline__ void aa_row_end_cells(typename S::T* f, const Geom& g
     }
 }
 
+// Boundary-list entries (boundary_entry of lbm_step.cu, in place).
+template <int Q, class S, bool Odd>
+__device__ __forceinline__ void aa_boundary_entry(typename S::T* f, const BoundaryList& bl, uint32_t e, const Geom& g,
+                                                  const StepParams& p, int* __restrict__ diverged, const AaSide& sd) {
+    using L = Lattice<Q>;
+    using T = typename S::T;
+    const uint32_t c = __ldg(bl.cells + e);
+    const unsigned long long lk = __ldg(bl.links + e);
+    const unsigned cls = (unsigned)(lk >> kClassShift) & 7u;
+    const uint32_t nxy = (uint32_t)g.nxy;
+    const int z = (int)(c / nxy);
+    const uint32_t rem = c - (uint32_t)z * nxy;
+    const int y = (int)(rem / (uint32_t)g.nx);
+    const int x = (int)(rem - (uint32_t)y * (uint32_t)g.nx);
+    const size_t row = (size_t)z * g.ny + y;
+    const int col = outm_col(x, g);
+
+    if (cls == kCellSolidFill) {
+        // f_i = w_i (LbmReference.cpp:264-267). In place the solid cell's
+        // slots carry its neighbours' bounced populations, so only the
+        // outlet's view of it, the moments, is written.
+        if (col >= 0) {
+            float wv[Q];
+            static_for<0, Q>([&](auto I) {
+                constexpr int i = decltype(I)::value;
+                wv[i] = L::w(i);
+            });
+            sd.outm[outm_index(sd, Odd ? 0 : 1, col, row)] = stored_moments<Q, S>(wv);
+        }
+        return;
+    }
+    const uint32_t co0 = __ldg(bl.coef_off + e);
+    uint32_t bzmask = 0;
+    static_for<0, Q>([&](auto I) {
+        constexpr int i = decltype(I)::value;
+        if ((((unsigned)(lk >> (3 * i))) & 6u) == 2u) bzmask |= 1u << i;
+    });
+    T* bz = static_cast<T*>(sd.bz);
+    float v[Q];
+    static_for<0, Q>([&](auto I) {
+        constexpr int i = decltype(I)::value;
+        constexpr int op = L::opp(i);
+        const unsigned kind = (unsigned)(lk >> (3 * i)) & 7u;
+        const size_t off = (size_t)link_offset<Q>(i, g);
+        size_t sa;
+        if (kind == kLinkStream) {  // f*_i(c - e_i)
+            sa = Odd ? (size_t)op * g.ps + (c - off) : (size_t)i * g.ps + c;
+        } else if (kind == kLinkEdge) {  // f*_m(c) for the mirrored / bounced m
+            const int py = y - L::ey(i), pz = z - L::ez(i);
+            const int m = edge_plane<Q, i>(py < 0 || py >= g.ny, pz < 0 || pz >= g.nz, p);
+            sa = (size_t)L::opp(m) * g.ps + c;
+        } else {  // f*_op(c); before an even step it sits in the solid neighbour c - e_i
+            sa = Odd ? (size_t)i * g.ps + c : (size_t)op * g.ps + (c - off);
+        }
+        const float va = S::dec(ld_plain<S>(f + sa), L::w(i));
+        float r = va;
+        if (kind == kLinkBzNear || kind == kLinkBzFar) {
+            const uint32_t slot = co0 + __popc(bzmask & ((1u << i) - 1u));
+            const float2 kc = __ldg(bl.coef + slot);
+            float vb;
+            if (kind == kLinkBzNear) {  // f*_op(c + e_i)
+                const size_t sb = Odd ? (size_t)i * g.ps + (c + off) : (size_t)op * g.ps + c;
+                vb = S::dec(ld_plain<S>(f + sb), L::w(i));
+            } else {  // f*_i(c), kept from the previous step
+                vb = S::dec(bz[slot], L::w(i));
+            }
+            r = kc.x * va + kc.y * vb;
+        }
+        v[i] = r;
+    });
+    if (collide<Q, S::kExact>(v, p.tau, p.cs)) atomicOr(diverged, 1);
+    static_for<0, Q>([&](auto I) {
+        constexpr int i = decltype(I)::value;
+        const T t = S::enc(v[i], L::w(i));
+        f[out_slot<Q, i, Odd>(c, x, y, z, g)] = t;
+        if ((((unsigned)(lk >> (3 * i))) & 7u) == kLinkBzFar) bz[co0 + __popc(bzmask & ((1u << i) - 1u))] = t;
+    });
+    if (col >= 0) sd.outm[outm_index(sd, Odd ? 0 : 1, col, row)] = stored_moments<Q, S>(v);
+}
+
+// aa_boundary_entry with the learned closure: its slots around the collision
+// of boundary_entry_learned (link values in floats, then the two-phase
+// collision on offsets with the warp-wide closure). Every lane of a warp runs
+// the closure (e == end: no entry); only live fluid entries store. s_in and
+// s_out are the warp's closure buffers.
+template <int Q, class S, bool Odd>
+__device__ __forceinline__ void aa_boundary_entry_learned(typename S::T* f, const BoundaryList& bl, uint32_t e,
+                                                          uint32_t end, const Geom& g, const StepParams& p,
+                                                          int* __restrict__ diverged, const AaSide& sd,
+                                                          const ClosureDev& cl, uint32_t* s_in, float2* s_out) {
+    static_assert(!S::kExact, "the learned closure runs on the 16-bit offset formats");
+    using L = Lattice<Q>;
+    using T = typename S::T;
+    const bool live = e < end;
+    const uint32_t c = live ? __ldg(bl.cells + e) : 0u;
+    const unsigned long long lk = live ? __ldg(bl.links + e) : 0ull;
+    const unsigned cls = (unsigned)(lk >> kClassShift) & 7u;
+    const bool fluid = live && cls != kCellSolidFill;
+    const uint32_t nxy = (uint32_t)g.nxy;
+    const int z = (int)(c / nxy);
+    const uint32_t rem = c - (uint32_t)z * nxy;
+    const int y = (int)(rem / (uint32_t)g.nx);
+    const int x = (int)(rem - (uint32_t)y * (uint32_t)g.nx);
+    const size_t row = (size_t)z * g.ny + y;
+    const int col = live ? outm_col(x, g) : -1;
+    if (live && !fluid && col >= 0) {  // a solid cell: only the outlet's view of it (aa_boundary_entry)
+        float wv[Q];
+        static_for<0, Q>([&](auto I) {
+            constexpr int i = decltype(I)::value;
+            wv[i] = L::w(i);
+        });
+        sd.outm[outm_index(sd, Odd ? 0 : 1, col, row)] = stored_moments<Q, S>(wv);
+    }
+    T* bz = static_cast<T*>(sd.bz);
+    const uint32_t co0 = fluid ? __ldg(bl.coef_off + e) : 0u;
+    uint32_t bzmask = 0;
+    static_for<0, Q>([&](auto I) {
+        constexpr int i = decltype(I)::value;
+        if ((((unsigned)(lk >> (3 * i))) & 6u) == 2u) bzmask |= 1u << i;
+    });
+    float2 h[Q];
+    if (fluid) {
+        static_for<0, Q>([&](auto I) {
+            constexpr int i = decltype(I)::value;
+            constexpr int op = L::opp(i);
+            const unsigned kind = (unsigned)(lk >> (3 * i)) & 7u;
+            const size_t off = (size_t)link_offset<Q>(i, g);
+            size_t sa;
+            if (kind == kLinkStream) {  // f*_i(c - e_i)
+                sa = Odd ? (size_t)op * g.ps + (c - off) : (size_t)i * g.ps + c;
+            } else if (kind == kLinkEdge) {  // f*_m(c) for the mirrored / bounced m
+                const int py = y - L::ey(i), pz = z - L::ez(i);
+                const int m = edge_plane<Q, i>(py < 0 || py >= g.ny, pz < 0 || pz >= g.nz, p);
+                sa = (size_t)L::opp(m) * g.ps + c;
+            } else {  // f*_op(c); before an even step it sits in the solid neighbour c - e_i
+                sa = Odd ? (size_t)i * g.ps + c : (size_t)op * g.ps + (c - off);
+            }
+            const float va = S::dec(ld_plain<S>(f + sa), L::w(i));
+            float r = va;
+            if (kind == kLinkBzNear || kind == kLinkBzFar) {
+                const uint32_t slot = co0 + __popc(bzmask & ((1u << i) - 1u));
+                const float2 kc = __ldg(bl.coef + slot);
+                float vb;
+                if (kind == kLinkBzNear) {  // f*_op(c + e_i)
+                    const size_t sb = Odd ? (size_t)i * g.ps + (c + off) : (size_t)op * g.ps + c;
+                    vb = S::dec(ld_plain<S>(f + sb), L::w(i));
+                } else {  // f*_i(c), kept from the previous step
+                    vb = S::dec(bz[slot], L::w(i));
+                }
+                r = kc.x * va + kc.y * vb;
+            }
+            h[i] = make_float2((r - L::w(i)) * 256.0f, 0.0f);
+        });
+    } else {
+        static_for<0, Q>([&](auto I) { h[decltype(I)::value] = make_float2(0.0f, 0.0f); });
+    }
+    Mom2 mo;
+    const unsigned bad = moments2<Q>(h, mo) & (fluid ? 1u : 0u);
+    float x0, x1, x2;
+    closure_invariants(mo.pxx.x, mo.pyy.x, mo.pzz.x, mo.pxy.x, mo.pxz.x, mo.pyz.x, mo.pp.x, mo.inv.x, x0, x1, x2);
+    const float x3 = fluid ? (float)__ldg(cl.wall + c) * 0.0625f : 0.0f;
+    const bool lin = fluid && closure_wall_ok(cl, __ldg(cl.wall + c)) && closure_in_range(cl, x0, x1, x2);
+    const float sg = smagorinsky_g(mo.pp.x, mo.rho.x, mo.inv.x, p.tau, p.cs);
+    const float ds = closure_anchored(cl) ? smagorinsky_d3(mo.pp.x, mo.rho.x, mo.inv.x, p.tau, p.cs) : 0.0f;
+    uint32_t* in = s_in + (threadIdx.x & 31) * 8;
+    closure_pack_inputs(cl, x0, x1, x2, x3, in);
+    closure_pack_inputs(cl, 0.0f, 0.0f, 0.0f, 0.0f, in + 4);
+    __syncwarp();
+    float2 nu = make_float2(0.0f, 0.0f);  // warps with no cell in range skip the MLP
+    if (__any_sync(0xffffffffu, lin)) nu = closure_warp_mlp(cl.frag, s_in, s_out);
+    if (!fluid) return;
+    const float gx = lin ? closure_g(cl, nu.x, p.tau, ds) : sg;
+    relax2<Q>(h, mo, make_float2(gx, gx));
+    if (bad) atomicOr(diverged, 1);
+    float vf[Q];
+    static_for<0, Q>([&](auto I) {
+        constexpr int i = decltype(I)::value;
+        vf[i] = L::w(i) + h[i].x * (1.0f / 256.0f);
+        const T t = S::enc(vf[i], L::w(i));
+        f[out_slot<Q, i, Odd>(c, x, y, z, g)] = t;
+        if ((((unsigned)(lk >> (3 * i))) & 7u) == kLinkBzFar) bz[co0 + __popc(bzmask & ((1u << i) - 1u))] = t;
+    });
+    if (col >= 0) sd.outm[outm_index(sd, Odd ? 0 : 1, col, row)] = stored_moments<Q, S>(vf);
+}
+
 }  // namespace
 
 // Bulk cells (bulk mask) of lattices with even nx; see the file comment.
@@ -203,12 +388,18 @@ template <int Q, class S, bool Odd>
 __global__ void __launch_bounds__(32 * kBulkRows, 4) k_bulk_pairs_aa(typename S::T* f,
                                                                    const uint32_t* __restrict__ bulk_bits, Geom g,
                                                                    StepParams p, PlanePtrs pp, int z0,
-                                                                   int* __restrict__ diverged, AaSide sd) {
+                                                                   int* __restrict__ diverged, AaSide sd,
+                                                                   BoundarySpan bnd) {
     using L = Lattice<Q>;
     using T = typename S::T;
     using T2 = typename S::T2;
+    uint32_t e;
+    if (boundary_block(bnd, e)) {
+        if (e < bnd.end) aa_boundary_entry<Q, S, Odd>(f, bnd.list, e, g, p, diverged, sd);
+        return;
+    }
     const int y = blockIdx.y * kBulkRows + threadIdx.y;
-    const int z = z0 + blockIdx.z;
+    const int z = z0 + (int)(blockIdx.z - bnd.slabs);
     if (y >= g.ny) return;
     const size_t row = (size_t)z * g.ny + y;
     const int k = 2 * threadIdx.x;
@@ -368,88 +559,6 @@ __global__ void __launch_bounds__(32 * kBulkRows, 4) k_bulk_pairs_aa(typename S:
     }
 }
 
-// Boundary-list entries (boundary_entry of lbm_step.cu, in place).
-template <int Q, class S, bool Odd>
-__global__ void __launch_bounds__(128) k_boundary_aa(typename S::T* f, BoundaryList bl, uint32_t begin, uint32_t end,
-                                                     Geom g, StepParams p, int* __restrict__ diverged, AaSide sd) {
-    using L = Lattice<Q>;
-    using T = typename S::T;
-    const uint32_t e = begin + blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= end) return;
-    const uint32_t c = __ldg(bl.cells + e);
-    const unsigned long long lk = __ldg(bl.links + e);
-    const unsigned cls = (unsigned)(lk >> kClassShift) & 7u;
-    const uint32_t nxy = (uint32_t)g.nxy;
-    const int z = (int)(c / nxy);
-    const uint32_t rem = c - (uint32_t)z * nxy;
-    const int y = (int)(rem / (uint32_t)g.nx);
-    const int x = (int)(rem - (uint32_t)y * (uint32_t)g.nx);
-    const size_t row = (size_t)z * g.ny + y;
-    const int col = outm_col(x, g);
-
-    if (cls == kCellSolidFill) {
-        // f_i = w_i (LbmReference.cpp:264-267). In place the solid cell's
-        // slots carry its neighbours' bounced populations, so only the
-        // outlet's view of it, the moments, is written.
-        if (col >= 0) {
-            float wv[Q];
-            static_for<0, Q>([&](auto I) {
-                constexpr int i = decltype(I)::value;
-                wv[i] = L::w(i);
-            });
-            sd.outm[outm_index(sd, Odd ? 0 : 1, col, row)] = stored_moments<Q, S>(wv);
-        }
-        return;
-    }
-    const uint32_t co0 = __ldg(bl.coef_off + e);
-    uint32_t bzmask = 0;
-    static_for<0, Q>([&](auto I) {
-        constexpr int i = decltype(I)::value;
-        if ((((unsigned)(lk >> (3 * i))) & 6u) == 2u) bzmask |= 1u << i;
-    });
-    T* bz = static_cast<T*>(sd.bz);
-    float v[Q];
-    static_for<0, Q>([&](auto I) {
-        constexpr int i = decltype(I)::value;
-        constexpr int op = L::opp(i);
-        const unsigned kind = (unsigned)(lk >> (3 * i)) & 7u;
-        const size_t off = (size_t)link_offset<Q>(i, g);
-        size_t sa;
-        if (kind == kLinkStream) {  // f*_i(c - e_i)
-            sa = Odd ? (size_t)op * g.ps + (c - off) : (size_t)i * g.ps + c;
-        } else if (kind == kLinkEdge) {  // f*_m(c) for the mirrored / bounced m
-            const int py = y - L::ey(i), pz = z - L::ez(i);
-            const int m = edge_plane<Q, i>(py < 0 || py >= g.ny, pz < 0 || pz >= g.nz, p);
-            sa = (size_t)L::opp(m) * g.ps + c;
-        } else {  // f*_op(c); before an even step it sits in the solid neighbour c - e_i
-            sa = Odd ? (size_t)i * g.ps + c : (size_t)op * g.ps + (c - off);
-        }
-        const float va = S::dec(ld_plain<S>(f + sa), L::w(i));
-        float r = va;
-        if (kind == kLinkBzNear || kind == kLinkBzFar) {
-            const uint32_t slot = co0 + __popc(bzmask & ((1u << i) - 1u));
-            const float2 kc = __ldg(bl.coef + slot);
-            float vb;
-            if (kind == kLinkBzNear) {  // f*_op(c + e_i)
-                const size_t sb = Odd ? (size_t)i * g.ps + (c + off) : (size_t)op * g.ps + c;
-                vb = S::dec(ld_plain<S>(f + sb), L::w(i));
-            } else {  // f*_i(c), kept from the previous step
-                vb = S::dec(bz[slot], L::w(i));
-            }
-            r = kc.x * va + kc.y * vb;
-        }
-        v[i] = r;
-    });
-    if (collide<Q, S::kExact>(v, p.tau, p.cs)) atomicOr(diverged, 1);
-    static_for<0, Q>([&](auto I) {
-        constexpr int i = decltype(I)::value;
-        const T t = S::enc(v[i], L::w(i));
-        f[out_slot<Q, i, Odd>(c, x, y, z, g)] = t;
-        if ((((unsigned)(lk >> (3 * i))) & 7u) == kLinkBzFar) bz[co0 + __popc(bzmask & ((1u << i) - 1u))] = t;
-    });
-    if (col >= 0) sd.outm[outm_index(sd, Odd ? 0 : 1, col, row)] = stored_moments<Q, S>(v);
-}
-
 // Stores of a cell pair after the collision (v: scaled offsets or full
 // floats, as collide_pair leaves them): the aligned form for full pairs off
 // the faces (fast), or the general masked form with the edge and
@@ -514,7 +623,7 @@ __global__ void __launch_bounds__(32 * kBulkRows, 4) k_bulk_pairs_aa_learned(typ
                                                                            const uint32_t* __restrict__ bulk_bits,
                                                                            Geom g, StepParams p, PlanePtrs pp, int z0,
                                                                            int* __restrict__ diverged, AaSide sd,
-                                                                           ClosureDev cl) {
+                                                                           ClosureDev cl, BoundarySpan bnd) {
     static_assert(!S::kExact, "the learned closure runs on the 16-bit offset formats");
     using L = Lattice<Q>;
     using T = typename S::T;
@@ -522,8 +631,14 @@ __global__ void __launch_bounds__(32 * kBulkRows, 4) k_bulk_pairs_aa_learned(typ
     __shared__ uint32_t s_in[kBulkRows][32 * 8];
     __shared__ float2 s_out[kBulkRows][32];
     __shared__ float2 s_mo[kBulkRows][12][32];  // the relaxation's moments while the MLP runs
+    uint32_t e;
+    if (boundary_block(bnd, e)) {
+        aa_boundary_entry_learned<Q, S, Odd>(f, bnd.list, e, bnd.end, g, p, diverged, sd, cl, s_in[threadIdx.y],
+                                             s_out[threadIdx.y]);
+        return;
+    }
     const int y = blockIdx.y * kBulkRows + threadIdx.y;
-    const int z = z0 + blockIdx.z;
+    const int z = z0 + (int)(blockIdx.z - bnd.slabs);
     if (y >= g.ny) return;  // the whole warp: one row
     const size_t row = (size_t)z * g.ny + y;
     const int k = 2 * threadIdx.x;
@@ -632,113 +747,6 @@ __global__ void __launch_bounds__(32 * kBulkRows, 4) k_bulk_pairs_aa_learned(typ
     aa_store_pair<Q, S, Odd>(f, pp, g, sd, v, c, x, y, z, row, pair, fast);
 }
 
-// k_boundary_aa with the learned closure: the slots of k_boundary_aa around
-// the collision of k_boundary_pull_learned (link values in floats, then the
-// two-phase collision on offsets with the warp-wide closure). Every lane of
-// a warp runs the closure; only live fluid entries store.
-template <int Q, class S, bool Odd>
-__global__ void __launch_bounds__(128) k_boundary_aa_learned(typename S::T* f, BoundaryList bl, uint32_t begin,
-                                                             uint32_t end, Geom g, StepParams p,
-                                                             int* __restrict__ diverged, AaSide sd, ClosureDev cl) {
-    static_assert(!S::kExact, "the learned closure runs on the 16-bit offset formats");
-    using L = Lattice<Q>;
-    using T = typename S::T;
-    __shared__ uint32_t s_in[4][32 * 8];
-    __shared__ float2 s_out[4][32];
-    const uint32_t e = begin + blockIdx.x * blockDim.x + threadIdx.x;
-    const bool live = e < end;
-    const uint32_t c = live ? __ldg(bl.cells + e) : 0u;
-    const unsigned long long lk = live ? __ldg(bl.links + e) : 0ull;
-    const unsigned cls = (unsigned)(lk >> kClassShift) & 7u;
-    const bool fluid = live && cls != kCellSolidFill;
-    const uint32_t nxy = (uint32_t)g.nxy;
-    const int z = (int)(c / nxy);
-    const uint32_t rem = c - (uint32_t)z * nxy;
-    const int y = (int)(rem / (uint32_t)g.nx);
-    const int x = (int)(rem - (uint32_t)y * (uint32_t)g.nx);
-    const size_t row = (size_t)z * g.ny + y;
-    const int col = live ? outm_col(x, g) : -1;
-    if (live && !fluid && col >= 0) {  // a solid cell: only the outlet's view of it (k_boundary_aa)
-        float wv[Q];
-        static_for<0, Q>([&](auto I) {
-            constexpr int i = decltype(I)::value;
-            wv[i] = L::w(i);
-        });
-        sd.outm[outm_index(sd, Odd ? 0 : 1, col, row)] = stored_moments<Q, S>(wv);
-    }
-    T* bz = static_cast<T*>(sd.bz);
-    const uint32_t co0 = fluid ? __ldg(bl.coef_off + e) : 0u;
-    uint32_t bzmask = 0;
-    static_for<0, Q>([&](auto I) {
-        constexpr int i = decltype(I)::value;
-        if ((((unsigned)(lk >> (3 * i))) & 6u) == 2u) bzmask |= 1u << i;
-    });
-    float2 h[Q];
-    if (fluid) {
-        static_for<0, Q>([&](auto I) {
-            constexpr int i = decltype(I)::value;
-            constexpr int op = L::opp(i);
-            const unsigned kind = (unsigned)(lk >> (3 * i)) & 7u;
-            const size_t off = (size_t)link_offset<Q>(i, g);
-            size_t sa;
-            if (kind == kLinkStream) {  // f*_i(c - e_i)
-                sa = Odd ? (size_t)op * g.ps + (c - off) : (size_t)i * g.ps + c;
-            } else if (kind == kLinkEdge) {  // f*_m(c) for the mirrored / bounced m
-                const int py = y - L::ey(i), pz = z - L::ez(i);
-                const int m = edge_plane<Q, i>(py < 0 || py >= g.ny, pz < 0 || pz >= g.nz, p);
-                sa = (size_t)L::opp(m) * g.ps + c;
-            } else {  // f*_op(c); before an even step it sits in the solid neighbour c - e_i
-                sa = Odd ? (size_t)i * g.ps + c : (size_t)op * g.ps + (c - off);
-            }
-            const float va = S::dec(ld_plain<S>(f + sa), L::w(i));
-            float r = va;
-            if (kind == kLinkBzNear || kind == kLinkBzFar) {
-                const uint32_t slot = co0 + __popc(bzmask & ((1u << i) - 1u));
-                const float2 kc = __ldg(bl.coef + slot);
-                float vb;
-                if (kind == kLinkBzNear) {  // f*_op(c + e_i)
-                    const size_t sb = Odd ? (size_t)i * g.ps + (c + off) : (size_t)op * g.ps + c;
-                    vb = S::dec(ld_plain<S>(f + sb), L::w(i));
-                } else {  // f*_i(c), kept from the previous step
-                    vb = S::dec(bz[slot], L::w(i));
-                }
-                r = kc.x * va + kc.y * vb;
-            }
-            h[i] = make_float2((r - L::w(i)) * 256.0f, 0.0f);
-        });
-    } else {
-        static_for<0, Q>([&](auto I) { h[decltype(I)::value] = make_float2(0.0f, 0.0f); });
-    }
-    Mom2 mo;
-    const unsigned bad = moments2<Q>(h, mo) & (fluid ? 1u : 0u);
-    float x0, x1, x2;
-    closure_invariants(mo.pxx.x, mo.pyy.x, mo.pzz.x, mo.pxy.x, mo.pxz.x, mo.pyz.x, mo.pp.x, mo.inv.x, x0, x1, x2);
-    const float x3 = fluid ? (float)__ldg(cl.wall + c) * 0.0625f : 0.0f;
-    const bool lin = fluid && closure_wall_ok(cl, __ldg(cl.wall + c)) && closure_in_range(cl, x0, x1, x2);
-    const float sg = smagorinsky_g(mo.pp.x, mo.rho.x, mo.inv.x, p.tau, p.cs);
-    const float ds = closure_anchored(cl) ? smagorinsky_d3(mo.pp.x, mo.rho.x, mo.inv.x, p.tau, p.cs) : 0.0f;
-    const int warp = threadIdx.x >> 5;
-    uint32_t* in = &s_in[warp][(threadIdx.x & 31) * 8];
-    closure_pack_inputs(cl, x0, x1, x2, x3, in);
-    closure_pack_inputs(cl, 0.0f, 0.0f, 0.0f, 0.0f, in + 4);
-    __syncwarp();
-    float2 nu = make_float2(0.0f, 0.0f);  // warps with no cell in range skip the MLP
-    if (__any_sync(0xffffffffu, lin)) nu = closure_warp_mlp(cl.frag, s_in[warp], s_out[warp]);
-    if (!fluid) return;
-    const float gx = lin ? closure_g(cl, nu.x, p.tau, ds) : sg;
-    relax2<Q>(h, mo, make_float2(gx, gx));
-    if (bad) atomicOr(diverged, 1);
-    float vf[Q];
-    static_for<0, Q>([&](auto I) {
-        constexpr int i = decltype(I)::value;
-        vf[i] = L::w(i) + h[i].x * (1.0f / 256.0f);
-        const T t = S::enc(vf[i], L::w(i));
-        f[out_slot<Q, i, Odd>(c, x, y, z, g)] = t;
-        if ((((unsigned)(lk >> (3 * i))) & 7u) == kLinkBzFar) bz[co0 + __popc(bzmask & ((1u << i) - 1u))] = t;
-    });
-    if (col >= 0) sd.outm[outm_index(sd, Odd ? 0 : 1, col, row)] = stored_moments<Q, S>(vf);
-}
-
 // Side buffers from the current state (`layout`, read by a step of parity
 // par): the Bouzidi far-side values of every boundary entry ...
 template <int Q, class S>
@@ -789,9 +797,10 @@ __global__ void __launch_bounds__(128) k_aa_prime_rows(const typename S::T* f, G
 
 template <int Q, class S>
 static cudaError_t bulk_aa_t(void* f, const uint32_t* bits, const Geom& g, const StepParams& p, int z0, int zc,
-                             int* dv, cudaStream_t s, int* launched, int odd, const AaSide& sd) {
+                             int* dv, cudaStream_t s, int* launched, int odd, const AaSide& sd,
+                             const BoundarySpan& bnd) {
     *launched = 0;
-    if (zc <= 0) return cudaSuccess;
+    if (zc <= 0 && bnd.end <= bnd.begin) return cudaSuccess;
     if (g.nx % 2 != 0 || g.nx < 4) return cudaErrorNotSupported;
     using T = typename S::T;
     T* base = static_cast<T*>(f);
@@ -804,37 +813,26 @@ static cudaError_t bulk_aa_t(void* f, const uint32_t* bits, const Geom& g, const
         pp.dst[i] = base + (odd ? pi + off : po);
     }
     dim3 block(32, kBulkRows, 1);
-    dim3 grid((unsigned)((g.nx + 63) / 64), (unsigned)((g.ny + kBulkRows - 1) / kBulkRows), (unsigned)zc);
+    dim3 grid((unsigned)((g.nx + 63) / 64), (unsigned)((g.ny + kBulkRows - 1) / kBulkRows), 1);
+    const BoundarySpan bs = with_slabs(bnd, grid.x, grid.y);
+    grid.z = (unsigned)(zc > 0 ? zc : 0) + bs.slabs;
     if (odd)
-        k_bulk_pairs_aa<Q, S, true><<<grid, block, 0, s>>>(base, bits, g, p, pp, z0, dv, sd);
+        k_bulk_pairs_aa<Q, S, true><<<grid, block, 0, s>>>(base, bits, g, p, pp, z0, dv, sd, bs);
     else
-        k_bulk_pairs_aa<Q, S, false><<<grid, block, 0, s>>>(base, bits, g, p, pp, z0, dv, sd);
+        k_bulk_pairs_aa<Q, S, false><<<grid, block, 0, s>>>(base, bits, g, p, pp, z0, dv, sd, bs);
     ++*launched;
-    return cudaGetLastError();
-}
-
-template <int Q, class S>
-static cudaError_t boundary_aa_t(void* f, const BoundaryList& bl, uint32_t b, uint32_t e, const Geom& g,
-                                 const StepParams& p, int* dv, cudaStream_t s, int odd, const AaSide& sd) {
-    if (e <= b) return cudaSuccess;
-    const unsigned threads = 128;
-    const unsigned blocks = (e - b + threads - 1) / threads;
-    if (odd)
-        k_boundary_aa<Q, S, true><<<blocks, threads, 0, s>>>((typename S::T*)f, bl, b, e, g, p, dv, sd);
-    else
-        k_boundary_aa<Q, S, false><<<blocks, threads, 0, s>>>((typename S::T*)f, bl, b, e, g, p, dv, sd);
     return cudaGetLastError();
 }
 
 template <int Q, class S>
 static cudaError_t bulk_aa_learned_t(void* f, const uint32_t* bits, const Geom& g, const StepParams& p, int z0, int zc,
                                      int* dv, cudaStream_t s, int* launched, int odd, const AaSide& sd,
-                                     const ClosureDev& cl) {
+                                     const ClosureDev& cl, const BoundarySpan& bnd) {
     *launched = 0;
     if constexpr (S::kExact) {
         return cudaErrorNotSupported;
     } else {
-        if (zc <= 0) return cudaSuccess;
+        if (zc <= 0 && bnd.end <= bnd.begin) return cudaSuccess;
         if (g.nx % 2 != 0 || g.nx < 4) return cudaErrorNotSupported;
         using T = typename S::T;
         T* base = static_cast<T*>(f);
@@ -847,31 +845,14 @@ static cudaError_t bulk_aa_learned_t(void* f, const uint32_t* bits, const Geom& 
             pp.dst[i] = base + (odd ? pi + off : po);
         }
         dim3 block(32, kBulkRows, 1);
-        dim3 grid((unsigned)((g.nx + 63) / 64), (unsigned)((g.ny + kBulkRows - 1) / kBulkRows), (unsigned)zc);
+        dim3 grid((unsigned)((g.nx + 63) / 64), (unsigned)((g.ny + kBulkRows - 1) / kBulkRows), 1);
+        const BoundarySpan bs = with_slabs(bnd, grid.x, grid.y);
+        grid.z = (unsigned)(zc > 0 ? zc : 0) + bs.slabs;
         if (odd)
-            k_bulk_pairs_aa_learned<Q, S, true><<<grid, block, 0, s>>>(base, bits, g, p, pp, z0, dv, sd, cl);
+            k_bulk_pairs_aa_learned<Q, S, true><<<grid, block, 0, s>>>(base, bits, g, p, pp, z0, dv, sd, cl, bs);
         else
-            k_bulk_pairs_aa_learned<Q, S, false><<<grid, block, 0, s>>>(base, bits, g, p, pp, z0, dv, sd, cl);
+            k_bulk_pairs_aa_learned<Q, S, false><<<grid, block, 0, s>>>(base, bits, g, p, pp, z0, dv, sd, cl, bs);
         ++*launched;
-        return cudaGetLastError();
-    }
-}
-
-template <int Q, class S>
-static cudaError_t boundary_aa_learned_t(void* f, const BoundaryList& bl, uint32_t b, uint32_t e, const Geom& g,
-                                         const StepParams& p, int* dv, cudaStream_t s, int odd, const AaSide& sd,
-                                         const ClosureDev& cl) {
-    if constexpr (S::kExact) {
-        return cudaErrorNotSupported;
-    } else {
-        if (e <= b) return cudaSuccess;
-        const unsigned threads = 128;
-        const unsigned blocks = (e - b + threads - 1) / threads;
-        if (odd)
-            k_boundary_aa_learned<Q, S, true><<<blocks, threads, 0, s>>>((typename S::T*)f, bl, b, e, g, p, dv, sd, cl);
-        else
-            k_boundary_aa_learned<Q, S, false><<<blocks, threads, 0, s>>>((typename S::T*)f, bl, b, e, g, p, dv, sd,
-                                                                          cl);
         return cudaGetLastError();
     }
 }
@@ -905,26 +886,15 @@ static cudaError_t aa_prime_t(const void* f, const BoundaryList& bl, uint32_t co
     } while (0)
 
 cudaError_t launch_bulk_aa(int q, int storage, void* f, const uint32_t* bulk_bits, const Geom& g, const StepParams& p,
-                           int z0, int zc, int* diverged, cudaStream_t s, int* launched, int odd, const AaSide& sd) {
-    FC_DISPATCH(q, storage, bulk_aa_t, f, bulk_bits, g, p, z0, zc, diverged, s, launched, odd, sd);
-}
-
-cudaError_t launch_boundary_aa(int q, int storage, void* f, const BoundaryList& bl, uint32_t begin, uint32_t end,
-                               const Geom& g, const StepParams& p, int* diverged, cudaStream_t s, int odd,
-                               const AaSide& sd) {
-    FC_DISPATCH(q, storage, boundary_aa_t, f, bl, begin, end, g, p, diverged, s, odd, sd);
+                           int z0, int zc, int* diverged, cudaStream_t s, int* launched, int odd, const AaSide& sd,
+                           const BoundarySpan& bnd) {
+    FC_DISPATCH(q, storage, bulk_aa_t, f, bulk_bits, g, p, z0, zc, diverged, s, launched, odd, sd, bnd);
 }
 
 cudaError_t launch_bulk_aa_learned(int q, int storage, void* f, const uint32_t* bulk_bits, const Geom& g,
                                    const StepParams& p, int z0, int zc, int* diverged, cudaStream_t s, int* launched,
-                                   int odd, const AaSide& sd, const ClosureDev& cl) {
-    FC_DISPATCH(q, storage, bulk_aa_learned_t, f, bulk_bits, g, p, z0, zc, diverged, s, launched, odd, sd, cl);
-}
-
-cudaError_t launch_boundary_aa_learned(int q, int storage, void* f, const BoundaryList& bl, uint32_t begin,
-                                       uint32_t end, const Geom& g, const StepParams& p, int* diverged,
-                                       cudaStream_t s, int odd, const AaSide& sd, const ClosureDev& cl) {
-    FC_DISPATCH(q, storage, boundary_aa_learned_t, f, bl, begin, end, g, p, diverged, s, odd, sd, cl);
+                                   int odd, const AaSide& sd, const ClosureDev& cl, const BoundarySpan& bnd) {
+    FC_DISPATCH(q, storage, bulk_aa_learned_t, f, bulk_bits, g, p, z0, zc, diverged, s, launched, odd, sd, cl, bnd);
 }
 
 cudaError_t launch_aa_prime(int q, int storage, const void* f, const BoundaryList& bl, uint32_t count, const Geom& g,

@@ -14,6 +14,23 @@ namespace fc {
 constexpr int kBulkRows = 8;  // block = 32 x-lanes x 8 rows
 constexpr int kBatchChunk = 8;  // consecutive tiles a block of the batch kernel takes at a time
 
+// Blocks of a step launch that take boundary-list entries (BoundarySpan):
+// true for those, with the entry of this thread (one past the end for none).
+__device__ __forceinline__ bool boundary_block(const BoundarySpan& b, uint32_t& entry) {
+    if (blockIdx.z >= b.slabs) return false;
+    const size_t block = ((size_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+    const size_t e = (size_t)b.begin + block * (32 * kBulkRows) + threadIdx.y * 32 + threadIdx.x;
+    entry = e < b.end ? (uint32_t)e : b.end;
+    return true;
+}
+
+// Host: the span with the slabs of gx x gy blocks its entries need.
+inline BoundarySpan with_slabs(BoundarySpan b, unsigned gx, unsigned gy) {
+    const size_t per = (size_t)gx * gy * 32 * kBulkRows;
+    b.slabs = b.end > b.begin ? (unsigned)((b.end - b.begin + per - 1) / per) : 0u;
+    return b;
+}
+
 template <int Q>
 __device__ __forceinline__ long long link_offset(int i, const Geom& g) {
     return (long long)Lattice<Q>::ex(i) + (long long)Lattice<Q>::ey(i) * g.nx + (long long)Lattice<Q>::ez(i) * g.nxy;
