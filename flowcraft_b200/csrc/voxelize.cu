@@ -14,30 +14,38 @@
 //      pair, written in triangle order; a stable radix sort on the tile id
 //      groups them by tile keeping triangle order inside each tile, and a
 //      run-length encode gives each occupied tile its triangle list;
-//   3. raster: one 512-thread block per occupied tile, one cell per thread,
-//      triangles staged through shared memory in index order; each cell keeps
-//      its running signed distance, best normal projection and solid bit in
-//      registers and applies the reference's update rule (Voxelizer.cpp:
-//      236-293) for every triangle whose box holds it, so every cell sees the
-//      same triangles in the same order as the CPU loop and rounds the same
-//      IEEE operations (the library is built without FMA contraction, with
-//      IEEE division and square root);
+//   3. raster: a block per box of 4x4x2 cells of an occupied tile. It tests
+//      the tile's triangles against the box and computes the distances of
+//      those that overlap it, many at a time; each cell's running signed
+//      distance, best normal projection and solid bit then follow the
+//      reference's update rule (Voxelizer.cpp:236-293) over the triangles
+//      whose box holds the cell, in index order, so every cell sees the same
+//      triangles in the same order as the CPU loop and rounds the same IEEE
+//      operations (the library is built without FMA contraction, with IEEE
+//      division and square root);
 //   4. flood fill: fluid cells 6-connected to cell (0,0,0) are the exterior
-//      (Voxelizer.cpp:295-454). Labels start as the start of each x-run in a
-//      32-cell row segment (one warp ballot), then runs are joined across
-//      segment, row and layer boundaries with a lock-free union-find that
-//      links the larger root under the smaller (Playne & Hawick, "A new
-//      algorithm for parallel connected-component labelling on GPUs", IEEE
-//      TPDS 2018). The root of any component is its smallest cell index, so
-//      the exterior is the component whose root is 0;
-//   5. finalize: unreached fluid becomes solid and the signed distance is
-//      reconciled with the classification (Voxelizer.cpp:456-481).
+//      (Voxelizer.cpp:295-454). A tile without triangles holds no solid cell
+//      and is one node; in an occupied tile every x-run of fluid cells in an
+//      8-cell row is a node. Nodes are joined across rows, layers and tile
+//      faces with a lock-free union-find that links larger roots under
+//      smaller ones (Playne & Hawick, "A new algorithm for parallel
+//      connected-component labelling on GPUs", IEEE TPDS 2018). Occupied
+//      tiles are the few along the surface, so the forest is small (the
+//      aircraft at 640 cells: 0.3M nodes for 31M cells) and stays in L2;
+//   5. finalize: one pass writes every cell: unreached fluid becomes solid and
+//      the signed distance is reconciled with the classification
+//      (Voxelizer.cpp:456-481). Tiles without triangles are written without
+//      being read.
+// Measured on a B200, the 57,516-triangle aircraft on 640x308x158 cells, mesh
+// and grid on the device: 3.30 -> 0.57 ms (flood fill and finalize 2.0 -> 0.13,
+// raster 0.95 -> 0.29).
 //
 // Every loop over the union-find forest is bounded: labels strictly decrease
 // along a parent chain, and the loops also stop after a fixed iteration count,
 // setting an error bit the host turns into FC_LBM_ERR_CUDA.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <chrono>
 #include <climits>
 #include <cmath>
@@ -54,7 +62,9 @@ namespace {
 
 constexpr int kTile = 8;                    // raster tile edge (cells)
 constexpr int kTileCells = kTile * kTile * kTile;
-constexpr int kTriWords = 18;               // a[3] b[3] c[3] n[3] lo[3] hi[3]
+constexpr int kTileRows = kTile * kTile;    // 8-cell x rows of a tile
+constexpr int kTileNodes = kTileRows * kTile / 2;  // runs an occupied tile can hold
+constexpr int kTriWords = 20;               // a[3] b[3] c[3] n[3] lo[3] hi[3] pad[2]
 constexpr int kBoundsBlocks = 148;
 constexpr int kBoundsThreads = 256;
 constexpr unsigned kMaxFindHops = 1u << 26;
@@ -63,9 +73,10 @@ constexpr int kWaitTimeoutMs = 600000;
 constexpr int kErrBadIndex = 1;
 constexpr int kErrUnionBound = 2;
 
-struct Tri {
+struct alignas(16) Tri {  // read as 16-byte vectors
     float a[3], b[3], c[3], n[3];
     int lo[3], hi[3];  // clamped cell box, grid axes (x spans world y, y spans world x)
+    int pad[2];
 };
 static_assert(sizeof(Tri) == kTriWords * 4, "triangle record layout");
 
@@ -203,15 +214,18 @@ struct GridOut {
     float origin[3];
 };
 
-// Voxelizer.cpp:146-166, one thread.
-__global__ void k_grid_final(const Pick* __restrict__ partial, int blocks, int target_res, float padx, float pady,
+// Voxelizer.cpp:146-166: a warp per bound, then one thread.
+constexpr int kGridThreads = 6 * 32;
+__global__ void __launch_bounds__(kGridThreads) k_grid_final(const Pick* __restrict__ partial, int blocks, int target_res, float padx, float pady,
                              float padz, GridOut* out) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    Pick r[6];
-    for (int k = 0; k < 6; ++k) {
-        r[k] = partial[k];
-        for (int b = 1; b < blocks; ++b) r[k] = k < 3 ? pick_min(r[k], partial[b * 6 + k]) : pick_max(r[k], partial[b * 6 + k]);
-    }
+    __shared__ Pick r[6];
+    const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    Pick p = partial[k];
+    for (int b = lane; b < blocks; b += 32) p = k < 3 ? pick_min(p, partial[b * 6 + k]) : pick_max(p, partial[b * 6 + k]);
+    for (int off = 16; off > 0; off >>= 1) p = k < 3 ? pick_min(p, shfl_pick(p, off)) : pick_max(p, shfl_pick(p, off));
+    if (lane == 0) r[k] = p;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
     const V3 mn{r[0].v, r[1].v, r[2].v}, mx{r[3].v, r[4].v, r[5].v};
     const V3 size = vsub(mx, mn);
     const V3 pad{size.x * padx, size.y * pady, size.z * padz};
@@ -241,9 +255,17 @@ struct GridDev {
     float ox, oy, oz;
 };
 
+// Status words of a call: error bits, and the tiles that hold a triangle.
+struct Status {
+    int err;
+    unsigned occupied;
+};
+
+// Also marks every tile a triangle's box touches in `slot` (zeroed) and counts
+// the marked tiles.
 __global__ void k_tri_prep(const float* __restrict__ pos, unsigned nv, const uint32_t* __restrict__ idx,
                            unsigned ntri, GridDev g, Tri* __restrict__ tris, unsigned long long* __restrict__ counts,
-                           int* __restrict__ err) {
+                           uint32_t* __restrict__ slot, Status* __restrict__ st) {
     const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t > ntri) return;
     if (t == ntri) {  // the scan's trailing slot, so offsets[ntri] is the pair total
@@ -252,7 +274,7 @@ __global__ void k_tri_prep(const float* __restrict__ pos, unsigned nv, const uin
     }
     const uint32_t i0 = idx[3 * (size_t)t], i1 = idx[3 * (size_t)t + 1], i2 = idx[3 * (size_t)t + 2];
     if (i0 >= nv || i1 >= nv || i2 >= nv) {
-        atomicOr(err, kErrBadIndex);
+        atomicOr(&st->err, kErrBadIndex);
         counts[t] = 0;
         return;
     }
@@ -261,7 +283,7 @@ __global__ void k_tri_prep(const float* __restrict__ pos, unsigned nv, const uin
     const V3 c{pos[3 * (size_t)i2], pos[3 * (size_t)i2 + 1], pos[3 * (size_t)i2 + 2]};
     const V3 rn = vcross(vsub(b, a), vsub(c, a));
     const float nl = vlen(rn);
-    Tri r;
+    Tri r{};
     r.a[0] = a.x, r.a[1] = a.y, r.a[2] = a.z;
     r.b[0] = b.x, r.b[1] = b.y, r.b[2] = b.z;
     r.c[0] = c.x, r.c[1] = c.y, r.c[2] = c.z;
@@ -289,9 +311,18 @@ __global__ void k_tri_prep(const float* __restrict__ pos, unsigned nv, const uin
         hi2 = hi2 > g.nz - 1 ? g.nz - 1 : hi2;
         r.lo[0] = lo0, r.lo[1] = lo1, r.lo[2] = lo2;
         r.hi[0] = hi0, r.hi[1] = hi1, r.hi[2] = hi2;
-        if (lo0 <= hi0 && lo1 <= hi1 && lo2 <= hi2)
+        if (lo0 <= hi0 && lo1 <= hi1 && lo2 <= hi2) {
             cnt = (unsigned long long)(hi0 / kTile - lo0 / kTile + 1) * (hi1 / kTile - lo1 / kTile + 1) *
                   (hi2 / kTile - lo2 / kTile + 1);
+            unsigned fresh = 0;
+            for (int z = lo2 / kTile; z <= hi2 / kTile; ++z)
+                for (int y = lo1 / kTile; y <= hi1 / kTile; ++y)
+                    for (int x = lo0 / kTile; x <= hi0 / kTile; ++x) {
+                        uint32_t* m = slot + (((size_t)z * g.ty + y) * g.tx + x);
+                        if (__ldcg(m) == 0u && atomicExch(m, 1u) == 0u) ++fresh;
+                    }
+            if (fresh) atomicAdd(&st->occupied, fresh);
+        }
     }
     tris[t] = r;
     counts[t] = cnt;
@@ -319,82 +350,200 @@ __global__ void k_tri_emit(const Tri* __restrict__ tris, const unsigned long lon
 
 // ---- 3. raster ----
 
-__global__ void k_vox_init(uint8_t* __restrict__ solid, float* __restrict__ sdf, size_t n) {
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        solid[i] = 0;
-        sdf[i] = INFINITY;
-    }
+// slot[tile] = its place in the list of occupied tiles + 1 (0: no triangle)
+__global__ void k_tile_slots(const uint32_t* __restrict__ run_tile, unsigned runs, uint32_t* __restrict__ slot) {
+    const unsigned k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < runs) slot[run_tile[k]] = k + 1u;
 }
 
-__global__ void __launch_bounds__(kTileCells) k_vox_raster(const Tri* __restrict__ tris,
-                                                          const uint32_t* __restrict__ tile_tris,
-                                                          const uint32_t* __restrict__ run_tile,
-                                                          const uint32_t* __restrict__ run_len,
-                                                          const unsigned long long* __restrict__ run_off, GridDev g,
-                                                          uint8_t* __restrict__ solid, float* __restrict__ sdf) {
-    __shared__ Tri s_tri[kTileCells];
-    const uint32_t tile = run_tile[blockIdx.x];
-    const unsigned count = run_len[blockIdx.x];
-    const unsigned long long first = run_off[blockIdx.x];
-    const int tx = (int)(tile % (uint32_t)g.tx);
-    const int ty = (int)((tile / (uint32_t)g.tx) % (uint32_t)g.ty);
-    const int tz = (int)(tile / ((uint32_t)g.tx * (uint32_t)g.ty));
-    const int x = tx * kTile + (threadIdx.x & 7);
-    const int y = ty * kTile + ((threadIdx.x >> 3) & 7);
-    const int z = tz * kTile + (threadIdx.x >> 6);
+// Block 16k + w: box w (4x4x2 cells, one per lane) of occupied tile k. The
+// list order matters only to the running state, not to a triangle's distance
+// from a cell, so all threads compute the distances of a chunk of the box's
+// triangles at once, one (triangle, cell) pair each, for the cells inside the
+// triangle's own box only; warp 0 then applies the update rule to them in
+// order. A list can be long (thousands of triangles where a mesh comes to a
+// point), and a triangle's box covers a fifth of the cells of the boxes it
+// overlaps. The 57,516-triangle aircraft on 31M cells, B200: one triangle after
+// another per cell 0.78 ms, a triangle per warp 0.35 ms, a pair per thread in
+// blocks of 256 0.29 ms (of 512 0.35). What is left is latency: a block's
+// chain of list, box and triangle loads, at 46 % of the warp slots and 35 % of
+// the issue slots; a branch-free closest_on_triangle measured the same. Also
+// writes the fluid bits of the box's rows, which the flood fill runs on.
+constexpr int kRasterThreads = 256;
+constexpr int kRasterWarps = kRasterThreads / 32;
+constexpr int kRasterChunk = 64;  // distances kept at a time
+constexpr int kTileBoxes = kTileCells / 32;
+__global__ void __launch_bounds__(kRasterThreads) k_vox_raster(const Tri* __restrict__ tris,
+                                                               const uint32_t* __restrict__ tile_tris,
+                                                               const uint32_t* __restrict__ run_tile,
+                                                               const uint32_t* __restrict__ run_len,
+                                                               const unsigned long long* __restrict__ run_off,
+                                                               GridDev g, uint8_t* __restrict__ solid,
+                                                               float* __restrict__ sdf, uint8_t* __restrict__ mask) {
+    __shared__ uint32_t s_hit[kRasterThreads];
+    __shared__ float2 s_res[kRasterChunk][32];  // distance and signed normal projection; NaN: outside the box
+    __shared__ unsigned s_count[kRasterWarps];
+    // the chunk's triangles: their cells of the box (first cell and size per
+    // axis) and the pairs up to and including each
+    __shared__ uint32_t s_clip[kRasterChunk], s_pairs[kRasterChunk], s_part[kRasterChunk / 32];
+    const unsigned k = blockIdx.x / kTileBoxes, w = blockIdx.x % kTileBoxes;
+    const uint32_t tile = run_tile[k];
+    const unsigned count = run_len[k];
+    const uint32_t* list = tile_tris + run_off[k];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // the block's box, and this lane's cell in it
+    const int lx = (w & 1) * 4, ly = ((w >> 1) & 1) * 4, lz = (w >> 2) * 2;
+    const int bx = (int)(tile % (uint32_t)g.tx) * kTile + lx;
+    const int by = (int)((tile / (uint32_t)g.tx) % (uint32_t)g.ty) * kTile + ly;
+    const int bz = (int)(tile / ((uint32_t)g.tx * (uint32_t)g.ty)) * kTile + lz;
+    const int x = bx + (lane & 3), y = by + ((lane >> 2) & 3), z = bz + (lane >> 4);
     const bool inside = x < g.nx && y < g.ny && z < g.nz;
-    // CellCenter: world x from grid y, world y from grid x (VoxelGrid.h:43-56)
-    const V3 ctr{g.ox + ((float)y + 0.5f) * g.cs, g.oy + ((float)x + 0.5f) * g.cs, g.oz + ((float)z + 0.5f) * g.cs};
     const float tie = g.cs * 1e-3f;
     float sd = INFINITY, bp = -1.0f;
     bool sol = false;
-    for (unsigned base = 0; base < count; base += kTileCells) {
-        const unsigned m = count - base < (unsigned)kTileCells ? count - base : (unsigned)kTileCells;
+    const bool empty = bx >= g.nx || by >= g.ny || bz >= g.nz;  // a box behind the grid's edge
+    for (unsigned base = 0; base < count && !empty; base += kRasterThreads) {
+        // the list's next triangles that overlap the box, in list order
+        bool hit = false;
+        uint32_t mine = 0;
+        if (base + threadIdx.x < count) {
+            mine = list[base + threadIdx.x];
+            const int4* r = reinterpret_cast<const int4*>(tris + mine) + 3;
+            const int4 u = __ldg(r), v = __ldg(r + 1);  // lo[0..2] hi[0] | hi[1..2]
+            hit = bx <= u.w && bx + 3 >= u.x && by <= v.x && by + 3 >= u.y && bz <= v.y && bz + 1 >= u.z;
+        }
+        const unsigned hits = __ballot_sync(0xffffffffu, hit);
+        if (lane == 0) s_count[warp] = __popc(hits);
         __syncthreads();
-        if (threadIdx.x < m) s_tri[threadIdx.x] = tris[tile_tris[first + base + threadIdx.x]];
+        unsigned place = 0, m = 0;
+        for (int j = 0; j < kRasterWarps; ++j) {
+            if (j < warp) place += s_count[j];
+            m += s_count[j];
+        }
+        if (hit) s_hit[place + __popc(hits & ((1u << lane) - 1u))] = mine;
         __syncthreads();
-        if (!inside) continue;
-        for (unsigned k = 0; k < m; ++k) {
-            const Tri& r = s_tri[k];
-            if (x < r.lo[0] || x > r.hi[0] || y < r.lo[1] || y > r.hi[1] || z < r.lo[2] || z > r.hi[2]) continue;
-            const V3 a{r.a[0], r.a[1], r.a[2]}, b{r.b[0], r.b[1], r.b[2]}, c{r.c[0], r.c[1], r.c[2]};
-            const V3 un{r.n[0], r.n[1], r.n[2]};
-            const V3 cl = closest_on_triangle(ctr, a, b, c);
-            const V3 diff = vsub(ctr, cl);
-            const float dist = vlen(diff);
-            const float nd = vdot(diff, un);
-            const float and_ = fabsf(nd);
-            const float bd = fabsf(sd);
-            // Voxelizer.cpp:258-290: a clearly nearer triangle replaces the
-            // cell's distance; within the tie tolerance the one whose normal
-            // points more directly at the cell decides the sign
-            if (dist + tie < bd) {
-                sd = nd < 0.0f ? -dist : dist;
-                bp = and_;
-            } else if (dist <= bd + tie) {
-                if (and_ > bp) {
-                    const float md = dist < bd ? dist : bd;
-                    sd = nd < 0.0f ? -md : md;
-                    bp = and_;
-                } else if (dist < bd) {
-                    sd = sd < 0.0f ? -dist : dist;
+        for (unsigned c0 = 0; c0 < m; c0 += kRasterChunk) {
+            const unsigned c1 = c0 + kRasterChunk < m ? c0 + kRasterChunk : m;
+            if (threadIdx.x < kRasterChunk) {
+                unsigned n = 0;
+                if (c0 + threadIdx.x < c1) {
+                    const int4* r = reinterpret_cast<const int4*>(tris + s_hit[c0 + threadIdx.x]) + 3;
+                    const int4 u = __ldg(r), v = __ldg(r + 1);
+                    const int x0 = max(u.x, bx), x1 = min(u.w, bx + 3), y0 = max(u.y, by), y1 = min(v.x, by + 3),
+                              z0 = max(u.z, bz), z1 = min(v.y, bz + 1);
+                    s_clip[threadIdx.x] = (uint32_t)((x0 - bx) | (y0 - by) << 2 | (z0 - bz) << 4 | (x1 - x0) << 5 |
+                                                     (y1 - y0) << 7 | (z1 - z0) << 9);
+                    n = (unsigned)((x1 - x0 + 1) * (y1 - y0 + 1) * (z1 - z0 + 1));
+                }
+                for (int o = 1; o < 32; o <<= 1) {
+                    const unsigned t = __shfl_up_sync(0xffffffffu, n, o);
+                    if (lane >= o) n += t;
+                }
+                s_pairs[threadIdx.x] = n;
+                if (lane == 31) s_part[warp] = n;
+            }
+            for (unsigned r = threadIdx.x; r < (c1 - c0) * 32u; r += kRasterThreads)
+                s_res[r >> 5][r & 31u].x = __int_as_float(0x7fffffff);
+            __syncthreads();
+            if (threadIdx.x < kRasterChunk) {
+                unsigned n = s_pairs[threadIdx.x];
+                for (int j = 0; j < warp; ++j) n += s_part[j];
+                s_pairs[threadIdx.x] = n;
+            }
+            __syncthreads();
+            const unsigned total = s_pairs[kRasterChunk - 1];
+            for (unsigned pr = threadIdx.x; pr < total; pr += kRasterThreads) {
+                unsigned lo = 0, hi = c1 - c0 - 1;  // the first triangle whose pairs pass pr
+                while (lo < hi) {
+                    const unsigned mid = (lo + hi) >> 1;
+                    if (s_pairs[mid] > pr)
+                        hi = mid;
+                    else
+                        lo = mid + 1;
+                }
+                const unsigned first = lo ? s_pairs[lo - 1] : 0u, clip = s_clip[lo];
+                const unsigned wx = ((clip >> 5) & 3u) + 1u, wy = ((clip >> 7) & 3u) + 1u;
+                const unsigned q = pr - first, qy = q / wx, qz = qy / wy;
+                const unsigned cx = (clip & 3u) + q - qy * wx, cy = ((clip >> 2) & 3u) + qy - qz * wy,
+                               cz = ((clip >> 4) & 1u) + qz;
+                // CellCenter: world x from grid y, world y from grid x (VoxelGrid.h:43-56)
+                const V3 at{g.ox + ((float)(by + (int)cy) + 0.5f) * g.cs, g.oy + ((float)(bx + (int)cx) + 0.5f) * g.cs,
+                            g.oz + ((float)(bz + (int)cz) + 0.5f) * g.cs};
+                const float4* r = reinterpret_cast<const float4*>(tris + s_hit[c0 + lo]);
+                const float4 f0 = __ldg(r), f1 = __ldg(r + 1), f2 = __ldg(r + 2);
+                const V3 a{f0.x, f0.y, f0.z}, b{f0.w, f1.x, f1.y}, c{f1.z, f1.w, f2.x};
+                const V3 diff = vsub(at, closest_on_triangle(at, a, b, c));
+                s_res[lo][cx | cy << 2 | cz << 4] = make_float2(vlen(diff), vdot(diff, V3{f2.y, f2.z, f2.w}));
+            }
+            __syncthreads();
+            if (warp == 0) {
+#pragma unroll 4
+                for (unsigned h = c0; h < c1; ++h) {
+                    const float dist = s_res[h - c0][lane].x, nd = s_res[h - c0][lane].y;
+                    const float and_ = fabsf(nd);
+                    const float bd = fabsf(sd);
+                    // Voxelizer.cpp:258-290: a clearly nearer triangle replaces the
+                    // cell's distance; within the tie tolerance the one whose normal
+                    // points more directly at the cell decides the sign
+                    if (dist + tie < bd) {
+                        sd = nd < 0.0f ? -dist : dist;
+                        bp = and_;
+                    } else if (dist <= bd + tie) {
+                        if (and_ > bp) {
+                            const float md = dist < bd ? dist : bd;
+                            sd = nd < 0.0f ? -md : md;
+                            bp = and_;
+                        } else if (dist < bd) {
+                            sd = sd < 0.0f ? -dist : dist;
+                        }
+                    }
+                    if (dist <= g.cr) sol = true;
                 }
             }
-            if (dist <= g.cr) sol = true;
+            __syncthreads();
         }
     }
+    if (warp != 0) return;
+    const unsigned fluid = __ballot_sync(0xffffffffu, inside && !sol);
     if (inside) {
         const size_t i = ((size_t)z * g.ny + y) * g.nx + x;
         solid[i] = sol ? 1 : 0;
         sdf[i] = sd;
     }
+    if (lane < 8)  // row (y, z) of the box: four bits
+        mask[((size_t)k * kTileRows + (lz + (lane >> 2)) * kTile + ly + (lane & 3)) * 2 + (w & 1)] =
+            (uint8_t)((fluid >> (4 * lane)) & 0xfu);
 }
 
-// ---- 4. flood fill (connected components of fluid cells) ----
+// ---- 4. flood fill (connected components of fluid nodes) ----
 
-__device__ __forceinline__ uint32_t find_root(const uint32_t* __restrict__ L, uint32_t a, int* err) {
+// Node ids: a tile without triangles is its tile index; the run of fluid
+// cells that starts at bit b of row r of occupied tile k is ntiles +
+// kTileNodes k + 4 r + b / 2 (two runs of a row are at least two bits apart).
+// Id is 32 bits wherever the ids fit.
+template <class Id>
+struct Flood {
+    int tx, ty, tz;
+    Id ntiles;
+    const uint32_t* slot;
+    const uint8_t* mask;  // fluid bits of the occupied tiles' rows: a byte per four cells
+    Id* L;
+    int* err;
+    __device__ __forceinline__ Id run(uint32_t slot1, int row, unsigned m, int bit) const {
+        const unsigned starts = m & ~(m << 1);
+        const int b = 31 - __clz(starts & ((2u << bit) - 1u));
+        return ntiles + (Id)(slot1 - 1u) * kTileNodes + (Id)(row * (kTile / 2) + (b >> 1));
+    }
+    __device__ __forceinline__ unsigned row_mask(uint32_t slot1, int row) const {
+        const unsigned v = reinterpret_cast<const uint16_t*>(mask)[(size_t)(slot1 - 1u) * kTileRows + row];
+        return (v & 0xfu) | (v >> 4);
+    }
+};
+
+template <class Id>
+__device__ __forceinline__ Id find_root(const Id* __restrict__ L, Id a, int* err) {
     for (unsigned hop = 0; hop < kMaxFindHops; ++hop) {
-        const uint32_t p = __ldcg(L + a);
+        const Id p = __ldcg(L + a);
         if (p == a) return a;
         a = p;
     }
@@ -402,17 +551,18 @@ __device__ __forceinline__ uint32_t find_root(const uint32_t* __restrict__ L, ui
     return a;
 }
 
-__device__ void unite(uint32_t* L, uint32_t a, uint32_t b, int* err) {
+template <class Id>
+__device__ void unite(Id* L, Id a, Id b, int* err) {
     for (int it = 0; it < kMaxMergeRetries; ++it) {
         a = find_root(L, a, err);
         b = find_root(L, b, err);
         if (a == b) return;
         if (a < b) {
-            const uint32_t old = atomicMin(L + b, a);
+            const Id old = atomicMin(L + b, a);
             if (old == b) return;
             b = old;
         } else {
-            const uint32_t old = atomicMin(L + a, b);
+            const Id old = atomicMin(L + a, b);
             if (old == a) return;
             a = old;
         }
@@ -420,83 +570,172 @@ __device__ void unite(uint32_t* L, uint32_t a, uint32_t b, int* err) {
     atomicOr(err, kErrUnionBound);
 }
 
-// One warp per 32-cell segment of an x row; segments never straddle rows.
-struct SegPos {
-    size_t row;  // z * ny + y
-    int x, y, z;
-    bool valid;
-};
-
-__device__ __forceinline__ SegPos seg_pos(int nx, int ny, int nz, int wpr) {
-    const size_t warp = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    SegPos s;
-    const size_t row = warp / (size_t)wpr;
-    s.row = row;
-    s.x = (int)(warp % (size_t)wpr) * 32 + lane;
-    s.y = (int)(row % (size_t)ny);
-    s.z = (int)(row / (size_t)ny);
-    s.valid = s.z < nz;
-    return s;
+// Labels: one thread per tile row gives each empty tile the first tile of its
+// x-run of empty tiles; the runs of occupied tiles label themselves.
+template <class Id>
+__global__ void k_ff_label(Flood<Id> f, unsigned occupied) {
+    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const size_t step = (size_t)gridDim.x * blockDim.x;
+    for (size_t row = t; row < (size_t)f.ty * f.tz; row += step) {
+        Id start = 0;
+        bool open = false;
+        for (int x = 0; x < f.tx; ++x) {
+            const Id i = (Id)(row * f.tx + x);
+            const bool empty = f.slot[i] == 0u;
+            if (empty && !open) start = i;
+            open = empty;
+            f.L[i] = empty ? start : i;
+        }
+    }
+    for (size_t k = t; k < (size_t)occupied * kTileNodes; k += step) f.L[f.ntiles + k] = (Id)(f.ntiles + k);
 }
 
-__global__ void k_ff_init(const uint8_t* __restrict__ solid, uint32_t* __restrict__ L, int nx, int ny, int nz,
-                          int wpr) {
-    const SegPos s = seg_pos(nx, ny, nz, wpr);
-    if (!s.valid) return;  // warp-uniform
-    const int lane = threadIdx.x & 31;
-    const size_t i = s.row * nx + s.x;
-    const bool fl = s.x < nx && !solid[i];
-    const unsigned F = __ballot_sync(0xffffffffu, fl);
-    const unsigned starts = F & ~(F << 1);
-    if (fl) {
-        const unsigned upto = starts & (0xffffffffu >> (31 - lane));
-        const int start = 31 - __clz(upto);
-        L[i] = (uint32_t)(s.row * nx + (s.x - lane + start));
-    }
+// Joins empty tiles with the row below and the layer below, once per stretch
+// of tiles that are empty on both sides.
+template <class Id>
+__global__ void k_ff_tiles(Flood<Id> f) {
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= (size_t)f.ntiles || f.slot[i] != 0u) return;
+    const int x = (int)(i % f.tx);
+    const size_t row = i / f.tx;
+    const int y = (int)(row % f.ty), z = (int)(row / f.ty);
+    const bool left = x > 0 && f.slot[i - 1] == 0u;
+    auto join = [&](size_t below) {
+        if (f.slot[below] == 0u && !(left && f.slot[below - 1] == 0u)) unite<Id>(f.L, (Id)i, (Id)below, f.err);
+    };
+    if (y > 0) join(i - f.tx);
+    if (z > 0) join(i - (size_t)f.tx * f.ty);
 }
 
-// Joins runs across the segment's left edge and to the row below and the layer
-// below. Within a segment only the first cell of every stretch where both the
-// cell and its neighbour are fluid unites: the rest of the stretch is already
-// in the same runs on both sides.
-__global__ void k_ff_merge(const uint8_t* __restrict__ solid, uint32_t* __restrict__ L, int nx, int ny, int nz,
-                           int wpr, int* __restrict__ err) {
-    const SegPos s = seg_pos(nx, ny, nz, wpr);
-    if (!s.valid) return;
-    const int lane = threadIdx.x & 31;
-    const size_t i = s.row * nx + s.x;
-    const bool in = s.x < nx;
-    const bool fl = in && !solid[i];
-    const unsigned F = __ballot_sync(0xffffffffu, fl);
-    if (lane == 0 && fl && s.x > 0 && !solid[i - 1]) unite(L, (uint32_t)i, (uint32_t)(i - 1), err);
-    if (s.y > 0) {
-        const unsigned B = F & __ballot_sync(0xffffffffu, in && !solid[i - nx]);
-        if ((B & ~(B << 1)) >> lane & 1u) unite(L, (uint32_t)i, (uint32_t)(i - nx), err);
+// Joins the runs of an occupied tile (one thread per row) with those of the
+// row below, the layer below and the tile to the left, and with empty tiles
+// on every side.
+template <class Id>
+__global__ void __launch_bounds__(kTileRows) k_ff_runs(Flood<Id> f, const uint32_t* __restrict__ run_tile) {
+    const uint32_t s1 = blockIdx.x + 1u, tile = run_tile[blockIdx.x];
+    const int row = threadIdx.x, ly = row & (kTile - 1), lz = row / kTile;
+    const unsigned m = f.row_mask(s1, row);
+    if (!m) return;
+    const int x = (int)(tile % (uint32_t)f.tx);
+    const uint32_t tr = tile / (uint32_t)f.tx;
+    const int y = (int)(tr % (uint32_t)f.ty), z = (int)(tr / (uint32_t)f.ty);
+    // this row with row `r2` of the tile `other` (s2 = its slot; 0: empty, all fluid)
+    auto rows = [&](uint32_t other, uint32_t s2, int r2) {
+        const unsigned o = s2 ? f.row_mask(s2, r2) : 0xffu;
+        const unsigned both = m & o;
+        for (unsigned b = both & ~(both << 1); b; b &= b - 1u) {
+            const int bit = __ffs(b) - 1;
+            unite<Id>(f.L, f.run(s1, row, m, bit), s2 ? f.run(s2, r2, o, bit) : (Id)other, f.err);
+        }
+    };
+    const uint32_t dy = (uint32_t)f.tx, dz = (uint32_t)f.tx * (uint32_t)f.ty;
+    if (ly > 0)
+        rows(tile, s1, row - 1);
+    else if (y > 0)
+        rows(tile - dy, f.slot[tile - dy], row + kTile - 1);
+    if (lz > 0)
+        rows(tile, s1, row - kTile);
+    else if (z > 0)
+        rows(tile - dz, f.slot[tile - dz], row + kTileRows - kTile);
+    if (ly == kTile - 1 && y + 1 < f.ty && f.slot[tile + dy] == 0u) rows(tile + dy, 0u, 0);
+    if (lz == kTile - 1 && z + 1 < f.tz && f.slot[tile + dz] == 0u) rows(tile + dz, 0u, 0);
+    if ((m & 1u) && x > 0) {
+        const uint32_t s2 = f.slot[tile - 1];
+        if (!s2) {
+            unite<Id>(f.L, f.run(s1, row, m, 0), (Id)(tile - 1), f.err);
+        } else {
+            const unsigned o = f.row_mask(s2, row);
+            if (o & 0x80u) unite<Id>(f.L, f.run(s1, row, m, 0), f.run(s2, row, o, 7), f.err);
+        }
     }
-    if (s.z > 0) {
-        const size_t layer = (size_t)nx * ny;
-        const unsigned B = F & __ballot_sync(0xffffffffu, in && !solid[i - layer]);
-        if ((B & ~(B << 1)) >> lane & 1u) unite(L, (uint32_t)i, (uint32_t)(i - layer), err);
+    if ((m & 0x80u) && x + 1 < f.tx && f.slot[tile + 1] == 0u)
+        unite<Id>(f.L, f.run(s1, row, m, 7), (Id)(tile + 1), f.err);
+}
+
+// The reached cells: a byte per empty tile, the bits of every row of the
+// occupied tiles. Nothing is reached when cell 0 is solid.
+template <class Id>
+__global__ void k_ff_reached(Flood<Id> f, unsigned occupied, uint8_t* __restrict__ tile_reached,
+                             uint8_t* __restrict__ row_reached) {
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= (size_t)f.ntiles + (size_t)occupied * kTileRows) return;
+    const uint32_t s0 = f.slot[0];
+    const unsigned m0 = s0 ? f.row_mask(s0, 0) : 1u;
+    const bool seed = (m0 & 1u) != 0u;
+    const Id r0 = seed ? find_root<Id>(f.L, s0 ? f.run(s0, 0, m0, 0) : (Id)0, f.err) : (Id)0;
+    if (i < (size_t)f.ntiles) {
+        if (f.slot[i] == 0u) tile_reached[i] = seed && find_root<Id>(f.L, (Id)i, f.err) == r0 ? 1 : 0;
+        return;
     }
+    const size_t k = i - (size_t)f.ntiles;
+    const uint32_t s1 = (uint32_t)(k / kTileRows) + 1u;
+    const int row = (int)(k % kTileRows);
+    const unsigned m = f.row_mask(s1, row);
+    unsigned r = 0;
+    if (seed)
+        for (unsigned b = m & ~(m << 1); b; b &= b - 1u) {
+            const int bit = __ffs(b) - 1;
+            if (find_root<Id>(f.L, f.run(s1, row, m, bit), f.err) == r0)
+                r |= m & ~(m + (1u << bit));  // the run: the carry out of its lowest bit clears it
+        }
+    row_reached[k] = (uint8_t)r;
 }
 
 // ---- 5. finalize ----
 
-__global__ void k_vox_finalize(uint8_t* __restrict__ solid, float* __restrict__ sdf, const uint32_t* __restrict__ L,
-                               size_t n, float cr, int* __restrict__ err) {
-    // cell 0 keeps its class through this pass (fluid there is the root 0 of
-    // its own component), so every thread may read it
-    const bool seed = solid[0] == 0;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        bool s = solid[i] != 0;
-        if (!s) s = !seed || find_root(L, L[i], err) != 0u;
-        const float d = fabsf(sdf[i]);
-        if (!s)
-            sdf[i] = d;
-        else if (d > cr)
-            sdf[i] = -d;
-        solid[i] = s ? 1 : 0;
+// One warp per 128-cell segment of an x row, four cells of one tile per lane
+// (tiles start on multiples of 8). kVec: rows start on four-cell boundaries
+// and the arrays are aligned, so the four cells move as one vector.
+template <bool kVec>
+__global__ void __launch_bounds__(256) k_vox_finalize(uint8_t* __restrict__ solid, float* __restrict__ sdf, GridDev g,
+                                                      const uint32_t* __restrict__ slot,
+                                                      const uint8_t* __restrict__ tile_reached,
+                                                      const uint8_t* __restrict__ row_reached, int segs) {
+    const size_t warp = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const size_t row = warp / (size_t)segs;
+    if (row >= (size_t)g.ny * g.nz) return;
+    const int x = (int)(warp - row * (size_t)segs) * 128 + (int)(threadIdx.x & 31) * 4;
+    if (x >= g.nx) return;
+    const int y = (int)(row % (size_t)g.ny), z = (int)(row / (size_t)g.ny);
+    const size_t tile = ((size_t)(z / kTile) * g.ty + y / kTile) * g.tx + x / kTile;
+    const uint32_t s1 = slot[tile];
+    const size_t i = row * g.nx + x;
+    const int n = g.nx - x < 4 ? g.nx - x : 4;
+    uint8_t s[4];
+    float d[4];
+    if (!s1) {
+        const bool out = tile_reached[tile] != 0;
+        for (int k = 0; k < 4; ++k) {
+            s[k] = out ? 0 : 1;
+            d[k] = out ? INFINITY : -INFINITY;
+        }
+    } else {
+        const unsigned r = row_reached[(size_t)(s1 - 1u) * kTileRows + (z & (kTile - 1)) * kTile + (y & (kTile - 1))] >>
+                           (x & (kTile - 1));
+        if constexpr (kVec) {
+            const uchar4 a = *reinterpret_cast<const uchar4*>(solid + i);
+            const float4 b = *reinterpret_cast<const float4*>(sdf + i);
+            s[0] = a.x, s[1] = a.y, s[2] = a.z, s[3] = a.w;
+            d[0] = b.x, d[1] = b.y, d[2] = b.z, d[3] = b.w;
+        } else {
+            for (int k = 0; k < n; ++k) s[k] = solid[i + k], d[k] = sdf[i + k];
+        }
+        for (int k = 0; k < 4; ++k) {
+            if (!kVec && k >= n) break;
+            const bool so = s[k] != 0 || !((r >> k) & 1u);
+            const float a = fabsf(d[k]);
+            if (!so)
+                d[k] = a;
+            else if (a > g.cr)
+                d[k] = -a;
+            s[k] = so ? 1 : 0;
+        }
+    }
+    if constexpr (kVec) {
+        *reinterpret_cast<uchar4*>(solid + i) = make_uchar4(s[0], s[1], s[2], s[3]);
+        *reinterpret_cast<float4*>(sdf + i) = make_float4(d[0], d[1], d[2], d[3]);
+    } else {
+        for (int k = 0; k < n; ++k) solid[i + k] = s[k], sdf[i + k] = d[k];
     }
 }
 
@@ -530,22 +769,45 @@ int wait_on(cudaStream_t s) {
     return rc;
 }
 
+// One array of a combined allocation.
+struct Part {
+    void** p;
+    size_t bytes;
+    template <class T>
+    Part(T** q, size_t count) : p(reinterpret_cast<void**>(q)), bytes(count * sizeof(T)) {}
+    Part(void** q, size_t b) : p(q), bytes(b) {}
+};
+
 // Stream-ordered scratch allocations, freed together on the same stream when
 // the call returns (every path that hands results back has waited first).
 struct Scratch {
     cudaStream_t s;
-    void* ptrs[24] = {};
+    void* ptrs[8] = {};
     int n = 0;
     explicit Scratch(cudaStream_t st) : s(st) {}
     template <class T>
     cudaError_t get(T** p, size_t bytes) {
         *p = nullptr;
-        if (n >= 24) return cudaErrorInvalidValue;
+        if (n >= 8) return cudaErrorInvalidValue;
         void* q = nullptr;
         const cudaError_t e = cudaMallocAsync(&q, bytes ? bytes : 16, s);
         if (e != cudaSuccess) return e;
         ptrs[n++] = q;
         *p = static_cast<T*>(q);
+        return cudaSuccess;
+    }
+    // Several arrays in one allocation, each on a 256-byte boundary: the calls
+    // in a pipeline of short kernels are host time that the device waits for.
+    cudaError_t get_all(std::initializer_list<Part> parts) {
+        size_t total = 0;
+        for (const Part& p : parts) total += (p.bytes + 255) / 256 * 256;
+        char* base = nullptr;
+        const cudaError_t e = get(&base, total);
+        if (e != cudaSuccess) return e;
+        for (const Part& p : parts) {
+            *p.p = base;
+            base += (p.bytes + 255) / 256 * 256;
+        }
         return cudaSuccess;
     }
     ~Scratch() {
@@ -585,7 +847,7 @@ int grid_on_device(const float* d_pos, size_t nv, const fc_voxel_params* p, cuda
     VX_TRY(sc.get(&d_out, sizeof(GridOut)));
     k_bounds_partial<<<kBoundsBlocks, kBoundsThreads, 0, s>>>(d_pos, (unsigned)nv, partial);
     VX_TRY(cudaGetLastError());
-    k_grid_final<<<1, 32, 0, s>>>(partial, kBoundsBlocks, p->target_resolution, p->padding[0], p->padding[1],
+    k_grid_final<<<1, kGridThreads, 0, s>>>(partial, kBoundsBlocks, p->target_resolution, p->padding[0], p->padding[1],
                                   p->padding[2], d_out);
     VX_TRY(cudaGetLastError());
     VX_TRY(cudaMemcpyAsync(host, d_out, sizeof(GridOut), cudaMemcpyDeviceToHost, s));
@@ -593,11 +855,32 @@ int grid_on_device(const float* d_pos, size_t nv, const fc_voxel_params* p, cuda
     return FC_LBM_OK;
 }
 
+// The flood fill's kernels: labels, joins, reached flags.
+template <class Id>
+int flood(const GridDev& g, uint64_t ntiles, unsigned occupied, const uint32_t* slot, const uint8_t* mask,
+          const uint32_t* run_tile, Id* L, uint8_t* tile_reached, uint8_t* row_reached, Status* st, cudaStream_t s) {
+    const Flood<Id> f{g.tx, g.ty, g.tz, (Id)ntiles, slot, mask, L, &st->err};
+    const uint64_t rows = std::max<uint64_t>((uint64_t)g.ty * g.tz, (uint64_t)occupied * kTileNodes);
+    k_ff_label<Id><<<(unsigned)std::min<uint64_t>((rows + 127) / 128, 148 * 32), 128, 0, s>>>(f, occupied);
+    VX_TRY(cudaGetLastError());
+    const uint64_t tile_blocks = (ntiles + 127) / 128;
+    const uint64_t reach_blocks = (ntiles + (uint64_t)occupied * kTileRows + 127) / 128;
+    if (reach_blocks > (uint64_t)INT32_MAX) return FC_LBM_ERR_TOO_LARGE;
+    k_ff_tiles<Id><<<(unsigned)tile_blocks, 128, 0, s>>>(f);
+    VX_TRY(cudaGetLastError());
+    if (occupied > 0) {
+        k_ff_runs<Id><<<occupied, kTileRows, 0, s>>>(f, run_tile);
+        VX_TRY(cudaGetLastError());
+    }
+    k_ff_reached<Id><<<(unsigned)reach_blocks, 128, 0, s>>>(f, occupied, tile_reached, row_reached);
+    VX_TRY(cudaGetLastError());
+    return FC_LBM_OK;
+}
+
 int voxelize_on_device(const float* d_pos, size_t nv, const uint32_t* d_idx, size_t ni, const int32_t dims[3],
                        float cell_size, const float origin[3], uint8_t* d_solid, float* d_sdf, cudaStream_t s,
                        Scratch& sc) {
     const int nx = dims[0], ny = dims[1], nz = dims[2];
-    const size_t n = (size_t)nx * ny * nz;
     GridDev g;
     g.nx = nx, g.ny = ny, g.nz = nz;
     g.tx = (nx + kTile - 1) / kTile, g.ty = (ny + kTile - 1) / kTile, g.tz = (nz + kTile - 1) / kTile;
@@ -607,94 +890,87 @@ int voxelize_on_device(const float* d_pos, size_t nv, const uint32_t* d_idx, siz
     const unsigned ntri = (unsigned)(ni / 3);
     const uint64_t ntiles = (uint64_t)g.tx * g.ty * g.tz;
 
-    int* d_err = nullptr;
-    VX_TRY(sc.get(&d_err, sizeof(int)));
-    VX_TRY(cudaMemsetAsync(d_err, 0, sizeof(int), s));
-    const int init_blocks = (int)std::min<size_t>((n + 255) / 256, (size_t)148 * 16);
-    k_vox_init<<<init_blocks, 256, 0, s>>>(d_solid, d_sdf, n);
-    VX_TRY(cudaGetLastError());
-
-    if (ntri > 0) {
-        Tri* tris = nullptr;
-        unsigned long long *counts = nullptr, *offsets = nullptr;
-        VX_TRY(sc.get(&tris, sizeof(Tri) * ntri));
-        VX_TRY(sc.get(&counts, sizeof(unsigned long long) * (ntri + 1)));
-        VX_TRY(sc.get(&offsets, sizeof(unsigned long long) * (ntri + 1)));
-        k_tri_prep<<<(ntri + 1 + 255) / 256, 256, 0, s>>>(d_pos, (unsigned)nv, d_idx, ntri, g, tris, counts, d_err);
-        VX_TRY(cudaGetLastError());
-        size_t tmp_bytes = 0;
+    // the first half: triangle records, tile marks, and the sizes of the rest
+    Status* d_st = nullptr;
+    uint32_t* slot = nullptr;
+    Tri* tris = nullptr;
+    unsigned long long *counts = nullptr, *offsets = nullptr;
+    void* tmp = nullptr;
+    size_t tmp_bytes = 0;
+    if (ntri > 0)
         VX_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, counts, offsets, (int64_t)ntri + 1, s));
-        void* tmp = nullptr;
-        VX_TRY(sc.get(&tmp, tmp_bytes));
+    VX_TRY(sc.get_all({{&d_st, 1}, {&slot, ntiles}, {&tris, ntri}, {&counts, (size_t)ntri + 1},
+                       {&offsets, (size_t)ntri + 1}, {&tmp, tmp_bytes}}));
+    VX_TRY(cudaMemsetAsync(d_st, 0, sizeof(Status), s));
+    VX_TRY(cudaMemsetAsync(slot, 0, sizeof(uint32_t) * ntiles, s));
+    Status st{};
+    unsigned long long pairs = 0;
+    if (ntri > 0) {
+        k_tri_prep<<<(ntri + 1 + 255) / 256, 256, 0, s>>>(d_pos, (unsigned)nv, d_idx, ntri, g, tris, counts, slot,
+                                                          d_st);
+        VX_TRY(cudaGetLastError());
         VX_TRY(cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, counts, offsets, (int64_t)ntri + 1, s));
-        unsigned long long pairs = 0;
-        int herr = 0;
         VX_TRY(cudaMemcpyAsync(&pairs, offsets + ntri, sizeof(pairs), cudaMemcpyDeviceToHost, s));
-        VX_TRY(cudaMemcpyAsync(&herr, d_err, sizeof(int), cudaMemcpyDeviceToHost, s));
+        VX_TRY(cudaMemcpyAsync(&st, d_st, sizeof(st), cudaMemcpyDeviceToHost, s));
         VX_RC(wait_on(s));
-        if (herr & kErrBadIndex) return FC_LBM_ERR_INVALID_ARG;
+        if (st.err & kErrBadIndex) return FC_LBM_ERR_INVALID_ARG;
         if (pairs > (unsigned long long)INT32_MAX) return FC_LBM_ERR_TOO_LARGE;
-        if (pairs > 0) {
-            uint32_t *k0, *k1, *v0, *v1, *run_tile, *run_len;
-            unsigned long long* run_off = nullptr;
-            int* d_runs = nullptr;
-            VX_TRY(sc.get(&k0, 4 * pairs));
-            VX_TRY(sc.get(&k1, 4 * pairs));
-            VX_TRY(sc.get(&v0, 4 * pairs));
-            VX_TRY(sc.get(&v1, 4 * pairs));
-            k_tri_emit<<<(ntri + 255) / 256, 256, 0, s>>>(tris, offsets, ntri, g, k0, v0);
-            VX_TRY(cudaGetLastError());
-            cub::DoubleBuffer<uint32_t> kb(k0, k1), vb(v0, v1);
-            const int end_bit = bits_for(ntiles);
-            size_t sort_bytes = 0;
-            VX_TRY(cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, kb, vb, (int)pairs, 0, end_bit, s));
-            void* sort_tmp = nullptr;
-            VX_TRY(sc.get(&sort_tmp, sort_bytes));
-            VX_TRY(cub::DeviceRadixSort::SortPairs(sort_tmp, sort_bytes, kb, vb, (int)pairs, 0, end_bit, s));
-            const uint64_t max_runs = std::min<uint64_t>(pairs, ntiles);
-            VX_TRY(sc.get(&run_tile, 4 * max_runs));
-            VX_TRY(sc.get(&run_len, 4 * max_runs));
-            VX_TRY(sc.get(&run_off, 8 * max_runs));
-            VX_TRY(sc.get(&d_runs, sizeof(int)));
-            size_t rle_bytes = 0;
-            VX_TRY(cub::DeviceRunLengthEncode::Encode(nullptr, rle_bytes, kb.Current(), run_tile, run_len, d_runs,
-                                                       (int)pairs, s));
-            void* rle_tmp = nullptr;
-            VX_TRY(sc.get(&rle_tmp, rle_bytes));
-            VX_TRY(cub::DeviceRunLengthEncode::Encode(rle_tmp, rle_bytes, kb.Current(), run_tile, run_len, d_runs,
-                                                       (int)pairs, s));
-            int runs = 0;
-            VX_TRY(cudaMemcpyAsync(&runs, d_runs, sizeof(int), cudaMemcpyDeviceToHost, s));
-            VX_RC(wait_on(s));
-            size_t scan2 = 0;
-            VX_TRY(cub::DeviceScan::ExclusiveSum(nullptr, scan2, run_len, run_off, (int64_t)runs, s));
-            void* scan2_tmp = nullptr;
-            VX_TRY(sc.get(&scan2_tmp, scan2));
-            VX_TRY(cub::DeviceScan::ExclusiveSum(scan2_tmp, scan2, run_len, run_off, (int64_t)runs, s));
-            if (runs > 0) {
-                k_vox_raster<<<runs, kTileCells, 0, s>>>(tris, vb.Current(), run_tile, run_len, run_off, g, d_solid,
-                                                         d_sdf);
-                VX_TRY(cudaGetLastError());
-            }
-        }
     }
-
-    uint32_t* L = nullptr;
-    VX_TRY(sc.get(&L, sizeof(uint32_t) * n));
-    const int wpr = (nx + 31) / 32;
-    const size_t segs = (size_t)wpr * ny * nz;
-    const size_t ff_blocks = (segs * 32 + 255) / 256;
-    if (ff_blocks > (size_t)INT32_MAX) return FC_LBM_ERR_TOO_LARGE;
-    k_ff_init<<<(unsigned)ff_blocks, 256, 0, s>>>(d_solid, L, nx, ny, nz, wpr);
+    // the second half: the tiles' triangle lists and the flood fill's nodes
+    const unsigned runs = st.occupied;  // the runs of equal tile ids after the sort
+    if (runs > (unsigned)INT32_MAX / kTileBoxes) return FC_LBM_ERR_TOO_LARGE;
+    const uint64_t nodes = ntiles + (uint64_t)runs * kTileNodes;
+    const bool wide = nodes >= 0xffffffffull;
+    uint32_t *k0 = nullptr, *k1 = nullptr, *v0 = nullptr, *v1 = nullptr, *run_tile = nullptr, *run_len = nullptr;
+    unsigned long long* run_off = nullptr;
+    int* d_runs = nullptr;
+    uint8_t *mask = nullptr, *tile_reached = nullptr, *row_reached = nullptr;
+    char* labels = nullptr;
+    size_t sort_bytes = 0, rle_bytes = 0, scan_bytes = 0;
+    const int end_bit = bits_for(ntiles);
+    if (pairs > 0) {
+        cub::DoubleBuffer<uint32_t> kb(k0, k1), vb(v0, v1);
+        VX_TRY(cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, kb, vb, (int)pairs, 0, end_bit, s));
+        VX_TRY(cub::DeviceRunLengthEncode::Encode(nullptr, rle_bytes, k0, run_tile, run_len, d_runs, (int)pairs, s));
+        VX_TRY(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, run_len, run_off, (int64_t)runs, s));
+    }
+    VX_TRY(sc.get_all({{&k0, pairs}, {&k1, pairs}, {&v0, pairs}, {&v1, pairs}, {&run_tile, runs}, {&run_len, runs},
+                       {&run_off, runs}, {&d_runs, 1}, {&mask, (size_t)runs * kTileRows * 2}, {&tile_reached, ntiles},
+                       {&row_reached, (size_t)runs * kTileRows}, {&labels, nodes * (wide ? 8 : 4)},
+                       {&tmp, std::max(sort_bytes, std::max(rle_bytes, scan_bytes))}}));
+    if (pairs > 0) {
+        k_tri_emit<<<(ntri + 255) / 256, 256, 0, s>>>(tris, offsets, ntri, g, k0, v0);
+        VX_TRY(cudaGetLastError());
+        cub::DoubleBuffer<uint32_t> kb(k0, k1), vb(v0, v1);
+        VX_TRY(cub::DeviceRadixSort::SortPairs(tmp, sort_bytes, kb, vb, (int)pairs, 0, end_bit, s));
+        VX_TRY(cub::DeviceRunLengthEncode::Encode(tmp, rle_bytes, kb.Current(), run_tile, run_len, d_runs, (int)pairs,
+                                                   s));
+        VX_TRY(cub::DeviceScan::ExclusiveSum(tmp, scan_bytes, run_len, run_off, (int64_t)runs, s));
+        k_tile_slots<<<(runs + 255) / 256, 256, 0, s>>>(run_tile, runs, slot);
+        VX_TRY(cudaGetLastError());
+        k_vox_raster<<<kTileBoxes * runs, kRasterThreads, 0, s>>>(tris, vb.Current(), run_tile, run_len, run_off, g,
+                                                                  d_solid, d_sdf, mask);
+        VX_TRY(cudaGetLastError());
+    }
+    VX_RC(wide ? flood(g, ntiles, runs, slot, mask, run_tile, reinterpret_cast<unsigned long long*>(labels),
+                       tile_reached, row_reached, d_st, s)
+               : flood(g, ntiles, runs, slot, mask, run_tile, reinterpret_cast<uint32_t*>(labels), tile_reached,
+                       row_reached, d_st, s));
+    const int segs = (nx + 127) / 128;
+    const size_t fin_blocks = ((size_t)segs * ny * nz * 32 + 255) / 256;
+    if (fin_blocks > (size_t)INT32_MAX) return FC_LBM_ERR_TOO_LARGE;
+    const bool vec = nx % 4 == 0 && reinterpret_cast<uintptr_t>(d_solid) % 4 == 0 &&
+                     reinterpret_cast<uintptr_t>(d_sdf) % 16 == 0;
+    if (vec)
+        k_vox_finalize<true><<<(unsigned)fin_blocks, 256, 0, s>>>(d_solid, d_sdf, g, slot, tile_reached, row_reached,
+                                                                  segs);
+    else
+        k_vox_finalize<false><<<(unsigned)fin_blocks, 256, 0, s>>>(d_solid, d_sdf, g, slot, tile_reached, row_reached,
+                                                                   segs);
     VX_TRY(cudaGetLastError());
-    k_ff_merge<<<(unsigned)ff_blocks, 256, 0, s>>>(d_solid, L, nx, ny, nz, wpr, d_err);
-    VX_TRY(cudaGetLastError());
-    k_vox_finalize<<<init_blocks, 256, 0, s>>>(d_solid, d_sdf, L, n, g.cr, d_err);
-    VX_TRY(cudaGetLastError());
-    int herr = 0;
-    VX_TRY(cudaMemcpyAsync(&herr, d_err, sizeof(int), cudaMemcpyDeviceToHost, s));
+    VX_TRY(cudaMemcpyAsync(&st, d_st, sizeof(st), cudaMemcpyDeviceToHost, s));
     VX_RC(wait_on(s));
-    return herr ? FC_LBM_ERR_CUDA : FC_LBM_OK;
+    return st.err ? FC_LBM_ERR_CUDA : FC_LBM_OK;
 }
 
 bool finite3(const float* v) { return std::isfinite(v[0]) && std::isfinite(v[1]) && std::isfinite(v[2]); }
