@@ -14,6 +14,7 @@
 
 #include "aa.cuh"
 #include "collide.cuh"
+#include "collide2.cuh"
 #include "fc_lbm.h"
 #include "lbm_internal.h"
 #include "storage.cuh"
@@ -57,19 +58,34 @@ __device__ float bounce_rt(const typename S::T* __restrict__ f, const uint8_t* _
     return inv * plain + (1.0f - inv) * load_at<Q, S, I>(f, ca, ax, ay, az, g, layout);
 }
 
+// The directions to a solid cell's fluid neighbours, their flags loaded
+// together. Most solid cells of a body have none and carry no force.
+template <int Q>
+__device__ __forceinline__ unsigned open_links(const uint8_t* __restrict__ solid, const Geom& g, int x, int y, int z) {
+    using L = Lattice<Q>;
+    unsigned open = 0;
+    static_for<1, Q>([&](auto I) {
+        constexpr int i = decltype(I)::value;
+        const int ax = x + L::ex(i), ay = y + L::ey(i), az = z + L::ez(i);
+        if (inb(g, ax, ay, az) && !solid[cidx(g, ax, ay, az)]) open |= 1u << i;
+    });
+    return open;
+}
+
 template <int Q, class S>
 __device__ float4 solid_force(const typename S::T* __restrict__ f, const uint8_t* __restrict__ solid,
                               const float* __restrict__ sdf, const Geom& g, int x, int y, int z, size_t c,
                               int layout) {
     using L = Lattice<Q>;
     float fx = 0.0f, fy = 0.0f, fz = 0.0f, ws = 0.0f;
+    const unsigned open = open_links<Q>(solid, g, x, y, z);
+    if (!open) return make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     static_for<1, Q>([&](auto I) {
         constexpr int i = decltype(I)::value;
         constexpr int X = L::ex(i), Y = L::ey(i), Z = L::ez(i);
+        if (!((open >> i) & 1u)) return;
         const int ax = x + X, ay = y + Y, az = z + Z;
-        if (!inb(g, ax, ay, az)) return;
         const size_t ca = cidx(g, ax, ay, az);
-        if (solid[ca]) return;
         const float plain = load_at<Q, S, L::opp(i)>(f, ca, ax, ay, az, g, layout);
         const float bounced = bounce_rt<Q, S, i>(f, solid, sdf, g, ax, ay, az, ca, c, layout);
         const float dp = (plain + bounced) - 2.0f * L::w(i);
@@ -260,49 +276,223 @@ __device__ __forceinline__ void stat_block_reduce(StatAcc& acc, double* out) {
     }
 }
 
+// The reductions run over groups of 128 cells, one warp per group, four cells
+// per lane: one 4-byte load of solid flags per lane. The solid cells of a
+// group are listed in shared memory and shared out over the lanes; those with
+// a fluid neighbour, the few that carry a force, collect in a queue of the
+// warp and are evaluated 32 at a time, so that the long force code runs with
+// full warps instead of in the few lanes that hit one. Lane l holds cells 4l
+// .. 4l + 3 of a plane-major group, which lets its populations come four at a
+// time, and cells l, l + 32, ... of an in-place one.
+constexpr int kGroup = 128;
+constexpr int kStatsWarps = kStatsThreads / 32;
+// Resident blocks per SM. The grids stop at one wave of them: each block ends
+// in a barrier and a reduction. (Four k_stats blocks spill: 444 us against 417.)
+constexpr int kStatsPerSm = 3, kAeroPerSm = 2;
+
+__device__ __forceinline__ size_t group_cell(size_t base, int lane, int j, bool planes) {
+    return base + (planes ? 4 * lane + j : lane + 32 * j);
+}
+
+// The flags of this lane's four cells of a group, a byte each (nonzero:
+// solid); cells past the lattice read as fluid. words: `solid` is on a 4-byte
+// boundary.
+__device__ __forceinline__ uint32_t group_word(const uint8_t* __restrict__ solid, size_t base, size_t n, int lane,
+                                               bool planes, bool words) {
+    if (planes && words && base + 4 * lane + 4 <= n)
+        return __ldg(reinterpret_cast<const uint32_t*>(solid + base + 4 * lane));
+    uint32_t w = 0;
+    for (int j = 0; j < 4; ++j) {
+        const size_t c = group_cell(base, lane, j, planes);
+        if (c < n) w |= (uint32_t)solid[c] << (8 * j);
+    }
+    return w;
+}
+
+// Bit j: this lane's j-th cell is solid.
+__device__ __forceinline__ unsigned solid_bits(uint32_t w) {
+    unsigned b = 0;
+    for (int j = 0; j < 4; ++j) b |= ((w >> (8 * j)) & 0xffu) ? 1u << j : 0u;
+    return b;
+}
+
+// Bit j: this lane's j-th cell lies inside the lattice.
+__device__ __forceinline__ unsigned inside_bits(size_t base, size_t n, int lane, bool planes) {
+    if (base + kGroup <= n) return 0xfu;
+    unsigned b = 0;
+    for (int j = 0; j < 4; ++j) b |= group_cell(base, lane, j, planes) < n ? 1u << j : 0u;
+    return b;
+}
+
+__device__ __forceinline__ void cell_xyz(const Geom& g, size_t c, int& x, int& y, int& z) {
+    // cells and layers count below 2^32: 32-bit divisions
+    const uint32_t cc = (uint32_t)c, nxy = (uint32_t)g.nxy, zz = cc / nxy, rem = cc - zz * nxy,
+                   yy = rem / (uint32_t)g.nx;
+    z = (int)zz;
+    y = (int)yy;
+    x = (int)(rem - yy * (uint32_t)g.nx);
+}
+
+// Group of warp w (of W) in its k-th turn, rotated from turn to turn: with a
+// plain stride a warp would meet the same part of every row, and a body would
+// fall to a few warps.
+__device__ __forceinline__ size_t group_base(unsigned w, unsigned W, unsigned k) {
+    return ((size_t)k * W + (w + 37u * (k % W)) % W) * kGroup;
+}
+
+struct SolidLists {
+    uint8_t group[kGroup];   // the group's solid cells, relative to its base
+    uint32_t queue[64];      // solid cells with a fluid neighbour, not evaluated yet
+};
+
+// every(x, y, z) for each solid cell of the group (bits `sol` of this lane),
+// force(cell) for each queued cell once 32 are queued; with `last`, for all.
+template <int Q, class Every, class Force>
+__device__ __forceinline__ void group_solids(SolidLists& sl, unsigned& queued, size_t base, int lane, bool planes,
+                                             unsigned sol, bool last, const uint8_t* __restrict__ solid,
+                                             const Geom& g, Every&& every, Force&& force) {
+    if (!last && !__any_sync(0xffffffffu, sol != 0u)) return;
+    unsigned at = __popc(sol);
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned t = __shfl_up_sync(0xffffffffu, at, o);
+        if (lane >= o) at += t;
+    }
+    const unsigned total = __shfl_sync(0xffffffffu, at, 31);
+    at -= __popc(sol);
+    for (int j = 0; j < 4; ++j)
+        if ((sol >> j) & 1u) sl.group[at++] = (uint8_t)(group_cell(0, lane, j, planes));
+    __syncwarp();
+#pragma unroll 1
+    for (unsigned k = 0; k < total || (last && queued > 0); k += 32) {
+        bool open = false;
+        size_t c = 0;
+        if (k + lane < total) {
+            c = base + sl.group[k + lane];
+            int x, y, z;
+            cell_xyz(g, c, x, y, z);
+            every(x, y, z);
+            open = open_links<Q>(solid, g, x, y, z) != 0u;
+        }
+        const unsigned hits = __ballot_sync(0xffffffffu, open);
+        if (open) sl.queue[queued + __popc(hits & ((1u << lane) - 1u))] = (uint32_t)c;  // below 32 + 32
+        queued += __popc(hits);
+        __syncwarp();
+        if (queued >= 32 || (last && k + 32 >= total)) {
+            if (lane < (int)queued) force((size_t)sl.queue[lane]);
+            const uint32_t rest = sl.queue[32 + lane];
+            __syncwarp();
+            sl.queue[lane] = rest;
+            queued -= queued < 32 ? queued : 32;
+            __syncwarp();
+        }
+    }
+    __syncwarp();
+}
+
+// Four populations of one plane from an address on a four-element boundary,
+// as two pairs.
+template <class S>
+__device__ __forceinline__ void load4(const typename S::T* p, float w, float2& lo, float2& hi) {
+    using T2 = typename S::T2;
+    if constexpr (S::kBytes == 4) {
+        const float4 q = __ldg(reinterpret_cast<const float4*>(p));
+        lo = make_float2(q.x, q.y), hi = make_float2(q.z, q.w);
+    } else {
+        const uint2 q = __ldg(reinterpret_cast<const uint2*>(p));
+        // dec: h / 2^8 + w
+        lo = fma2(S::raw2(*reinterpret_cast<const T2*>(&q.x)), bc2(kOffsetScaleInv), bc2(w));
+        hi = fma2(S::raw2(*reinterpret_cast<const T2*>(&q.y)), bc2(kOffsetScaleInv), bc2(w));
+    }
+}
+
+// B200, 512x256x256 D3Q19 FP16 with a wing: 501 -> 372 us (one cell per thread,
+// 2-byte loads, the force in the lanes that hit a solid cell, before); what is
+// left is arithmetic: the IEEE divisions and roots of four cells per lane.
 template <int Q, class S, int Lay>
-__global__ void __launch_bounds__(kStatsThreads) k_stats(const typename S::T* __restrict__ f,
+__global__ void __launch_bounds__(kStatsThreads, kStatsPerSm) k_stats(const typename S::T* __restrict__ f,
                                                          const uint8_t* __restrict__ solid,
                                                          const float* __restrict__ sdf, Geom g,
-                                                         double* __restrict__ partials, int layout_in) {
+                                                         double* __restrict__ partials, bool words, bool vec) {
+    using L = Lattice<Q>;
     // the layout is a compile-time constant, so every slot folds to its
-    // formula (plane * n + c for plane-major states)
-    const int layout = Lay;
-    (void)layout_in;
+    // formula (plane * stride + c for plane-major states)
+    constexpr bool planes = Lay == kLayoutPlanes;
+    __shared__ SolidLists s_lists[kStatsWarps];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned w = blockIdx.x * kStatsWarps + warp, W = gridDim.x * kStatsWarps;
     StatAcc acc;
-    for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < g.n; c += (size_t)gridDim.x * blockDim.x) {
-        const bool sol = solid[c];
-        // cell coordinates only where they are used: the solid-cell force and
-        // the in-place layouts (the plane-major slot is plane * n + c)
-        int x = 0, y = 0, z = 0;
-        if (sol || layout != kLayoutPlanes) {
-            z = (int)(c / (size_t)g.nxy);
-            const size_t rem = c - (size_t)z * g.nxy;
-            y = (int)(rem / g.nx);
-            x = (int)(rem - (size_t)y * g.nx);
+    unsigned queued = 0;
+    bool last = false;
+    for (unsigned k = 0; !last; ++k) {  // the last turn has no group: it empties the queue
+        last = (size_t)k * W * kGroup >= g.n;
+        const size_t base = group_base(w, W, k);
+        unsigned fluid = 0, sol = 0;
+        if (!last) {
+            sol = solid_bits(group_word(solid, base, g.n, lane, planes, words));
+            fluid = inside_bits(base, g.n, lane, planes) & ~sol;
         }
-        if (sol) {
-            const float4 v = solid_force<Q, S>(f, solid, sdf, g, x, y, z, c, layout);
+        float4 m[4];
+        if (planes && vec && base + kGroup <= g.n) {  // moments<Q> of four cells
+            if (fluid) {
+                const float2 zero = bc2(0.0f);
+                float2 r[2] = {zero, zero}, a[2] = {zero, zero}, b[2] = {zero, zero}, c[2] = {zero, zero};
+                static_for<0, Q>([&](auto I) {
+                    constexpr int i = decltype(I)::value;
+                    constexpr int X = L::ex(i), Y = L::ey(i), Z = L::ez(i);
+                    float2 v[2];
+                    load4<S>(f + (size_t)i * g.ps + base + 4 * lane, L::w(i), v[0], v[1]);
+                    for (int j = 0; j < 2; ++j) {
+                        r[j] = add2(r[j], v[j]);
+                        if constexpr (X > 0) a[j] = add2(a[j], v[j]);
+                        if constexpr (X < 0) a[j] = sub2(a[j], v[j]);
+                        if constexpr (Y > 0) b[j] = add2(b[j], v[j]);
+                        if constexpr (Y < 0) b[j] = sub2(b[j], v[j]);
+                        if constexpr (Z > 0) c[j] = add2(c[j], v[j]);
+                        if constexpr (Z < 0) c[j] = sub2(c[j], v[j]);
+                    }
+                });
+                for (int j = 0; j < 2; ++j) {
+                    if (r[j].x > 1e-6f) a[j].x /= r[j].x, b[j].x /= r[j].x, c[j].x /= r[j].x;
+                    if (r[j].y > 1e-6f) a[j].y /= r[j].y, b[j].y /= r[j].y, c[j].y /= r[j].y;
+                    m[2 * j] = make_float4(r[j].x, a[j].x, b[j].x, c[j].x);
+                    m[2 * j + 1] = make_float4(r[j].y, a[j].y, b[j].y, c[j].y);
+                }
+            }
+        } else {
+            for (int j = 0; j < 4; ++j) {
+                if (!((fluid >> j) & 1u)) continue;
+                const size_t c = group_cell(base, lane, j, planes);
+                int x = 0, y = 0, z = 0;
+                if (!planes) cell_xyz(g, c, x, y, z);
+                m[j] = fluid_moments<Q, S>(f, g, c, x, y, z, Lay);
+            }
+        }
+        for (int j = 0; j < 4; ++j) {
+            if (!((fluid >> j) & 1u)) continue;
+            if (!isfinite(m[j].x) || !isfinite(m[j].y) || !isfinite(m[j].z) || !isfinite(m[j].w)) {
+                acc.nan = 1;
+                continue;
+            }
+            const float sp = sqrtf(speed2(m[j].y, m[j].z, m[j].w));
+            acc.mn = fminf(acc.mn, m[j].x);
+            acc.mx = fmaxf(acc.mx, m[j].x);
+            acc.vmax = fmaxf(acc.vmax, sp);
+            acc.dsum += (double)m[j].x;
+            acc.ssum += (double)sp;
+            acc.count += 1.0;
+        }
+        group_solids<Q>(s_lists[warp], queued, base, lane, planes, sol, last, solid, g, [](int, int, int) {},
+                        [&](size_t c) {
+            int x, y, z;
+            cell_xyz(g, c, x, y, z);
+            const float4 v = solid_force<Q, S>(f, solid, sdf, g, x, y, z, c, Lay);
             if (isfinite(v.x) && isfinite(v.y) && isfinite(v.z) && isfinite(v.w)) {
                 acc.fx += (double)v.y;
                 acc.fy += (double)v.z;
                 acc.fz += (double)v.w;
                 acc.smax = fmaxf(acc.smax, v.x);
             }
-            continue;
-        }
-        const float4 m = fluid_moments<Q, S>(f, g, c, x, y, z, layout);
-        if (!isfinite(m.x) || !isfinite(m.y) || !isfinite(m.z) || !isfinite(m.w)) {
-            acc.nan = 1;
-            continue;
-        }
-        const float sp = sqrtf(speed2(m.y, m.z, m.w));
-        acc.mn = fminf(acc.mn, m.x);
-        acc.mx = fmaxf(acc.mx, m.x);
-        acc.vmax = fmaxf(acc.vmax, sp);
-        acc.dsum += (double)m.x;
-        acc.ssum += (double)sp;
-        acc.count += 1.0;
+        });
     }
     stat_block_reduce(acc, partials + (size_t)blockIdx.x * kStatsSlots);
 }
@@ -371,62 +561,97 @@ __device__ void aero_block_reduce(double* a, double* out) {
     }
 }
 
+// B200, 512x256x256 D3Q19 FP16 with a wing: 392 -> 112 us, and the final kernel 75
+// -> 13 us (one flag per thread and load, the force in the lanes that hit a
+// solid cell, one thread per column of the final patch, before).
 template <int Q, class S, int Lay>
 __global__ void __launch_bounds__(kStatsThreads) k_aero(const typename S::T* __restrict__ f,
                                                         const uint8_t* __restrict__ solid,
                                                         const float* __restrict__ sdf, Geom g, float cs, float ox,
                                                         float oy, float oz, double* __restrict__ partials,
-                                                        int layout_in) {
-    // the layout is a compile-time constant, so every slot folds to its
-    // formula (plane * n + c for plane-major states)
-    const int layout = Lay;
-    (void)layout_in;
+                                                        bool words) {
+    // the layout is a compile-time constant, as in k_stats
+    constexpr bool planes = Lay == kLayoutPlanes;
+    __shared__ SolidLists s_lists[kStatsWarps];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned w = blockIdx.x * kStatsWarps + warp, W = gridDim.x * kStatsWarps;
     double a[kAeroSlots];
     aero_init(a);
-    for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < g.n; c += (size_t)gridDim.x * blockDim.x) {
-        if (!solid[c]) continue;
-        const int z = (int)(c / (size_t)g.nxy);
-        const size_t rem = c - (size_t)z * g.nxy;
-        const int y = (int)(rem / g.nx);
-        const int x = (int)(rem - (size_t)y * g.nx);
-        // VoxelGrid::CellCenter (VoxelGrid.h:53-55) in float
-        const float px = ox + ((float)y + 0.5f) * cs;
-        const float py = oy + ((float)x + 0.5f) * cs;
-        const float pz = oz + ((float)z + 0.5f) * cs;
-        a[kAgx] += (double)px;
-        a[kAgx + 1] += (double)py;
-        a[kAgx + 2] += (double)pz;
-        a[kAcount] += 1.0;
-        a[kAmaxz] = fmax(a[kAmaxz], (double)z);
-        const float4 v = solid_force<Q, S>(f, solid, sdf, g, x, y, z, c, layout);
-        if (!isfinite(v.x) || !isfinite(v.y) || !isfinite(v.z) || !isfinite(v.w)) {
-            a[kAnan] = 1.0;
-            continue;
+    unsigned queued = 0;
+    bool last = false, any = false;
+    // the flags of several groups in one trip to memory: a pass over a lattice
+    // is mostly flags without a solid cell
+    constexpr int kAhead = 4;
+    unsigned rot = w;  // group_base's rotation, stepped
+    size_t from[kAhead];
+    for (unsigned k0 = 0; !last; k0 += kAhead) {  // the last turn has no groups: it empties the queue
+        last = (size_t)k0 * W * kGroup >= g.n;
+        uint32_t flags[kAhead];
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k) {
+            const unsigned r = rot + 37u * k;
+            from[k] = ((size_t)(k0 + k) * W + (r < W ? r : r % W)) * kGroup;
+            flags[k] = last ? 0u : group_word(solid, from[k], g.n, lane, planes, words);
         }
-        a[kAfx] += (double)v.y;
-        a[kAfx + 1] += (double)v.z;
-        a[kAfx + 2] += (double)v.w;
-        const double wl = fabs((double)v.w);
-        a[kAlw] += wl;
-        a[kAlwx] += wl * px;
-        a[kAlwx + 1] += wl * py;
-        a[kAlwx + 2] += wl * pz;
-        const double wf = sqrt((double)v.y * v.y + (double)v.z * v.z + (double)v.w * v.w);
-        a[kAfw] += wf;
-        a[kAfwx] += wf * px;
-        a[kAfwx + 1] += wf * py;
-        a[kAfwx + 2] += wf * pz;
-        if (v.x > 0.0f) {
-            a[kAlo] = fmin(a[kAlo], (double)v.x);
-            a[kAhi] = fmax(a[kAhi], (double)v.x);
+        rot = (rot + 37u * kAhead) % W;
+        if (!last && !__any_sync(0xffffffffu, (flags[0] | flags[1] | flags[2] | flags[3]) != 0u)) continue;
+        any = any || !last;
+        // (one copy of the force code: the group is picked at run time)
+#pragma unroll 1
+        for (int k = 0; k < kAhead; ++k) {
+            const unsigned bits = solid_bits(k == 0 ? flags[0] : (k == 1 ? flags[1] : (k == 2 ? flags[2] : flags[3])));
+            const size_t base = k == 0 ? from[0] : (k == 1 ? from[1] : (k == 2 ? from[2] : from[3]));
+            auto every = [&](int x, int y, int z) {
+                // VoxelGrid::CellCenter (VoxelGrid.h:53-55) in float
+                a[kAgx] += (double)(ox + ((float)y + 0.5f) * cs);
+                a[kAgx + 1] += (double)(oy + ((float)x + 0.5f) * cs);
+                a[kAgx + 2] += (double)(oz + ((float)z + 0.5f) * cs);
+                a[kAcount] += 1.0;
+                a[kAmaxz] = fmax(a[kAmaxz], (double)z);
+            };
+            group_solids<Q>(s_lists[warp], queued, base, lane, planes, bits, last, solid, g, every,
+                            [&](size_t c) {
+                int x, y, z;
+                cell_xyz(g, c, x, y, z);
+                const float px = ox + ((float)y + 0.5f) * cs;
+                const float py = oy + ((float)x + 0.5f) * cs;
+                const float pz = oz + ((float)z + 0.5f) * cs;
+                const float4 v = solid_force<Q, S>(f, solid, sdf, g, x, y, z, c, Lay);
+                if (!isfinite(v.x) || !isfinite(v.y) || !isfinite(v.z) || !isfinite(v.w)) {
+                    a[kAnan] = 1.0;
+                    return;
+                }
+                a[kAfx] += (double)v.y;
+                a[kAfx + 1] += (double)v.z;
+                a[kAfx + 2] += (double)v.w;
+                const double wl = fabs((double)v.w);
+                a[kAlw] += wl;
+                a[kAlwx] += wl * px;
+                a[kAlwx + 1] += wl * py;
+                a[kAlwx + 2] += wl * pz;
+                const double wf = sqrt((double)v.y * v.y + (double)v.z * v.z + (double)v.w * v.w);
+                a[kAfw] += wf;
+                a[kAfwx] += wf * px;
+                a[kAfwx + 1] += wf * py;
+                a[kAfwx + 2] += wf * pz;
+                if (v.x > 0.0f) {
+                    a[kAlo] = fmin(a[kAlo], (double)v.x);
+                    a[kAhi] = fmax(a[kAhi], (double)v.x);
+                }
+            });
         }
     }
-    aero_block_reduce(a, partials + (size_t)blockIdx.x * kAeroSlots);
+    // most blocks meet no solid cell: their partials are the initial values
+    if (__syncthreads_or(any))
+        aero_block_reduce(a, partials + (size_t)blockIdx.x * kAeroSlots);
+    else if (threadIdx.x < 1)
+        for (int k = 0; k < kAeroSlots; ++k) partials[(size_t)blockIdx.x * kAeroSlots + k] = a[k];
 }
 
 // Reduces the partials, then computes the centre of pressure and the lift
 // arrow's base from a 5x5 patch of columns around it (FieldOverlay.cpp:
-// 580-618), one column per thread.
+// 580-618): the highest solid cell of the patch, all its cells over the
+// block's threads.
 __global__ void __launch_bounds__(kStatsThreads) k_aero_final(const double* __restrict__ partials, int blocks,
                                                               const uint8_t* __restrict__ solid, Geom g, float cs,
                                                               float ox, float oy, float oz,
@@ -453,19 +678,21 @@ __global__ void __launch_bounds__(kStatsThreads) k_aero_final(const double* __re
         cp[0] = c0, cp[1] = c1, cp[2] = c2;
     }
     __syncthreads();
-    if (threadIdx.x < 25) {
+    {
         const int nxm = g.nx - 1 > 0 ? g.nx - 1 : 0, nym = g.ny - 1 > 0 ? g.ny - 1 : 0;
         int gx = (int)floorf((cp[1] - oy) / cs), gy = (int)floorf((cp[0] - ox) / cs);
         gx = gx < 0 ? 0 : (gx > nxm ? nxm : gx);
         gy = gy < 0 ? 0 : (gy > nym ? nym : gy);
-        int x = gx + (int)(threadIdx.x % 5) - 2, y = gy + (int)(threadIdx.x / 5) - 2;
-        x = x < 0 ? 0 : (x > nxm ? nxm : x);
-        y = y < 0 ? 0 : (y > nym ? nym : y);
-        for (int z = g.nz - 1; z >= 0; --z)
-            if (solid[((size_t)z * g.ny + y) * g.nx + x]) {
-                atomicMax(&col_top, z);
-                break;
-            }
+        int top = -1;
+#pragma unroll 8
+        for (int k = threadIdx.x; k < 25 * g.nz; k += kStatsThreads) {
+            const int z = k / 25, col = k - 25 * z;
+            int x = gx + col % 5 - 2, y = gy + col / 5 - 2;
+            x = x < 0 ? 0 : (x > nxm ? nxm : x);
+            y = y < 0 ? 0 : (y > nym ? nym : y);
+            if (solid[((size_t)z * g.ny + y) * g.nx + x]) top = z;
+        }
+        if (top >= 0) atomicMax(&col_top, top);
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -497,6 +724,8 @@ __global__ void __launch_bounds__(kStatsThreads) k_aero_final(const double* __re
         result[15] = (double)maxz;
     }
 }
+
+static bool words_of(const uint8_t* solid) { return reinterpret_cast<uintptr_t>(solid) % 4 == 0; }
 
 int stats_blocks(const Geom& g) {
     const size_t want = (g.n + kStatsThreads * 8 - 1) / (kStatsThreads * 8);
@@ -553,7 +782,12 @@ static cudaError_t pops_in_t(void* f, const Geom& g, size_t cell0, size_t cells,
 template <int Q, class S>
 static cudaError_t stats_t(const void* f, const uint8_t* solid, const float* sdf, const Geom& g, double* partials,
                            int blocks, double* result, int layout, cudaStream_t s) {
-    FC_LAYOUT_LAUNCH(k_stats, blocks, kStatsThreads, (const typename S::T*)f, solid, sdf, g, partials, layout);
+    // four populations at a time where every plane and cell group starts on
+    // such a boundary
+    blocks = blocks < kStatsPerSm * 148 ? blocks : kStatsPerSm * 148;
+    const bool vec = g.ps % 4 == 0 && reinterpret_cast<uintptr_t>(f) % (4 * S::kBytes) == 0;
+    FC_LAYOUT_LAUNCH(k_stats, blocks, kStatsThreads, (const typename S::T*)f, solid, sdf, g, partials, words_of(solid),
+                     vec);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     k_stats_final<<<1, kStatsThreads, 0, s>>>(partials, blocks, result);
@@ -603,8 +837,9 @@ template <int Q, class S>
 static cudaError_t aero_t(const void* f, const uint8_t* solid, const float* sdf, const Geom& g, float cs, float ox,
                           float oy, float oz, double* partials, int blocks, double* result, int layout,
                           cudaStream_t s) {
+    blocks = blocks < kAeroPerSm * 148 ? blocks : kAeroPerSm * 148;
     FC_LAYOUT_LAUNCH(k_aero, blocks, kStatsThreads, (const typename S::T*)f, solid, sdf, g, cs, ox, oy, oz, partials,
-                     layout);
+                     words_of(solid));
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     k_aero_final<<<1, kStatsThreads, 0, s>>>(partials, blocks, solid, g, cs, ox, oy, oz, result);
