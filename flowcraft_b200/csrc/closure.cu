@@ -3,13 +3,12 @@
 // (closure.cuh holds the device inference).
 #include <cuda_runtime.h>
 
-#include <chrono>
 #include <cstring>
-#include <thread>
 
 #include <cub/device/device_scan.cuh>
 
 #include "fc_lbm.h"
+#include "host_wait.h"
 #include "lattice.cuh"
 #include "lbm_internal.h"
 #include "storage.cuh"
@@ -190,29 +189,17 @@ namespace {
 constexpr int kCoarseFields = 16;  // rho, u (3), tau_sgs (6), V (6)
 constexpr int kWaitTimeoutMs = 600000;
 
-// Waits for `s` by polling an event with a growing sleep, so a stuck device
-// surfaces as a timeout status instead of a hang.
+// Waits for `s` (bounded, host_wait.h).
 cudaError_t wait_bounded(cudaStream_t s, bool* timed_out) {
     *timed_out = false;
     cudaEvent_t ev;
     cudaError_t e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
     if (e != cudaSuccess) return e;
     e = cudaEventRecord(ev, s);
-    const auto t0 = std::chrono::steady_clock::now();
-    int sleep_us = 20;
-    while (e == cudaSuccess) {
-        const cudaError_t q = cudaEventQuery(ev);
-        if (q == cudaSuccess) break;
-        if (q != cudaErrorNotReady) {
-            e = q;
-            break;
-        }
-        if (std::chrono::steady_clock::now() - t0 > std::chrono::milliseconds(kWaitTimeoutMs)) {
-            *timed_out = true;
-            break;
-        }
-        std::this_thread::sleep_for(std::chrono::microseconds(sleep_us));
-        if (sleep_us < 2000) sleep_us *= 2;
+    if (e == cudaSuccess) e = poll_until([&] { return cudaEventQuery(ev); }, kWaitTimeoutMs);
+    if (e == cudaErrorNotReady) {
+        *timed_out = true;
+        e = cudaSuccess;
     }
     cudaEventDestroy(ev);
     return e;

@@ -46,17 +46,16 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <chrono>
 #include <climits>
 #include <cmath>
 #include <cstdint>
-#include <thread>
 
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_run_length_encode.cuh>
 #include <cub/device/device_scan.cuh>
 
 #include "fc_lbm.h"
+#include "host_wait.h"
 
 namespace {
 
@@ -748,23 +747,8 @@ int wait_on(cudaStream_t s) {
         cudaEventDestroy(ev);
         return FC_LBM_ERR_CUDA;
     }
-    const auto t0 = std::chrono::steady_clock::now();
-    int sleep_us = 20;
-    int rc = FC_LBM_OK;
-    for (;;) {
-        const cudaError_t q = cudaEventQuery(ev);
-        if (q == cudaSuccess) break;
-        if (q != cudaErrorNotReady) {
-            rc = FC_LBM_ERR_CUDA;
-            break;
-        }
-        if (std::chrono::steady_clock::now() - t0 > std::chrono::milliseconds(kWaitTimeoutMs)) {
-            rc = FC_LBM_ERR_TIMEOUT;
-            break;
-        }
-        std::this_thread::sleep_for(std::chrono::microseconds(sleep_us));
-        if (sleep_us < 2000) sleep_us *= 2;
-    }
+    const cudaError_t e = fc::poll_until([&] { return cudaEventQuery(ev); }, kWaitTimeoutMs);
+    const int rc = e == cudaSuccess ? FC_LBM_OK : (e == cudaErrorNotReady ? FC_LBM_ERR_TIMEOUT : FC_LBM_ERR_CUDA);
     cudaEventDestroy(ev);
     return rc;
 }
@@ -815,6 +799,35 @@ struct Scratch {
     }
 };
 
+// A few pinned bytes per host thread for the sizes and status a call reads
+// back. A copy to pageable memory waits for the stream inside the driver, and
+// the memory pool gives its memory back at such waits: the next call then maps
+// it anew, which costs more than the call's kernels.
+struct HostWords {
+    void* p = nullptr;
+    HostWords() {
+        if (cudaHostAlloc(&p, 64, cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();  // the caller falls back to pageable memory
+            p = nullptr;
+        }
+    }
+    ~HostWords() {
+        if (p) cudaFreeHost(p);
+    }
+};
+
+struct Answer {
+    unsigned long long pairs;
+    Status st;
+    GridOut grid;
+};
+static_assert(sizeof(Answer) <= 64, "one HostWords block");
+
+Answer* host_answer(Answer* fallback) {
+    static thread_local HostWords w;
+    return w.p ? static_cast<Answer*>(w.p) : fallback;
+}
+
 int code_of(cudaError_t e) {
     if (e == cudaSuccess) return FC_LBM_OK;
     if (e == cudaErrorMemoryAllocation) return FC_LBM_ERR_OUT_OF_MEMORY;
@@ -850,8 +863,11 @@ int grid_on_device(const float* d_pos, size_t nv, const fc_voxel_params* p, cuda
     k_grid_final<<<1, kGridThreads, 0, s>>>(partial, kBoundsBlocks, p->target_resolution, p->padding[0], p->padding[1],
                                   p->padding[2], d_out);
     VX_TRY(cudaGetLastError());
-    VX_TRY(cudaMemcpyAsync(host, d_out, sizeof(GridOut), cudaMemcpyDeviceToHost, s));
+    Answer own;
+    Answer* ans = host_answer(&own);
+    VX_TRY(cudaMemcpyAsync(&ans->grid, d_out, sizeof(GridOut), cudaMemcpyDeviceToHost, s));
     VX_RC(wait_on(s));
+    *host = ans->grid;
     return FC_LBM_OK;
 }
 
@@ -905,14 +921,18 @@ int voxelize_on_device(const float* d_pos, size_t nv, const uint32_t* d_idx, siz
     VX_TRY(cudaMemsetAsync(slot, 0, sizeof(uint32_t) * ntiles, s));
     Status st{};
     unsigned long long pairs = 0;
+    Answer own;
+    Answer* ans = host_answer(&own);
     if (ntri > 0) {
         k_tri_prep<<<(ntri + 1 + 255) / 256, 256, 0, s>>>(d_pos, (unsigned)nv, d_idx, ntri, g, tris, counts, slot,
                                                           d_st);
         VX_TRY(cudaGetLastError());
         VX_TRY(cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, counts, offsets, (int64_t)ntri + 1, s));
-        VX_TRY(cudaMemcpyAsync(&pairs, offsets + ntri, sizeof(pairs), cudaMemcpyDeviceToHost, s));
-        VX_TRY(cudaMemcpyAsync(&st, d_st, sizeof(st), cudaMemcpyDeviceToHost, s));
+        VX_TRY(cudaMemcpyAsync(&ans->pairs, offsets + ntri, sizeof(pairs), cudaMemcpyDeviceToHost, s));
+        VX_TRY(cudaMemcpyAsync(&ans->st, d_st, sizeof(st), cudaMemcpyDeviceToHost, s));
         VX_RC(wait_on(s));
+        pairs = ans->pairs;
+        st = ans->st;
         if (st.err & kErrBadIndex) return FC_LBM_ERR_INVALID_ARG;
         if (pairs > (unsigned long long)INT32_MAX) return FC_LBM_ERR_TOO_LARGE;
     }
@@ -968,9 +988,9 @@ int voxelize_on_device(const float* d_pos, size_t nv, const uint32_t* d_idx, siz
         k_vox_finalize<false><<<(unsigned)fin_blocks, 256, 0, s>>>(d_solid, d_sdf, g, slot, tile_reached, row_reached,
                                                                    segs);
     VX_TRY(cudaGetLastError());
-    VX_TRY(cudaMemcpyAsync(&st, d_st, sizeof(st), cudaMemcpyDeviceToHost, s));
+    VX_TRY(cudaMemcpyAsync(&ans->st, d_st, sizeof(st), cudaMemcpyDeviceToHost, s));
     VX_RC(wait_on(s));
-    return st.err ? FC_LBM_ERR_CUDA : FC_LBM_OK;
+    return ans->st.err ? FC_LBM_ERR_CUDA : FC_LBM_OK;
 }
 
 bool finite3(const float* v) { return std::isfinite(v[0]) && std::isfinite(v[1]) && std::isfinite(v[2]); }
