@@ -382,9 +382,10 @@ int guard_snapshot(fc_lbm* h, cudaStream_t s, int set) {
 
 // One step of the bulk cells of layers [z0, z0 + zc) and the boundary-list
 // entries [b, e), with or without the learned closure, ping-pong or in place.
+// chained: the launch right before it on `s` was another step of this lattice.
 cudaError_t launch_step(fc_lbm* h, const fc::StepParams& p, const void* fin, void* fout, int z0, int zc, uint32_t b,
-                        uint32_t e, cudaStream_t s, int* nl) {
-    const fc::BoundarySpan bnd{boundary_list(h), b, e, 0};
+                        uint32_t e, cudaStream_t s, int* nl, bool chained = false) {
+    const fc::BoundarySpan bnd{boundary_list(h), b, e, 0, chained};
     if (in_place(h) && h->closure_on)
         return fc::launch_bulk_aa_learned(h->q, h->storage, h->pop[0], h->d_bulk_bits, h->g, p, z0, zc,
                                           h->d_diverged, s, nl, h->cur, aa_side(h), h->closure, bnd);
@@ -399,7 +400,7 @@ cudaError_t launch_step(fc_lbm* h, const fc::StepParams& p, const void* fin, voi
                                 bnd, (h->flags & FC_OPTION_TMA_STAGING) ? 1 : 0);
 }
 
-int step_range_on(fc_lbm* h, cudaStream_t s, int z0, int zc) {
+int step_range_on(fc_lbm* h, cudaStream_t s, int z0, int zc, bool chained = false) {
     const int z1 = std::min(h->g.nz, z0 + zc);
     z0 = std::max(0, z0);
     if (z1 <= z0) return FC_LBM_OK;
@@ -407,9 +408,10 @@ int step_range_on(fc_lbm* h, cudaStream_t s, int z0, int zc) {
     const void* fin = h->pop[h->cur];
     void* fout = h->pop[1 - h->cur];
     FC_RC(guard_snapshot(h, s, 1 - h->cur));
+    chained = chained && !h->rb_pending;  // no wait on a readback in between
     int nl = 0;
     FC_TRY(h, launch_step(h, p, fin, fout, z0, h->n_bulk > 0 ? z1 - z0 : 0, h->z_begin[(size_t)z0],
-                          h->z_begin[(size_t)z1], s, &nl),
+                          h->z_begin[(size_t)z1], s, &nl, chained),
            "step");
     h->launches += nl;
     return FC_LBM_OK;
@@ -768,7 +770,7 @@ int fc_lbm_step(fc_lbm* h, void* stream, int32_t n) {
     cudaStream_t s = stream ? (cudaStream_t)stream : h->stream;
     FC_RC(enter_stream(h, s));
     for (int k = 0; k < n; ++k) {
-        FC_RC(step_range_on(h, s, 0, h->g.nz));
+        FC_RC(step_range_on(h, s, 0, h->g.nz, k > 0));
         h->cur = 1 - h->cur;
         h->steps_since_reset++;
     }

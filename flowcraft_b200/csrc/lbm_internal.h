@@ -84,6 +84,9 @@ struct BoundarySpan {
     BoundaryList list;
     uint32_t begin, end;
     unsigned slabs;  // set by the launcher
+    // the launch right before this one on the stream is another step of the
+    // same lattice (step_common.cuh, after_previous_step)
+    bool chained;
 };
 
 // ---- launchers (defined in the .cu files) ----

@@ -235,8 +235,9 @@ __device__ __forceinline__ void boundary_entry(const typename S::T* __restrict__
                                                typename S::T* __restrict__ fout, const BoundaryList& bl, uint32_t e,
                                                const Geom& g, const StepParams& p, int* __restrict__ diverged) {
     using L = Lattice<Q>;
-    const uint32_t c = __ldg(bl.cells + e);
     const unsigned long long lk = __ldg(bl.links + e);
+    const uint32_t co0 = __ldg(bl.coef_off + e);
+    const uint32_t c = after_previous_step(__ldg(bl.cells + e));
     const unsigned cls = (unsigned)(lk >> kClassShift) & 7u;
     const uint32_t nxy = (uint32_t)g.nxy;
     const uint32_t z = c / nxy;
@@ -252,7 +253,6 @@ __device__ __forceinline__ void boundary_entry(const typename S::T* __restrict__
         return;
     }
     // Fluid cell next to a wall (LbmReference.cpp:329-383).
-    const uint32_t co0 = __ldg(bl.coef_off + e);
     uint32_t bzmask = 0;  // directions that carry a Bouzidi coefficient pair
     static_for<0, Q>([&](auto I) {
         constexpr int i = decltype(I)::value;
@@ -303,8 +303,8 @@ __device__ __forceinline__ void boundary_entry_learned(const typename S::T* __re
     static_assert(!S::kExact, "the learned closure runs on the 16-bit offset formats");
     using L = Lattice<Q>;
     const bool live = e < end;
-    const uint32_t c = live ? __ldg(bl.cells + e) : 0u;
     const unsigned long long lk = live ? __ldg(bl.links + e) : 0ull;
+    const uint32_t c = after_previous_step(live ? __ldg(bl.cells + e) : 0u);
     const unsigned cls = (unsigned)(lk >> kClassShift) & 7u;
     const bool fluid = live && cls != kCellSolidFill;
     if (live && !fluid) {  // solid cell: f_i = w_i (LbmReference.cpp:264-267)
@@ -449,7 +449,7 @@ __device__ __forceinline__ void pairs_tile(const typename S::T* __restrict__ fin
         if (x + 1 == 0 || x + 1 == g.nx - 1) plane |= pair & 2u;
     }
     pair &= ~plane;
-    const uint32_t c = (uint32_t)(row * g.nx + x);
+    const uint32_t c = after_previous_step((uint32_t)(row * g.nx + x));
     if constexpr (!S::kExact) {  // the row-end cells by the whole warp (no interior warp holds one)
         row_end_cells<Q, S>(fin, fout, g, p, plane, x, c);
         plane = 0;
@@ -513,6 +513,7 @@ __global__ void __launch_bounds__(32 * kBulkRows, 4) k_bulk_pairs(const typename
                                                                 StepParams p, PlanePtrs pp, int z0,
                                                                 int* __restrict__ diverged, PairsShell sh,
                                                                 BoundarySpan bnd) {
+    step_enter();
     uint32_t e;
     if (boundary_block(bnd, e)) {
         if (e < bnd.end) boundary_entry<Q, S>(fin, fout, bnd.list, e, g, p, diverged);
@@ -569,6 +570,7 @@ __global__ void __launch_bounds__(32 * kBulkRows, 4) k_bulk_pairs_learned(const 
     __shared__ uint32_t s_in[kBulkRows][32 * 8];
     __shared__ float2 s_out[kBulkRows][32];
     __shared__ float2 s_mo[kBulkRows][12][32];  // the relaxation's moments while the MLP runs
+    step_enter();
     uint32_t e;
     if (boundary_block(bnd, e)) {
         boundary_entry_learned<Q, S>(fin, fout, bnd.list, e, bnd.end, g, p, diverged, cl, s_in[threadIdx.y],
@@ -593,7 +595,7 @@ __global__ void __launch_bounds__(32 * kBulkRows, 4) k_bulk_pairs_learned(const 
         plane |= pair & 2u;
         pair &= ~2u;
     }
-    const uint32_t c = (uint32_t)(row * g.nx + x);
+    const uint32_t row0 = after_previous_step((uint32_t)(row * g.nx)), c = row0 + (uint32_t)x;
     const bool face = (y == 0) | (y == g.ny - 1) | (z == 0) | (z == g.nz - 1);
     row_end_cells<Q, S>(fin, fout, g, p, plane, x, c);
     const bool va = pair & 1u, vb = pair & 2u;
@@ -604,7 +606,7 @@ __global__ void __launch_bounds__(32 * kBulkRows, 4) k_bulk_pairs_learned(const 
     // cell of a row end and wall cells), the masked general path on the faces.
     // Lanes beyond the row load their own row and store nothing.
     const bool fast = !face;
-    const uint32_t cs = x < g.nx ? c : (uint32_t)(row * g.nx);
+    const uint32_t cs = x < g.nx ? c : row0;
     float2 v[Q];
     if (fast) {
         static_for<0, Q>([&](auto I) {
@@ -1105,17 +1107,13 @@ static cudaError_t bulk_t(const void* fin, void* fout, const uint32_t* bits, con
     const BoundarySpan bs = with_slabs(bnd, grid.x, grid.y);
     grid.z = (unsigned)(zc > 0 ? zc : 0) + bs.slabs;
     auto launch = [&](auto P) {
-        k_bulk_pairs<Q, S, decltype(P)::value><<<grid, block, 0, s>>>(
-            (const typename S::T*)fin, (typename S::T*)fout, bits, g, p, pp, z0, dv, sh, bs);
+        return launch_step_kernel(k_bulk_pairs<Q, S, decltype(P)::value>, grid, block, s, bs.chained,
+                                  (const typename S::T*)fin, (typename S::T*)fout, bits, g, p, pp, z0, dv, sh, bs);
     };
-    if (par == kNxEven)
-        launch(std::integral_constant<int, kNxEven>{});
-    else if (par == kNxOddNyOdd)
-        launch(std::integral_constant<int, kNxOddNyOdd>{});
-    else
-        launch(std::integral_constant<int, kNxOddNyEven>{});
     ++*launched;
-    return cudaGetLastError();
+    if (par == kNxEven) return launch(std::integral_constant<int, kNxEven>{});
+    if (par == kNxOddNyOdd) return launch(std::integral_constant<int, kNxOddNyOdd>{});
+    return launch(std::integral_constant<int, kNxOddNyEven>{});
 }
 
 template <int Q, class S>
@@ -1133,12 +1131,13 @@ static cudaError_t bulk_learned_t(const void* fin, void* fout, const uint32_t* b
         dim3 grid((unsigned)((g.nx + 63) / 64), (unsigned)((g.ny + kBulkRows - 1) / kBulkRows), 1);
         const BoundarySpan bs = with_slabs(bnd, grid.x, grid.y);
         grid.z = (unsigned)(zc > 0 ? zc : 0) + bs.slabs;
-        if (tc)
-            k_bulk_pairs_learned_tc<Q, S><<<grid, block, 0, s>>>((const typename S::T*)fin, (typename S::T*)fout,
-                                                                 bits, g, p, pp, z0, dv, cl, bs);
-        else
-            k_bulk_pairs_learned<Q, S><<<grid, block, 0, s>>>((const typename S::T*)fin, (typename S::T*)fout, bits,
-                                                              g, p, pp, z0, dv, cl, bs);
+        if (!tc) {
+            ++*launched;
+            return launch_step_kernel(k_bulk_pairs_learned<Q, S>, grid, block, s, bs.chained,
+                                      (const typename S::T*)fin, (typename S::T*)fout, bits, g, p, pp, z0, dv, cl, bs);
+        }
+        k_bulk_pairs_learned_tc<Q, S><<<grid, block, 0, s>>>((const typename S::T*)fin, (typename S::T*)fout, bits, g,
+                                                             p, pp, z0, dv, cl, bs);
         ++*launched;
         return cudaGetLastError();
     }

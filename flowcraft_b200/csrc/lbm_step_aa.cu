@@ -202,8 +202,10 @@ __device__ __forceinline__ void aa_boundary_entry(typename S::T* f, const Bounda
                                                   const StepParams& p, int* __restrict__ diverged, const AaSide& sd) {
     using L = Lattice<Q>;
     using T = typename S::T;
-    const uint32_t c = __ldg(bl.cells + e);
     const unsigned long long lk = __ldg(bl.links + e);
+    const uint32_t co0 = __ldg(bl.coef_off + e);
+    const uint32_t c = __ldg(bl.cells + e);
+    previous_step_done();
     const unsigned cls = (unsigned)(lk >> kClassShift) & 7u;
     const uint32_t nxy = (uint32_t)g.nxy;
     const int z = (int)(c / nxy);
@@ -227,7 +229,6 @@ __device__ __forceinline__ void aa_boundary_entry(typename S::T* f, const Bounda
         }
         return;
     }
-    const uint32_t co0 = __ldg(bl.coef_off + e);
     uint32_t bzmask = 0;
     static_for<0, Q>([&](auto I) {
         constexpr int i = decltype(I)::value;
@@ -290,8 +291,9 @@ __device__ __forceinline__ void aa_boundary_entry_learned(typename S::T* f, cons
     using L = Lattice<Q>;
     using T = typename S::T;
     const bool live = e < end;
-    const uint32_t c = live ? __ldg(bl.cells + e) : 0u;
     const unsigned long long lk = live ? __ldg(bl.links + e) : 0ull;
+    const uint32_t c = live ? __ldg(bl.cells + e) : 0u;
+    previous_step_done();
     const unsigned cls = (unsigned)(lk >> kClassShift) & 7u;
     const bool fluid = live && cls != kCellSolidFill;
     const uint32_t nxy = (uint32_t)g.nxy;
@@ -393,6 +395,7 @@ __global__ void __launch_bounds__(32 * kBulkRows, 4) k_bulk_pairs_aa(typename S:
     using L = Lattice<Q>;
     using T = typename S::T;
     using T2 = typename S::T2;
+    step_enter();
     uint32_t e;
     if (boundary_block(bnd, e)) {
         if (e < bnd.end) aa_boundary_entry<Q, S, Odd>(f, bnd.list, e, g, p, diverged, sd);
@@ -417,6 +420,7 @@ __global__ void __launch_bounds__(32 * kBulkRows, 4) k_bulk_pairs_aa(typename S:
         pair &= ~2u;
     }
     const uint32_t c = (uint32_t)(row * g.nx + x);
+    previous_step_done();
     if constexpr (!S::kExact) {  // the row-end cells by the whole warp
         aa_row_end_cells<Q, S, Odd>(f, g, p, sd, plane, x, y, z, c, row);
         plane = 0;
@@ -631,6 +635,7 @@ __global__ void __launch_bounds__(32 * kBulkRows, 4) k_bulk_pairs_aa_learned(typ
     __shared__ uint32_t s_in[kBulkRows][32 * 8];
     __shared__ float2 s_out[kBulkRows][32];
     __shared__ float2 s_mo[kBulkRows][12][32];  // the relaxation's moments while the MLP runs
+    step_enter();
     uint32_t e;
     if (boundary_block(bnd, e)) {
         aa_boundary_entry_learned<Q, S, Odd>(f, bnd.list, e, bnd.end, g, p, diverged, sd, cl, s_in[threadIdx.y],
@@ -656,6 +661,7 @@ __global__ void __launch_bounds__(32 * kBulkRows, 4) k_bulk_pairs_aa_learned(typ
         pair &= ~2u;
     }
     const uint32_t c = (uint32_t)(row * g.nx + x);
+    previous_step_done();
     const uint32_t cs = x < g.nx ? c : (uint32_t)(row * g.nx);  // lanes past the row end read its first pair
     const bool face = (y == 0) | (y == g.ny - 1) | (z == 0) | (z == g.nz - 1);
     // off the faces every source slot lies inside the set (k_bulk_pairs_aa)
@@ -816,12 +822,9 @@ static cudaError_t bulk_aa_t(void* f, const uint32_t* bits, const Geom& g, const
     dim3 grid((unsigned)((g.nx + 63) / 64), (unsigned)((g.ny + kBulkRows - 1) / kBulkRows), 1);
     const BoundarySpan bs = with_slabs(bnd, grid.x, grid.y);
     grid.z = (unsigned)(zc > 0 ? zc : 0) + bs.slabs;
-    if (odd)
-        k_bulk_pairs_aa<Q, S, true><<<grid, block, 0, s>>>(base, bits, g, p, pp, z0, dv, sd, bs);
-    else
-        k_bulk_pairs_aa<Q, S, false><<<grid, block, 0, s>>>(base, bits, g, p, pp, z0, dv, sd, bs);
     ++*launched;
-    return cudaGetLastError();
+    return launch_step_kernel(odd ? k_bulk_pairs_aa<Q, S, true> : k_bulk_pairs_aa<Q, S, false>, grid, block, s,
+                              bs.chained, base, bits, g, p, pp, z0, dv, sd, bs);
 }
 
 template <int Q, class S>
@@ -848,12 +851,9 @@ static cudaError_t bulk_aa_learned_t(void* f, const uint32_t* bits, const Geom& 
         dim3 grid((unsigned)((g.nx + 63) / 64), (unsigned)((g.ny + kBulkRows - 1) / kBulkRows), 1);
         const BoundarySpan bs = with_slabs(bnd, grid.x, grid.y);
         grid.z = (unsigned)(zc > 0 ? zc : 0) + bs.slabs;
-        if (odd)
-            k_bulk_pairs_aa_learned<Q, S, true><<<grid, block, 0, s>>>(base, bits, g, p, pp, z0, dv, sd, cl, bs);
-        else
-            k_bulk_pairs_aa_learned<Q, S, false><<<grid, block, 0, s>>>(base, bits, g, p, pp, z0, dv, sd, cl, bs);
         ++*launched;
-        return cudaGetLastError();
+        return launch_step_kernel(odd ? k_bulk_pairs_aa_learned<Q, S, true> : k_bulk_pairs_aa_learned<Q, S, false>,
+                                  grid, block, s, bs.chained, base, bits, g, p, pp, z0, dv, sd, cl, bs);
     }
 }
 

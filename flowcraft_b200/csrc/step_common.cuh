@@ -14,6 +14,51 @@ namespace fc {
 constexpr int kBulkRows = 8;  // block = 32 x-lanes x 8 rows
 constexpr int kBatchChunk = 8;  // consecutive tiles a block of the batch kernel takes at a time
 
+// Chained steps overlap their ends: a step kernel lets the next one of its
+// lattice start as soon as its own blocks have all started
+// (programmatic dependent launch), and the next one's blocks, on SMs that the
+// last wave leaves idle, run up to here: launch, index arithmetic and the
+// loads of what no step writes (bulk mask, boundary list). The populations
+// wait until the step before is complete. Passing the cell index through the
+// wait makes every population address depend on it, so that no load, also no
+// read-only one, can be moved ahead of it.
+// B200, us per step, with the boundary list in its own kernel and full
+// serialization / now: 48x24x24 FP32 14.6 / 6.7, FP16 18.5 / 9.0; 128x64x64
+// FP32 27.0 / 19.5, FP16 30.0 / 15.3; 512x256x256 FP16 571 / 554.
+__device__ __forceinline__ uint32_t after_previous_step(uint32_t c) {
+    asm volatile("griddepcontrol.wait;" : "+r"(c)::"memory");
+    return c;
+}
+
+// The same for the in-place kernels, whose population loads are ordinary ones
+// that stay behind a memory clobber (with the index passed through, the FP32
+// kernels spill more and lost 2 % at 512x256x256).
+__device__ __forceinline__ void previous_step_done() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// First thing in a chained kernel. One thread waits whatever its block holds:
+// a step is never complete before the one it was chained to, so the wait above
+// covers every earlier step too.
+__device__ __forceinline__ void step_enter() {
+    asm volatile("griddepcontrol.launch_dependents;");
+    if ((blockIdx.x | blockIdx.y | blockIdx.z | threadIdx.x | threadIdx.y) == 0)
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// Host: launches a step kernel, chained to the launch before it if asked.
+template <class... P, class... A>
+cudaError_t launch_step_kernel(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t s, bool chained, A&&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = chained ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // Blocks of a step launch that take boundary-list entries (BoundarySpan):
 // true for those, with the entry of this thread (one past the end for none).
 __device__ __forceinline__ bool boundary_block(const BoundarySpan& b, uint32_t& entry) {
