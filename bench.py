@@ -565,7 +565,7 @@ def run_batch(args, cfg, rank, world, local_rank):
             "config": {"workload": cfg["desc"], "lattices": r["lattices"], "cells": cells,
                        "sizes": r["sizes"], "autotune": tuned,
                        "parallelism": f"replicas x{world}" if world > 1 else "single GPU"},
-            "diverged": r["diverged"], "gpu_launches": (2 if tuned["rows"] else r["lattices"] + 1) * steps,
+            "diverged": r["diverged"], "gpu_launches": (2 if tuned["rows"] else r["lattices"]) * steps,
             "clocks": clocks,
             "sequential": {"glups": world * cells * steps / (seq_ms / 1e3) / 1e9, "ms_per_step": seq_ms / steps,
                            "how": "the same lattices stepped one after another on one stream with LbmSolver.Step"}}

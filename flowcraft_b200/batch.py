@@ -1,8 +1,7 @@
 """Many lattices stepped together (``fc_lbm_batch_*`` in include/fc_lbm.h):
 one bulk launch over the tiles of every member per step (persistent, or one
-block per tile; or each member's own bulk kernel, side by side, when the
-autotuner finds that faster), pairs of steps replayed as a CUDA graph, block shape picked by an
-autotuner. The
+block per tile; or each member's own step kernels, side by side, when the
+autotuner finds that faster), block shape picked by an autotuner. The
 members stay ordinary ``LbmSolver`` objects (readbacks, forces, SetParams);
 the batch only steps them, bit-identically to ``LbmSolver.Step``."""
 from __future__ import annotations
@@ -15,7 +14,7 @@ from .lbm import FC_LBM_OK, LbmError, load_library
 
 # (rows, grid_mult): the persistent launch's block shapes (grid_mult 1, 2),
 # the one-block-per-tile launch (8, 0), then rows 0: every member's
-# own bulk kernel, run side by side on forked streams
+# own step kernels, run side by side on forked streams
 CANDIDATES = [(r, m) for r in (4, 8, 16) for m in (1, 2)] + [(8, 0), (0, 1)]
 
 

@@ -414,11 +414,10 @@ FC_LBM_API int fc_lbm_particles_set(fc_lbm* h, const float* points, size_t point
  * For sweeps such as a set of angles of attack: the members (initialized
  * handles on one device, one lattice model and storage format, even nx, no
  * learned closure) step together. Every step is one persistent bulk launch
- * over a work-list of the tiles of all members (or, when that is faster,
- * each member's own bulk kernel, run side by side on forked streams) and one
- * launch over all their boundary lists; pairs of steps replay as one CUDA
- * graph. Results are
- * bit-identical to stepping every member with fc_lbm_step. The members keep
+ * over a work-list of the tiles of all members and one launch over all their
+ * boundary lists, pairs of steps replayed as one CUDA graph; or, when that is
+ * faster, each member's own step kernels, side by side on forked streams.
+ * Results are bit-identical to stepping every member with fc_lbm_step. The members keep
  * their own state and API; they must outlive the batch and must not step on
  * their own while a batch step is queued. */
 typedef struct fc_lbm_batch fc_lbm_batch;
@@ -435,9 +434,9 @@ FC_LBM_API int fc_lbm_batch_step(fc_lbm_batch* b, int32_t n);
  * chunks of 8 tiles), or rows 8 with grid_mult 0 (one block per tile over the
  * tiles of every lattice, each lattice's in the order of its own launch, the
  * lattices one after another; one launch per 32 lattices). rows 0
- * replaces the batch launch by each member's own bulk kernel (the one
- * fc_lbm_step launches), spread over 4 forked streams; grid_mult is then
- * unused. Default 8, 1. */
+ * replaces the batch launches by each member's own step kernel (the one
+ * fc_lbm_step launches), spread over up to 16 forked streams; grid_mult is
+ * then unused. Default 8, 1. */
 FC_LBM_API int fc_lbm_batch_config(fc_lbm_batch* b, int32_t rows, int32_t grid_mult);
 /* Autotuner: times each of the FC_LBM_BATCH_CANDIDATES shapes (rows 4, 8, 16
  * x grid_mult 1, 2, in that order, then rows 8 with grid_mult 0, then rows 0)
