@@ -938,7 +938,6 @@ int voxelize_on_device(const float* d_pos, size_t nv, const uint32_t* d_idx, siz
     }
     // the second half: the tiles' triangle lists and the flood fill's nodes
     const unsigned runs = st.occupied;  // the runs of equal tile ids after the sort
-    if (runs > (unsigned)INT32_MAX / kTileBoxes) return FC_LBM_ERR_TOO_LARGE;
     const uint64_t nodes = ntiles + (uint64_t)runs * kTileNodes;
     const bool wide = nodes >= 0xffffffffull;
     uint32_t *k0 = nullptr, *k1 = nullptr, *v0 = nullptr, *v1 = nullptr, *run_tile = nullptr, *run_len = nullptr;
@@ -968,9 +967,15 @@ int voxelize_on_device(const float* d_pos, size_t nv, const uint32_t* d_idx, siz
         VX_TRY(cub::DeviceScan::ExclusiveSum(tmp, scan_bytes, run_len, run_off, (int64_t)runs, s));
         k_tile_slots<<<(runs + 255) / 256, 256, 0, s>>>(run_tile, runs, slot);
         VX_TRY(cudaGetLastError());
-        k_vox_raster<<<kTileBoxes * runs, kRasterThreads, 0, s>>>(tris, vb.Current(), run_tile, run_len, run_off, g,
-                                                                  d_solid, d_sdf, mask);
-        VX_TRY(cudaGetLastError());
+        // a tile's boxes next to each other in the launch (they read one list);
+        // a grid holds 2^31 - 1 blocks, so very many tiles take several launches
+        constexpr unsigned kLaunchTiles = (unsigned)INT32_MAX / kTileBoxes;
+        for (unsigned first = 0; first < runs; first += std::min(kLaunchTiles, runs - first)) {
+            k_vox_raster<<<kTileBoxes * std::min(kLaunchTiles, runs - first), kRasterThreads, 0, s>>>(
+                tris, vb.Current(), run_tile + first, run_len + first, run_off + first, g, d_solid, d_sdf,
+                mask + (size_t)first * kTileRows * 2);
+            VX_TRY(cudaGetLastError());
+        }
     }
     VX_RC(wide ? flood(g, ntiles, runs, slot, mask, run_tile, reinterpret_cast<unsigned long long*>(labels),
                        tile_reached, row_reached, d_st, s)
