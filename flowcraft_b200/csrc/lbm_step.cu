@@ -34,7 +34,7 @@ namespace fc {
 // One bulk cell off the faces and row ends: a pure pull from the 19 (15)
 // upstream neighbours.
 template <int Q, class S>
-__device__ __forceinline__ void bulk_cell(const typename S::T* __restrict__ fin, typename S::T* __restrict__ fout,
+__device__ __forceinline__ void bulk_cell(const typename S::T* fin, typename S::T* fout,
                                           const Geom& g, const StepParams& p, uint32_t c, int* __restrict__ diverged) {
     float f[Q];
     static_for<0, Q>([&](auto I) {
@@ -53,7 +53,7 @@ __device__ __forceinline__ void bulk_cell(const typename S::T* __restrict__ fin,
 // upstream neighbour's fIn moments with rho relaxed toward 1
 // (LbmReference.cpp:275-327).
 template <int Q, class S>
-__device__ __forceinline__ void plane_cell(const typename S::T* __restrict__ fin, typename S::T* __restrict__ fout,
+__device__ __forceinline__ void plane_cell(const typename S::T* fin, typename S::T* fout,
                                            const Geom& g, const StepParams& p, int x, size_t c) {
     float f[Q];
     if (x == p.inlet_x) {
@@ -88,7 +88,7 @@ __device__ __forceinline__ void plane_cell(const typename S::T* __restrict__ fin
 // plane_cell: there the warp-wide version costs more registers than the
 // kernel has to spare.)
 template <int Q, class S>
-__device__ __forceinline__ void row_end_cell(const typename S::T* __restrict__ fin, typename S::T* __restrict__ fout,
+__device__ __forceinline__ void row_end_cell(const typename S::T* fin, typename S::T* fout,
                                              const Geom& g, const StepParams& p, int px, size_t pc) {
     const unsigned lane = threadIdx.x & 31;
     const bool mine = lane < (unsigned)Q;
@@ -102,7 +102,7 @@ __device__ __forceinline__ void row_end_cell(const typename S::T* __restrict__ f
         return;
     }
     const size_t nb = p.reverse ? pc + 1 : pc - 1;
-    const float own = S::dec(S::ld(fin + (size_t)i * g.ps + nb), wi);
+    const float own = S::dec(ld_plain<S>(fin + (size_t)i * g.ps + nb), wi);
     float f[Q];
     static_for<0, Q>([&](auto I) { f[decltype(I)::value] = __shfl_sync(0xffffffffu, own, decltype(I)::value); });
     float nr, nu, nv, nw;
@@ -113,7 +113,7 @@ __device__ __forceinline__ void row_end_cell(const typename S::T* __restrict__ f
 }
 
 template <int Q, class S>
-__device__ __forceinline__ void row_end_cells(const typename S::T* __restrict__ fin, typename S::T* __restrict__ fout,
+__device__ __forceinline__ void row_end_cells(const typename S::T* fin, typename S::T* fout,
                                               const Geom& g, const StepParams& p, unsigned plane, int x, uint32_t c) {
     unsigned m = __ballot_sync(0xffffffffu, plane != 0u);
     while (m) {  // uniform: at most the two row ends
@@ -176,16 +176,16 @@ constexpr bool kOffsets = !S::kExact && Par == kNxEven;
 template <class S, int Par>
 __device__ __forceinline__ float pair_ld(const typename S::T* p, float w) {
     if constexpr (kOffsets<S, Par>)
-        return S::raw(S::ld(p));
+        return S::raw(ld_plain<S>(p));
     else
-        return S::dec(S::ld(p), w);
+        return S::dec(ld_plain<S>(p), w);
 }
 template <class S, int Par>
 __device__ __forceinline__ float2 pair_ld2(const typename S::T* p, float w) {
     if constexpr (kOffsets<S, Par>)
-        return S::raw2(S::ld2(p));
+        return S::raw2(ld2_plain<S>(p));
     else
-        return S::dec2(S::ld2(p), w);
+        return S::dec2(ld2_plain<S>(p), w);
 }
 
 template <int Q, class S, int Par>
@@ -231,8 +231,8 @@ __device__ __forceinline__ void store_pair(const PlanePtrs& pp, uint32_t c, cons
 // inlet/outlet planes) and the solid cells an outlet reads. Every link's source
 // address is formed with selects first and all loads issue together.
 template <int Q, class S>
-__device__ __forceinline__ void boundary_entry(const typename S::T* __restrict__ fin,
-                                               typename S::T* __restrict__ fout, const BoundaryList& bl, uint32_t e,
+__device__ __forceinline__ void boundary_entry(const typename S::T* fin,
+                                               typename S::T* fout, const BoundaryList& bl, uint32_t e,
                                                const Geom& g, const StepParams& p, int* __restrict__ diverged) {
     using L = Lattice<Q>;
     const unsigned long long lk = __ldg(bl.links + e);
@@ -295,8 +295,8 @@ __device__ __forceinline__ void boundary_entry(const typename S::T* __restrict__
 // the closure (e == end: no entry); only live fluid entries store. `in` and
 // `out` are the warp's closure buffers.
 template <int Q, class S>
-__device__ __forceinline__ void boundary_entry_learned(const typename S::T* __restrict__ fin,
-                                                       typename S::T* __restrict__ fout, const BoundaryList& bl,
+__device__ __forceinline__ void boundary_entry_learned(const typename S::T* fin,
+                                                       typename S::T* fout, const BoundaryList& bl,
                                                        uint32_t e, uint32_t end, const Geom& g, const StepParams& p,
                                                        int* __restrict__ diverged, const ClosureDev& cl,
                                                        uint32_t* s_in, float2* s_out) {
@@ -420,7 +420,7 @@ __device__ __forceinline__ void shell_item(const PairsShell& sh, int& bx, int& b
 // leave). k_bulk_pairs_tiles runs the same code for the tiles of many
 // lattices in one launch.
 template <int Q, class S, int Par = kNxEven>
-__device__ __forceinline__ void pairs_tile(const typename S::T* __restrict__ fin, typename S::T* __restrict__ fout,
+__device__ __forceinline__ void pairs_tile(const typename S::T* fin, typename S::T* fout,
                                            const uint32_t* __restrict__ bulk_bits, const Geom& g,
                                            const StepParams& p, const PlanePtrs& pp, int* __restrict__ diverged,
                                            int bx, int by, int z, bool shell) {
@@ -507,8 +507,8 @@ __device__ __forceinline__ void pairs_tile(const typename S::T* __restrict__ fin
 }
 
 template <int Q, class S, int Par>
-__global__ void __launch_bounds__(32 * kBulkRows, 4) k_bulk_pairs(const typename S::T* __restrict__ fin,
-                                                                typename S::T* __restrict__ fout,
+__global__ void __launch_bounds__(32 * kBulkRows, 4) k_bulk_pairs(const typename S::T* fin,
+                                                                typename S::T* fout,
                                                                 const uint32_t* __restrict__ bulk_bits, Geom g,
                                                                 StepParams p, PlanePtrs pp, int z0,
                                                                 int* __restrict__ diverged, PairsShell sh,
@@ -558,8 +558,8 @@ __global__ void __launch_bounds__(32 * kBulkRows, 4) k_bulk_pairs_tiles(const __
 // halves around the closure (moments2, closure_warp_mlp, relax2). Warps never
 // wait for one another: the closure's shared memory is private to each warp.
 template <int Q, class S>
-__global__ void __launch_bounds__(32 * kBulkRows, 4) k_bulk_pairs_learned(const typename S::T* __restrict__ fin,
-                                                                        typename S::T* __restrict__ fout,
+__global__ void __launch_bounds__(32 * kBulkRows, 4) k_bulk_pairs_learned(const typename S::T* fin,
+                                                                        typename S::T* fout,
                                                                         const uint32_t* __restrict__ bulk_bits,
                                                                         Geom g, StepParams p, PlanePtrs pp, int z0,
                                                                         int* __restrict__ diverged, ClosureDev cl,
@@ -612,8 +612,8 @@ __global__ void __launch_bounds__(32 * kBulkRows, 4) k_bulk_pairs_learned(const 
         static_for<0, Q>([&](auto I) {
             constexpr int i = decltype(I)::value;
             const T* src = static_cast<const T*>(pp.src[i]);
-            v[i] = L::ex(i) == 0 ? S::raw2(S::ld2(src + cs))
-                                 : make_float2(S::raw(S::ld(src + cs)), S::raw(S::ld(src + cs + 1u)));
+            v[i] = L::ex(i) == 0 ? S::raw2(ld2_plain<S>(src + cs))
+                                 : make_float2(S::raw(ld_plain<S>(src + cs)), S::raw(ld_plain<S>(src + cs + 1u)));
         });
     } else {
         static_for<0, Q>([&](auto I) {
@@ -627,7 +627,7 @@ __global__ void __launch_bounds__(32 * kBulkRows, 4) k_bulk_pairs_learned(const 
             const uint32_t sa = va ? c - off : cs;
             const uint32_t sb = vb ? c + 1u - off : cs + 1u;
             const T* base = fin + (size_t)pl * g.ps;
-            v[i] = make_float2(S::raw(S::ld(base + sa)), S::raw(S::ld(base + sb)));
+            v[i] = make_float2(S::raw(ld_plain<S>(base + sa)), S::raw(ld_plain<S>(base + sb)));
         });
     }
     Mom2 mo;
@@ -709,8 +709,8 @@ __global__ void __launch_bounds__(32 * kBulkRows, 4) k_bulk_pairs_learned(const 
 // nothing hides those waits: in a developed flow this kernel takes twice the
 // time of the warp-level one, which stays the default.
 template <int Q, class S>
-__global__ void __launch_bounds__(32 * kBulkRows, 4) k_bulk_pairs_learned_tc(const typename S::T* __restrict__ fin,
-                                                                           typename S::T* __restrict__ fout,
+__global__ void __launch_bounds__(32 * kBulkRows, 4) k_bulk_pairs_learned_tc(const typename S::T* fin,
+                                                                           typename S::T* fout,
                                                                            const uint32_t* __restrict__ bulk_bits,
                                                                            Geom g, StepParams p, PlanePtrs pp, int z0,
                                                                            int* __restrict__ diverged, ClosureDev cl,
@@ -765,8 +765,8 @@ __global__ void __launch_bounds__(32 * kBulkRows, 4) k_bulk_pairs_learned_tc(con
         static_for<0, Q>([&](auto I) {
             constexpr int i = decltype(I)::value;
             const T* src = static_cast<const T*>(pp.src[i]);
-            v[i] = L::ex(i) == 0 ? S::raw2(S::ld2(src + cs))
-                                 : make_float2(S::raw(S::ld(src + cs)), S::raw(S::ld(src + cs + 1u)));
+            v[i] = L::ex(i) == 0 ? S::raw2(ld2_plain<S>(src + cs))
+                                 : make_float2(S::raw(ld_plain<S>(src + cs)), S::raw(ld_plain<S>(src + cs + 1u)));
         });
     } else {
         static_for<0, Q>([&](auto I) {
@@ -780,7 +780,7 @@ __global__ void __launch_bounds__(32 * kBulkRows, 4) k_bulk_pairs_learned_tc(con
             const uint32_t sa = va ? c - off : cs;
             const uint32_t sb = vb ? c + 1u - off : cs + 1u;
             const T* base = fin + (size_t)pl * g.ps;
-            v[i] = make_float2(S::raw(S::ld(base + sa)), S::raw(S::ld(base + sb)));
+            v[i] = make_float2(S::raw(ld_plain<S>(base + sa)), S::raw(ld_plain<S>(base + sb)));
         });
     }
     Mom2 mo;

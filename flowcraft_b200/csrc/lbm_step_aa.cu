@@ -38,15 +38,6 @@ namespace fc {
 
 namespace {
 
-template <class S>
-__device__ __forceinline__ typename S::T ld_plain(const typename S::T* p) {
-    return *p;  // a coherent load: the kernel writes the same array
-}
-template <class S>
-__device__ __forceinline__ typename S::T2 ld2_plain(const typename S::T* p) {
-    return *reinterpret_cast<const typename S::T2*>(p);
-}
-
 __device__ __forceinline__ size_t outm_index(const AaSide& sd, int par, int col, size_t row) {
     return ((size_t)par * 2 + (size_t)col) * sd.rows + row;
 }

@@ -19,9 +19,12 @@ constexpr int kBatchChunk = 8;  // consecutive tiles a block of the batch kernel
 // (programmatic dependent launch), and the next one's blocks, on SMs that the
 // last wave leaves idle, run up to here: launch, index arithmetic and the
 // loads of what no step writes (bulk mask, boundary list). The populations
-// wait until the step before is complete. Passing the cell index through the
-// wait makes every population address depend on it, so that no load, also no
-// read-only one, can be moved ahead of it.
+// wait until the step before is complete. They come by ordinary loads
+// (ld_plain): a read-only load asks for data that nothing writes during the
+// kernel's life, and here the step before still does at its start (the two
+// kinds measured the same, within 1 % from 48x24x24 to 1024x512x512). Passing
+// the cell index through the wait makes every population address depend on
+// it, so that no load moves ahead of it.
 // B200, us per step, with the boundary list in its own kernel and full
 // serialization / now: 48x24x24 FP32 14.6 / 6.7, FP16 18.5 / 9.0; 128x64x64
 // FP32 27.0 / 19.5, FP16 30.0 / 15.3; 512x256x256 FP16 571 / 554.
@@ -94,9 +97,8 @@ __device__ __forceinline__ int edge_plane(bool oy, bool oz, const StepParams& p)
 }
 
 template <int Q, class S>
-__device__ __forceinline__ float load_plane(const typename S::T* __restrict__ f, int plane, size_t n, size_t cell,
-                                            float w) {
-    return S::dec(S::ld(f + (size_t)plane * n + cell), w);
+__device__ __forceinline__ float load_plane(const typename S::T* f, int plane, size_t n, size_t cell, float w) {
+    return S::dec(ld_plain<S>(f + (size_t)plane * n + cell), w);
 }
 
 // Both cells of a pair through the collision the storage format uses;

@@ -79,6 +79,20 @@ struct StoreBF16 {
     __device__ __forceinline__ static T ld(const T* p) { return __ldg(p); }
 };
 
+// A value or an aligned pair by an ordinary load, for the step kernels: the
+// in-place ones write the array they read, and a chained ping-pong one starts
+// while the step before still writes it (step_common.cuh). S::ld and S::ld2
+// are read-only loads, which hold only for data that nothing writes during
+// the kernel's life.
+template <class S>
+__device__ __forceinline__ typename S::T ld_plain(const typename S::T* p) {
+    return *p;
+}
+template <class S>
+__device__ __forceinline__ typename S::T2 ld2_plain(const typename S::T* p) {
+    return *reinterpret_cast<const typename S::T2*>(p);
+}
+
 // Population i of `cell` in an SoA plane set with plane stride n.
 template <int Q, class S>
 __device__ __forceinline__ float load_pop(const typename S::T* __restrict__ f, int i, size_t n, size_t cell) {
@@ -86,26 +100,26 @@ __device__ __forceinline__ float load_pop(const typename S::T* __restrict__ f, i
 }
 
 template <int Q, class S, int I>
-__device__ __forceinline__ float load_pop_c(const typename S::T* __restrict__ f, size_t n, size_t cell) {
-    return S::dec(S::ld(f + (size_t)I * n + cell), Lattice<Q>::w(I));
+__device__ __forceinline__ float load_pop_c(const typename S::T* f, size_t n, size_t cell) {
+    return S::dec(ld_plain<S>(f + (size_t)I * n + cell), Lattice<Q>::w(I));
 }
 
 // Same with 32-bit cell indices relative to one plane's base pointer (cells
 // per lattice are below 2^32, plane offsets are not).
 template <int Q, class S, int I>
-__device__ __forceinline__ float load_pop_i(const typename S::T* __restrict__ f, size_t n, uint32_t cell) {
+__device__ __forceinline__ float load_pop_i(const typename S::T* f, size_t n, uint32_t cell) {
     const typename S::T* plane = f + (size_t)I * n;
-    return S::dec(S::ld(plane + cell), Lattice<Q>::w(I));
+    return S::dec(ld_plain<S>(plane + cell), Lattice<Q>::w(I));
 }
 
 template <int Q, class S, int I>
-__device__ __forceinline__ void store_pop_i(typename S::T* __restrict__ f, size_t n, uint32_t cell, float v) {
+__device__ __forceinline__ void store_pop_i(typename S::T* f, size_t n, uint32_t cell, float v) {
     typename S::T* plane = f + (size_t)I * n;
     plane[cell] = S::enc(v, Lattice<Q>::w(I));
 }
 
 template <int Q, class S, int I>
-__device__ __forceinline__ void store_pop_c(typename S::T* __restrict__ f, size_t n, size_t cell, float v) {
+__device__ __forceinline__ void store_pop_c(typename S::T* f, size_t n, size_t cell, float v) {
     f[(size_t)I * n + cell] = S::enc(v, Lattice<Q>::w(I));
 }
 
