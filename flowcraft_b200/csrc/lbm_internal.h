@@ -73,8 +73,8 @@ struct BoundaryList {
 };
 
 // The boundary-list entries [begin, end) that a step kernel updates beside
-// its bulk cells. The launch's first `slabs` z slabs of blocks take them, one
-// entry per thread: an entry is a long chain of dependent loads, so its
+// its bulk cells. The launch's first `slabs` z slabs of blocks take them
+// (launch_with_slabs in step_common.cuh), one entry per thread: an entry is a long chain of dependent loads, so its
 // blocks start first and run under the bulk blocks instead of after them.
 // Against a kernel of their own behind the bulk kernel (10-25 us per step on a
 // B200): 48x24x24 FP32, 20 steps and a field, 562 -> 381 us; 256x128x128 FP32

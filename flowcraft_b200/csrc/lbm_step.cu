@@ -1094,26 +1094,24 @@ static cudaError_t bulk_t(const void* fin, void* fout, const uint32_t* bits, con
         sh.nf = zi1 > sh.zi0 ? (unsigned long long)(sh.gx - 2) * sh.nyf * (zi1 - sh.zi0) : 0ull;
         const unsigned long long ng = (unsigned long long)(sh.gx - 2) * sh.nyb * sh.nzf;
         sh.n = sh.ne + sh.nf + ng;
-        const BoundarySpan bs = with_slabs(bnd, (unsigned)sh.n, 1);
-        k_bulk_pairs<Q, S, kNxEven><<<dim3((unsigned)sh.n, 1, 1 + bs.slabs), block, 0, s>>>(
-            (const typename S::T*)fin, (typename S::T*)fout, bits, g, p, pp, z0, dv, sh, bs);
-        ++*launched;
-        return cudaGetLastError();
+        return launch_with_slabs(bnd, (unsigned)sh.n, 1, 1, launched, [&](const BoundarySpan& bs, unsigned layers) {
+            return launch_step_kernel(k_bulk_pairs<Q, S, kNxEven>, dim3((unsigned)sh.n, 1, layers + bs.slabs), block, s,
+                                      false, (const typename S::T*)fin, (typename S::T*)fout, bits, g, p, pp, z0, dv, sh,
+                                      bs);
+        });
     }
     // odd nx: one cell more, for the rows shifted to the left
     const int par = pair_parity(g);
     dim3 grid((unsigned)((g.nx + (par == kNxEven ? 0 : 1) + 63) / 64),
               (unsigned)((g.ny + kBulkRows - 1) / kBulkRows), 1);
-    const BoundarySpan bs = with_slabs(bnd, grid.x, grid.y);
-    grid.z = (unsigned)(zc > 0 ? zc : 0) + bs.slabs;
-    auto launch = [&](auto P) {
-        return launch_step_kernel(k_bulk_pairs<Q, S, decltype(P)::value>, grid, block, s, bs.chained,
-                                  (const typename S::T*)fin, (typename S::T*)fout, bits, g, p, pp, z0, dv, sh, bs);
-    };
-    ++*launched;
-    if (par == kNxEven) return launch(std::integral_constant<int, kNxEven>{});
-    if (par == kNxOddNyOdd) return launch(std::integral_constant<int, kNxOddNyOdd>{});
-    return launch(std::integral_constant<int, kNxOddNyEven>{});
+    const auto kernel = par == kNxEven ? k_bulk_pairs<Q, S, kNxEven>
+                                       : (par == kNxOddNyOdd ? k_bulk_pairs<Q, S, kNxOddNyOdd>
+                                                             : k_bulk_pairs<Q, S, kNxOddNyEven>);
+    return launch_with_slabs(bnd, grid.x, grid.y, zc > 0 ? zc : 0, launched, [&](const BoundarySpan& bs, unsigned layers) {
+        grid.z = layers + bs.slabs;
+        return launch_step_kernel(kernel, grid, block, s, bs.chained, (const typename S::T*)fin, (typename S::T*)fout,
+                                  bits, g, p, pp, z0, dv, sh, bs);
+    });
 }
 
 template <int Q, class S>
@@ -1129,17 +1127,13 @@ static cudaError_t bulk_learned_t(const void* fin, void* fout, const uint32_t* b
         const PlanePtrs pp = pp_of<Q, S>(fin, fout, g);
         dim3 block(32, kBulkRows, 1);
         dim3 grid((unsigned)((g.nx + 63) / 64), (unsigned)((g.ny + kBulkRows - 1) / kBulkRows), 1);
-        const BoundarySpan bs = with_slabs(bnd, grid.x, grid.y);
-        grid.z = (unsigned)(zc > 0 ? zc : 0) + bs.slabs;
-        if (!tc) {
-            ++*launched;
-            return launch_step_kernel(k_bulk_pairs_learned<Q, S>, grid, block, s, bs.chained,
-                                      (const typename S::T*)fin, (typename S::T*)fout, bits, g, p, pp, z0, dv, cl, bs);
-        }
-        k_bulk_pairs_learned_tc<Q, S><<<grid, block, 0, s>>>((const typename S::T*)fin, (typename S::T*)fout, bits, g,
-                                                             p, pp, z0, dv, cl, bs);
-        ++*launched;
-        return cudaGetLastError();
+        const auto kernel = tc ? k_bulk_pairs_learned_tc<Q, S> : k_bulk_pairs_learned<Q, S>;
+        return launch_with_slabs(bnd, grid.x, grid.y, zc > 0 ? zc : 0, launched,
+                                 [&](const BoundarySpan& bs, unsigned layers) {
+            grid.z = layers + bs.slabs;
+            return launch_step_kernel(kernel, grid, block, s, bs.chained && !tc, (const typename S::T*)fin,
+                                      (typename S::T*)fout, bits, g, p, pp, z0, dv, cl, bs);
+        });
     }
 }
 

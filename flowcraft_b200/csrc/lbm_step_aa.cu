@@ -811,11 +811,11 @@ static cudaError_t bulk_aa_t(void* f, const uint32_t* bits, const Geom& g, const
     }
     dim3 block(32, kBulkRows, 1);
     dim3 grid((unsigned)((g.nx + 63) / 64), (unsigned)((g.ny + kBulkRows - 1) / kBulkRows), 1);
-    const BoundarySpan bs = with_slabs(bnd, grid.x, grid.y);
-    grid.z = (unsigned)(zc > 0 ? zc : 0) + bs.slabs;
-    ++*launched;
-    return launch_step_kernel(odd ? k_bulk_pairs_aa<Q, S, true> : k_bulk_pairs_aa<Q, S, false>, grid, block, s,
-                              bs.chained, base, bits, g, p, pp, z0, dv, sd, bs);
+    const auto kernel = odd ? k_bulk_pairs_aa<Q, S, true> : k_bulk_pairs_aa<Q, S, false>;
+    return launch_with_slabs(bnd, grid.x, grid.y, zc > 0 ? zc : 0, launched, [&](const BoundarySpan& bs, unsigned layers) {
+        grid.z = layers + bs.slabs;
+        return launch_step_kernel(kernel, grid, block, s, bs.chained, base, bits, g, p, pp, z0, dv, sd, bs);
+    });
 }
 
 template <int Q, class S>
@@ -840,11 +840,12 @@ static cudaError_t bulk_aa_learned_t(void* f, const uint32_t* bits, const Geom& 
         }
         dim3 block(32, kBulkRows, 1);
         dim3 grid((unsigned)((g.nx + 63) / 64), (unsigned)((g.ny + kBulkRows - 1) / kBulkRows), 1);
-        const BoundarySpan bs = with_slabs(bnd, grid.x, grid.y);
-        grid.z = (unsigned)(zc > 0 ? zc : 0) + bs.slabs;
-        ++*launched;
-        return launch_step_kernel(odd ? k_bulk_pairs_aa_learned<Q, S, true> : k_bulk_pairs_aa_learned<Q, S, false>,
-                                  grid, block, s, bs.chained, base, bits, g, p, pp, z0, dv, sd, cl, bs);
+        const auto kernel = odd ? k_bulk_pairs_aa_learned<Q, S, true> : k_bulk_pairs_aa_learned<Q, S, false>;
+        return launch_with_slabs(bnd, grid.x, grid.y, zc > 0 ? zc : 0, launched,
+                                 [&](const BoundarySpan& bs, unsigned layers) {
+            grid.z = layers + bs.slabs;
+            return launch_step_kernel(kernel, grid, block, s, bs.chained, base, bits, g, p, pp, z0, dv, sd, cl, bs);
+        });
     }
 }
 

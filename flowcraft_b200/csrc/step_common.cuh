@@ -7,6 +7,7 @@
 #include "lbm_internal.h"
 #include "storage.cuh"
 
+#include <algorithm>
 #include <type_traits>
 
 namespace fc {
@@ -72,11 +73,29 @@ __device__ __forceinline__ bool boundary_block(const BoundarySpan& b, uint32_t& 
     return true;
 }
 
-// Host: the span with the slabs of gx x gy blocks its entries need.
-inline BoundarySpan with_slabs(BoundarySpan b, unsigned gx, unsigned gy) {
+// Host: the launches of a step's `layers` layers and the entries of `b`, in
+// slabs of gx x gy blocks ahead of the layers: launch(span, layers) enqueues
+// one kernel of span.slabs + layers block layers. Normally that is one; a grid
+// holds 65535 block layers, so entries that do not fit beside the layers (very
+// tall, narrow lattices) go out in launches of their own first.
+template <class F>
+cudaError_t launch_with_slabs(BoundarySpan b, unsigned gx, unsigned gy, unsigned layers, int* launched, F&& launch) {
+    constexpr size_t kMost = 65535;
     const size_t per = (size_t)gx * gy * 32 * kBulkRows;
-    b.slabs = b.end > b.begin ? (unsigned)((b.end - b.begin + per - 1) / per) : 0u;
-    return b;
+    for (;;) {
+        const size_t slabs = b.end > b.begin ? (b.end - b.begin + per - 1) / per : 0;
+        const bool whole = slabs + layers <= kMost;
+        if (whole && slabs + layers == 0) return cudaSuccess;
+        BoundarySpan part = b;
+        part.slabs = (unsigned)(whole ? slabs : std::min(slabs, kMost));
+        if (part.slabs * per < b.end - b.begin) part.end = (uint32_t)(b.begin + part.slabs * per);
+        const cudaError_t e = launch(part, whole ? layers : 0u);
+        if (e != cudaSuccess) return e;
+        ++*launched;
+        if (whole) return cudaSuccess;
+        b.begin = part.end;
+        b.chained = false;
+    }
 }
 
 template <int Q>
