@@ -68,6 +68,7 @@ struct fc_lbm {
     size_t stage_floats = 0;
     std::vector<uint8_t> solid_cpu;
     uint64_t steps_since_reset = 0;
+    uint64_t init_id = 0;  // of the last fc_lbm_init, unique in the process
     uint64_t launches = 0;
     // asynchronous field readback: a snapshot kernel on rb_stream into
     // d_snap, then the host copy; ev_snap marks the snapshot kernel's end
@@ -694,6 +695,8 @@ int fc_lbm_init(fc_lbm* h, const fc_grid_desc* grid, int32_t model, const fc_opt
         h->err = keep;
         return rc;
     }
+    static std::atomic<uint64_t> inits{0};
+    h->init_id = ++inits;
     h->cur = 0;
     h->steps_since_reset = 0;
     h->valid = true;
@@ -1515,8 +1518,9 @@ uint64_t fbits64(float f) {
 std::vector<uint64_t> batch_signature(const fc_lbm_batch* b) {
     std::vector<uint64_t> v{(uint64_t)b->rows, (uint64_t)b->mult};
     for (const fc_lbm* h : b->m) {
-        v.push_back((uint64_t)(uintptr_t)h->pop[0]);
-        v.push_back((uint64_t)(uintptr_t)h->pop[1]);
+        // stands for the geometry, the options and every device array: a
+        // re-initialized member may get the same addresses for another lattice
+        v.push_back(h->init_id);
         v.push_back((uint64_t)h->cur);
         v.push_back(fbits64(h->params.tau) | (fbits64(h->params.inlet_velocity) << 32));
         v.push_back(fbits64(h->params.smagorinsky_cs) | ((uint64_t)h->params.reverse_flow << 32) |
