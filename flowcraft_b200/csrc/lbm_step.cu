@@ -459,9 +459,13 @@ __device__ __forceinline__ void pairs_tile(const typename S::T* fin, typename S:
     const bool edge = (bx == 0) | (64 * bx + 64 - sh >= g.nx);
     if (shell && !face && !edge) return;  // an interior warp: done by k_bulk_tiles
 
-    // FP32: the one lane of a row end that holds an inlet or outlet cell finishes it alone
-    if (plane) plane_cell<Q, S>(fin, fout, g, p, plane == 1u ? x : x + 1, plane == 1u ? c : (size_t)c + 1);
-    if (!pair) return;
+    // FP32: the lane of a row end that holds an inlet or outlet cell finishes it alone
+    if (plane) plane_cell<Q, S>(fin, fout, g, p, plane & 1u ? x : x + 1, plane & 1u ? c : (size_t)c + 1);
+    if (!pair) {
+        // nx 2: both cells of the pair (after the first, when nothing else is live: no registers)
+        if (plane == 3u) plane_cell<Q, S>(fin, fout, g, p, x + 1, (size_t)c + 1);
+        return;
+    }
     float2 v[Q];
     if (!face) {
         if (pair != 3u && !edge) {  // one of the two is next to a wall (a boundary-list cell)
@@ -983,8 +987,11 @@ __global__ void __launch_bounds__(32 * ROWS, 32 / ROWS) k_bulk_pairs_batch(const
         const uint32_t c = (uint32_t)(row * g.nx + x);
         const bool face = (y == 0) | (y == g.ny - 1) | (z == 0) | (z == g.nz - 1);
         const bool edge = (bx == 0) | (64 * bx + 64 >= g.nx);
-        if (plane) plane_cell<Q, S>(fin, fout, g, p, plane == 1u ? x : x + 1, plane == 1u ? c : (size_t)c + 1);
-        if (!pair) continue;
+        if (plane) plane_cell<Q, S>(fin, fout, g, p, plane & 1u ? x : x + 1, plane & 1u ? c : (size_t)c + 1);
+        if (!pair) {
+            if (plane == 3u) plane_cell<Q, S>(fin, fout, g, p, x + 1, (size_t)c + 1);  // nx 2
+            continue;
+        }
         float2 v[Q];
         if (!face) {  // as k_bulk_pairs
             if (pair != 3u && !edge) {
