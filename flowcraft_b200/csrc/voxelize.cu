@@ -14,10 +14,11 @@
 //      pair, written in triangle order; a stable radix sort on the tile id
 //      groups them by tile keeping triangle order inside each tile, and a
 //      run-length encode gives each occupied tile its triangle list;
-//   3. raster: a block per box of 4x4x2 cells of an occupied tile. It tests
-//      the tile's triangles against the box and computes the distances of
-//      those that overlap it, many at a time; each cell's running signed
-//      distance, best normal projection and solid bit then follow the
+//   3. raster: a block per occupied tile where its list is short, else one per
+//      box of 4x4x2 cells, which tests the tile's triangles against the box and
+//      computes the distances of those that overlap it, many at a time. Each
+//      cell's running signed distance, best normal projection and solid bit
+//      follow the
 //      reference's update rule (Voxelizer.cpp:236-293) over the triangles
 //      whose box holds the cell, in index order, so every cell sees the same
 //      triangles in the same order as the CPU loop and rounds the same IEEE
@@ -254,17 +255,27 @@ struct GridDev {
     float ox, oy, oz;
 };
 
-// Status words of a call: error bits, and the tiles that hold a triangle.
+// Status words of a call: error bits, the tiles that hold a triangle, the
+// triangles in `big`, and the tiles with long lists.
 struct Status {
     int err;
-    unsigned occupied;
+    unsigned occupied, big, longest, long_tiles;
 };
 
-// Also marks every tile a triangle's box touches in `slot` (zeroed) and counts
-// the marked tiles.
+// Marks tile (x, y, z) in `slot`; 1 where it was not marked before.
+__device__ __forceinline__ unsigned mark_tile(uint32_t* __restrict__ slot, const GridDev& g, int x, int y, int z) {
+    uint32_t* m = slot + (((size_t)z * g.ty + y) * g.tx + x);
+    return __ldcg(m) == 0u && atomicExch(m, 1u) == 0u ? 1u : 0u;
+}
+
+// Also marks the tiles a triangle's box touches in `slot` (zeroed) and counts
+// the marked ones. A tile costs a thread a trip to memory, so the boxes of
+// more than kOwnTiles tiles go into the list `big` for k_tri_mark: two facets
+// across a 1024x512x512 grid took 316 ms with all of a triangle's tiles on its own thread.
+constexpr unsigned kOwnTiles = 32;
 __global__ void k_tri_prep(const float* __restrict__ pos, unsigned nv, const uint32_t* __restrict__ idx,
                            unsigned ntri, GridDev g, Tri* __restrict__ tris, unsigned long long* __restrict__ counts,
-                           uint32_t* __restrict__ slot, Status* __restrict__ st) {
+                           uint32_t* __restrict__ slot, uint32_t* __restrict__ big, Status* __restrict__ st) {
     const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t > ntri) return;
     if (t == ntri) {  // the scan's trailing slot, so offsets[ntri] is the pair total
@@ -313,18 +324,46 @@ __global__ void k_tri_prep(const float* __restrict__ pos, unsigned nv, const uin
         if (lo0 <= hi0 && lo1 <= hi1 && lo2 <= hi2) {
             cnt = (unsigned long long)(hi0 / kTile - lo0 / kTile + 1) * (hi1 / kTile - lo1 / kTile + 1) *
                   (hi2 / kTile - lo2 / kTile + 1);
-            unsigned fresh = 0;
-            for (int z = lo2 / kTile; z <= hi2 / kTile; ++z)
-                for (int y = lo1 / kTile; y <= hi1 / kTile; ++y)
-                    for (int x = lo0 / kTile; x <= hi0 / kTile; ++x) {
-                        uint32_t* m = slot + (((size_t)z * g.ty + y) * g.tx + x);
-                        if (__ldcg(m) == 0u && atomicExch(m, 1u) == 0u) ++fresh;
-                    }
-            if (fresh) atomicAdd(&st->occupied, fresh);
+            if (cnt > kOwnTiles) {
+                big[atomicAdd(&st->big, 1u)] = t;
+            } else {
+                unsigned fresh = 0;
+                for (int z = lo2 / kTile; z <= hi2 / kTile; ++z)
+                    for (int y = lo1 / kTile; y <= hi1 / kTile; ++y)
+                        for (int x = lo0 / kTile; x <= hi0 / kTile; ++x) fresh += mark_tile(slot, g, x, y, z);
+                if (fresh) atomicAdd(&st->occupied, fresh);
+            }
         }
     }
     tris[t] = r;
     counts[t] = cnt;
+}
+
+// Marks the tiles of the triangles in `big`, kMarkParts warps each (the ones
+// past a box's tiles leave at once), a tile per lane. Not where the call is
+// about to be refused for its number of pairs, which these boxes make up.
+constexpr unsigned kMarkParts = 128;
+constexpr unsigned kMarkBlocks = 148 * 8;
+__global__ void __launch_bounds__(256) k_tri_mark(const Tri* __restrict__ tris, const uint32_t* __restrict__ big,
+                                                  const unsigned long long* __restrict__ pairs, GridDev g,
+                                                  uint32_t* __restrict__ slot, Status* __restrict__ st) {
+    const unsigned lane = threadIdx.x & 31u;
+    const size_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, warps = (gridDim.x * blockDim.x) >> 5;
+    const size_t items = (size_t)st->big * kMarkParts;
+    if (items == 0 || *pairs > (unsigned long long)INT32_MAX) return;
+    for (size_t i = warp; i < items; i += warps) {
+        const Tri& r = tris[big[i / kMarkParts]];
+        const int x0 = r.lo[0] / kTile, y0 = r.lo[1] / kTile, z0 = r.lo[2] / kTile;
+        const unsigned wx = r.hi[0] / kTile - x0 + 1, wy = r.hi[1] / kTile - y0 + 1, wz = r.hi[2] / kTile - z0 + 1;
+        const size_t count = (size_t)wx * wy * wz;
+        unsigned fresh = 0;
+        for (size_t k = (i % kMarkParts) * 32 + lane; k < count; k += kMarkParts * 32) {
+            const size_t row = k / wx;
+            fresh += mark_tile(slot, g, x0 + (int)(k - row * wx), y0 + (int)(row % wy), z0 + (int)(row / wy));
+        }
+        fresh = __reduce_add_sync(0xffffffffu, fresh);
+        if (lane == 0 && fresh) atomicAdd(&st->occupied, fresh);
+    }
 }
 
 __global__ void k_tri_emit(const Tri* __restrict__ tris, const unsigned long long* __restrict__ offsets,
@@ -349,14 +388,105 @@ __global__ void k_tri_emit(const Tri* __restrict__ tris, const unsigned long lon
 
 // ---- 3. raster ----
 
-// slot[tile] = its place in the list of occupied tiles + 1 (0: no triangle)
-__global__ void k_tile_slots(const uint32_t* __restrict__ run_tile, unsigned runs, uint32_t* __restrict__ slot) {
+// A tile with at most kShortList triangles is rasterized by one block, one with
+// more by a block per box (k_vox_raster).
+// Whole call on a B200, every tile by one block / by boxes, average list in
+// brackets: two facets across 640x320x320 (2) 6.5 / 13.7 ms; icosphere of 1280
+// triangles at 640 cells (4) 0.84 / 1.23 ms, of 20480 (20) 0.98 / 1.12, of 5120
+// at 128 cells (87) 0.54 / 0.48; wing at 256 cells (54) 0.62 / 0.56; aircraft at
+// 640 (274) 2.11 / 0.86, at 96 (6781) 10.7 / 2.1.
+constexpr unsigned kShortList = 32, kLongestList = 512;
+
+// slot[tile] = its place in the list of occupied tiles + 1 (0: no triangle);
+// the places of the tiles with long lists in `long_tiles`: more than
+// kLongestList triangles from the front, the others from the back.
+__global__ void k_tile_slots(const uint32_t* __restrict__ run_tile, const uint32_t* __restrict__ run_len,
+                             unsigned runs, uint32_t* __restrict__ slot, uint32_t* __restrict__ long_tiles,
+                             Status* __restrict__ st) {
     const unsigned k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < runs) slot[run_tile[k]] = k + 1u;
+    if (k >= runs) return;
+    slot[run_tile[k]] = k + 1u;
+    if (run_len[k] > kLongestList)
+        long_tiles[atomicAdd(&st->longest, 1u)] = k;
+    else if (run_len[k] > kShortList)
+        long_tiles[runs - 1u - atomicAdd(&st->long_tiles, 1u)] = k;
 }
 
-// Block 16k + w: box w (4x4x2 cells, one per lane) of occupied tile k. The
-// list order matters only to the running state, not to a triangle's distance
+// A cell's running state, and the update by one more triangle of its list
+// (distance, signed normal projection; a NaN distance changes nothing).
+struct CellState {
+    float sd = INFINITY, bp = -1.0f;
+    bool sol = false;
+    __device__ __forceinline__ void add(float dist, float nd, float tie, float cr) {
+        const float and_ = fabsf(nd);
+        const float bd = fabsf(sd);
+        // Voxelizer.cpp:258-290: a clearly nearer triangle replaces the
+        // cell's distance; within the tie tolerance the one whose normal
+        // points more directly at the cell decides the sign
+        if (dist + tie < bd) {
+            sd = nd < 0.0f ? -dist : dist;
+            bp = and_;
+        } else if (dist <= bd + tie) {
+            if (and_ > bp) {
+                const float md = dist < bd ? dist : bd;
+                sd = nd < 0.0f ? -md : md;
+                bp = and_;
+            } else if (dist < bd) {
+                sd = sd < 0.0f ? -dist : dist;
+            }
+        }
+        if (dist <= cr) sol = true;
+    }
+};
+
+// Short lists: a block per tile, two cells per thread, the triangles staged
+// through shared memory in list order. What a block costs before and after its
+// triangles is paid once per tile here, once per box in the other form.
+constexpr int kRasterThreads = 256;
+__device__ __forceinline__ void raster_tile(unsigned tile_at, uint32_t tile, unsigned count,
+                                            const uint32_t* __restrict__ list, const Tri* __restrict__ tris,
+                                            const GridDev& g, uint8_t* __restrict__ solid, float* __restrict__ sdf,
+                                            uint8_t* __restrict__ mask) {
+    __shared__ Tri s_tri[kShortList];
+    if (threadIdx.x < count) s_tri[threadIdx.x] = tris[list[threadIdx.x]];
+    __syncthreads();
+    const int x = (int)(tile % (uint32_t)g.tx) * kTile + (threadIdx.x & 7);
+    const int y = (int)((tile / (uint32_t)g.tx) % (uint32_t)g.ty) * kTile + ((threadIdx.x >> 3) & 7);
+    const int z0 = (int)(tile / ((uint32_t)g.tx * (uint32_t)g.ty)) * kTile;
+    const float tie = g.cs * 1e-3f;
+#pragma unroll 1
+    for (int c = threadIdx.x; c < kTileCells; c += kRasterThreads) {
+        const int z = z0 + (c >> 6);
+        const bool inside = x < g.nx && y < g.ny && z < g.nz;
+        // CellCenter: world x from grid y, world y from grid x (VoxelGrid.h:43-56)
+        const V3 at{g.ox + ((float)y + 0.5f) * g.cs, g.oy + ((float)x + 0.5f) * g.cs, g.oz + ((float)z + 0.5f) * g.cs};
+        CellState cell;
+        for (unsigned k = 0; inside && k < count; ++k) {
+            const Tri& r = s_tri[k];
+            if (x < r.lo[0] || x > r.hi[0] || y < r.lo[1] || y > r.hi[1] || z < r.lo[2] || z > r.hi[2]) continue;
+            const V3 a{r.a[0], r.a[1], r.a[2]}, b{r.b[0], r.b[1], r.b[2]}, d{r.c[0], r.c[1], r.c[2]};
+            const V3 diff = vsub(at, closest_on_triangle(at, a, b, d));
+            cell.add(vlen(diff), vdot(diff, V3{r.n[0], r.n[1], r.n[2]}), tie, g.cr);
+        }
+        const unsigned fluid = __ballot_sync(0xffffffffu, inside && !cell.sol);
+        if (inside) {
+            const size_t i = ((size_t)z * g.ny + y) * g.nx + x;
+            solid[i] = cell.sol ? 1 : 0;
+            sdf[i] = cell.sd;
+        }
+        const unsigned lane = threadIdx.x & 31u;
+        if (lane < 4) {  // the warp's four rows, eight bits each
+            const unsigned r = (fluid >> (8 * lane)) & 0xffu;
+            reinterpret_cast<uint16_t*>(mask)[(size_t)tile_at * kTileRows + (c >> 5) * 4 + lane] =
+                (uint16_t)((r & 0xfu) | (r >> 4) << 8);
+        }
+    }
+}
+
+// The first 16 x most blocks take the tiles with long lists, box by box: block
+// 16k + w box w (4x4x2 cells, one per lane) of the k-th such tile, the longest
+// lists first, since a box of thousands of triangles outlasts the rest. The
+// other blocks take the short ones and fill in behind. The list order matters only to the running state, not to a triangle's distance
 // from a cell, so all threads compute the distances of a chunk of the box's
 // triangles at once, one (triangle, cell) pair each, for the cells inside the
 // triangle's own box only; warp 0 then applies the update rule to them in
@@ -368,24 +498,32 @@ __global__ void k_tile_slots(const uint32_t* __restrict__ run_tile, unsigned run
 // chain of list, box and triangle loads, at 46 % of the warp slots and 35 % of
 // the issue slots; a branch-free closest_on_triangle measured the same. Also
 // writes the fluid bits of the box's rows, which the flood fill runs on.
-constexpr int kRasterThreads = 256;
 constexpr int kRasterWarps = kRasterThreads / 32;
 constexpr int kRasterChunk = 64;  // distances kept at a time
 constexpr int kTileBoxes = kTileCells / 32;
-__global__ void __launch_bounds__(kRasterThreads) k_vox_raster(const Tri* __restrict__ tris,
-                                                               const uint32_t* __restrict__ tile_tris,
-                                                               const uint32_t* __restrict__ run_tile,
-                                                               const uint32_t* __restrict__ run_len,
-                                                               const unsigned long long* __restrict__ run_off,
-                                                               GridDev g, uint8_t* __restrict__ solid,
-                                                               float* __restrict__ sdf, uint8_t* __restrict__ mask) {
+__global__ void __launch_bounds__(kRasterThreads) k_vox_raster(
+    const Tri* __restrict__ tris, const uint32_t* __restrict__ tile_tris, const uint32_t* __restrict__ run_tile,
+    const uint32_t* __restrict__ run_len, const unsigned long long* __restrict__ run_off, unsigned runs,
+    const uint32_t* __restrict__ long_tiles, unsigned most, const Status* __restrict__ st, GridDev g,
+    uint8_t* __restrict__ solid, float* __restrict__ sdf, uint8_t* __restrict__ mask) {
+    unsigned k;
+    if (blockIdx.x >= kTileBoxes * most) {
+        k = blockIdx.x - kTileBoxes * most;
+        if (run_len[k] <= kShortList)
+            raster_tile(k, run_tile[k], run_len[k], tile_tris + run_off[k], tris, g, solid, sdf, mask);
+        return;
+    }
+    k = blockIdx.x / kTileBoxes;
+    const unsigned longest = st->longest;
+    if (k >= longest + st->long_tiles) return;
+    k = long_tiles[k < longest ? k : runs - 1u - (k - longest)];
     __shared__ uint32_t s_hit[kRasterThreads];
     __shared__ float2 s_res[kRasterChunk][32];  // distance and signed normal projection; NaN: outside the box
     __shared__ unsigned s_count[kRasterWarps];
     // the chunk's triangles: their cells of the box (first cell and size per
     // axis) and the pairs up to and including each
     __shared__ uint32_t s_clip[kRasterChunk], s_pairs[kRasterChunk], s_part[kRasterChunk / 32];
-    const unsigned k = blockIdx.x / kTileBoxes, w = blockIdx.x % kTileBoxes;
+    const unsigned w = blockIdx.x % kTileBoxes;
     const uint32_t tile = run_tile[k];
     const unsigned count = run_len[k];
     const uint32_t* list = tile_tris + run_off[k];
@@ -398,8 +536,7 @@ __global__ void __launch_bounds__(kRasterThreads) k_vox_raster(const Tri* __rest
     const int x = bx + (lane & 3), y = by + ((lane >> 2) & 3), z = bz + (lane >> 4);
     const bool inside = x < g.nx && y < g.ny && z < g.nz;
     const float tie = g.cs * 1e-3f;
-    float sd = INFINITY, bp = -1.0f;
-    bool sol = false;
+    CellState cell;
     const bool empty = bx >= g.nx || by >= g.ny || bz >= g.nz;  // a box behind the grid's edge
     for (unsigned base = 0; base < count && !empty; base += kRasterThreads) {
         // the list's next triangles that overlap the box, in list order
@@ -478,36 +615,18 @@ __global__ void __launch_bounds__(kRasterThreads) k_vox_raster(const Tri* __rest
             if (warp == 0) {
 #pragma unroll 4
                 for (unsigned h = c0; h < c1; ++h) {
-                    const float dist = s_res[h - c0][lane].x, nd = s_res[h - c0][lane].y;
-                    const float and_ = fabsf(nd);
-                    const float bd = fabsf(sd);
-                    // Voxelizer.cpp:258-290: a clearly nearer triangle replaces the
-                    // cell's distance; within the tie tolerance the one whose normal
-                    // points more directly at the cell decides the sign
-                    if (dist + tie < bd) {
-                        sd = nd < 0.0f ? -dist : dist;
-                        bp = and_;
-                    } else if (dist <= bd + tie) {
-                        if (and_ > bp) {
-                            const float md = dist < bd ? dist : bd;
-                            sd = nd < 0.0f ? -md : md;
-                            bp = and_;
-                        } else if (dist < bd) {
-                            sd = sd < 0.0f ? -dist : dist;
-                        }
-                    }
-                    if (dist <= g.cr) sol = true;
+                    cell.add(s_res[h - c0][lane].x, s_res[h - c0][lane].y, tie, g.cr);
                 }
             }
             __syncthreads();
         }
     }
     if (warp != 0) return;
-    const unsigned fluid = __ballot_sync(0xffffffffu, inside && !sol);
+    const unsigned fluid = __ballot_sync(0xffffffffu, inside && !cell.sol);
     if (inside) {
         const size_t i = ((size_t)z * g.ny + y) * g.nx + x;
-        solid[i] = sol ? 1 : 0;
-        sdf[i] = sd;
+        solid[i] = cell.sol ? 1 : 0;
+        sdf[i] = cell.sd;
     }
     if (lane < 8)  // row (y, z) of the box: four bits
         mask[((size_t)k * kTileRows + (lz + (lane >> 2)) * kTile + ly + (lane & 3)) * 2 + (w & 1)] =
@@ -908,14 +1027,14 @@ int voxelize_on_device(const float* d_pos, size_t nv, const uint32_t* d_idx, siz
 
     // the first half: triangle records, tile marks, and the sizes of the rest
     Status* d_st = nullptr;
-    uint32_t* slot = nullptr;
+    uint32_t *slot = nullptr, *big = nullptr;
     Tri* tris = nullptr;
     unsigned long long *counts = nullptr, *offsets = nullptr;
     void* tmp = nullptr;
     size_t tmp_bytes = 0;
     if (ntri > 0)
         VX_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, counts, offsets, (int64_t)ntri + 1, s));
-    VX_TRY(sc.get_all({{&d_st, 1}, {&slot, ntiles}, {&tris, ntri}, {&counts, (size_t)ntri + 1},
+    VX_TRY(sc.get_all({{&d_st, 1}, {&slot, ntiles}, {&big, ntri}, {&tris, ntri}, {&counts, (size_t)ntri + 1},
                        {&offsets, (size_t)ntri + 1}, {&tmp, tmp_bytes}}));
     VX_TRY(cudaMemsetAsync(d_st, 0, sizeof(Status), s));
     VX_TRY(cudaMemsetAsync(slot, 0, sizeof(uint32_t) * ntiles, s));
@@ -924,10 +1043,12 @@ int voxelize_on_device(const float* d_pos, size_t nv, const uint32_t* d_idx, siz
     Answer own;
     Answer* ans = host_answer(&own);
     if (ntri > 0) {
-        k_tri_prep<<<(ntri + 1 + 255) / 256, 256, 0, s>>>(d_pos, (unsigned)nv, d_idx, ntri, g, tris, counts, slot,
+        k_tri_prep<<<(ntri + 1 + 255) / 256, 256, 0, s>>>(d_pos, (unsigned)nv, d_idx, ntri, g, tris, counts, slot, big,
                                                           d_st);
         VX_TRY(cudaGetLastError());
         VX_TRY(cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, counts, offsets, (int64_t)ntri + 1, s));
+        k_tri_mark<<<kMarkBlocks, 256, 0, s>>>(tris, big, offsets + ntri, g, slot, d_st);
+        VX_TRY(cudaGetLastError());
         VX_TRY(cudaMemcpyAsync(&ans->pairs, offsets + ntri, sizeof(pairs), cudaMemcpyDeviceToHost, s));
         VX_TRY(cudaMemcpyAsync(&ans->st, d_st, sizeof(st), cudaMemcpyDeviceToHost, s));
         VX_RC(wait_on(s));
@@ -940,7 +1061,8 @@ int voxelize_on_device(const float* d_pos, size_t nv, const uint32_t* d_idx, siz
     const unsigned runs = st.occupied;  // the runs of equal tile ids after the sort
     const uint64_t nodes = ntiles + (uint64_t)runs * kTileNodes;
     const bool wide = nodes >= 0xffffffffull;
-    uint32_t *k0 = nullptr, *k1 = nullptr, *v0 = nullptr, *v1 = nullptr, *run_tile = nullptr, *run_len = nullptr;
+    uint32_t *k0 = nullptr, *k1 = nullptr, *v0 = nullptr, *v1 = nullptr;
+    uint32_t *run_tile = nullptr, *run_len = nullptr, *long_tiles = nullptr;
     unsigned long long* run_off = nullptr;
     int* d_runs = nullptr;
     uint8_t *mask = nullptr, *tile_reached = nullptr, *row_reached = nullptr;
@@ -954,6 +1076,7 @@ int voxelize_on_device(const float* d_pos, size_t nv, const uint32_t* d_idx, siz
         VX_TRY(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, run_len, run_off, (int64_t)runs, s));
     }
     VX_TRY(sc.get_all({{&k0, pairs}, {&k1, pairs}, {&v0, pairs}, {&v1, pairs}, {&run_tile, runs}, {&run_len, runs},
+                       {&long_tiles, runs},
                        {&run_off, runs}, {&d_runs, 1}, {&mask, (size_t)runs * kTileRows * 2}, {&tile_reached, ntiles},
                        {&row_reached, (size_t)runs * kTileRows}, {&labels, nodes * (wide ? 8 : 4)},
                        {&tmp, std::max(sort_bytes, std::max(rle_bytes, scan_bytes))}}));
@@ -965,17 +1088,16 @@ int voxelize_on_device(const float* d_pos, size_t nv, const uint32_t* d_idx, siz
         VX_TRY(cub::DeviceRunLengthEncode::Encode(tmp, rle_bytes, kb.Current(), run_tile, run_len, d_runs, (int)pairs,
                                                    s));
         VX_TRY(cub::DeviceScan::ExclusiveSum(tmp, scan_bytes, run_len, run_off, (int64_t)runs, s));
-        k_tile_slots<<<(runs + 255) / 256, 256, 0, s>>>(run_tile, runs, slot);
+        k_tile_slots<<<(runs + 255) / 256, 256, 0, s>>>(run_tile, run_len, runs, slot, long_tiles, d_st);
         VX_TRY(cudaGetLastError());
-        // a tile's boxes next to each other in the launch (they read one list);
-        // a grid holds 2^31 - 1 blocks, so very many tiles take several launches
-        constexpr unsigned kLaunchTiles = (unsigned)INT32_MAX / kTileBoxes;
-        for (unsigned first = 0; first < runs; first += std::min(kLaunchTiles, runs - first)) {
-            k_vox_raster<<<kTileBoxes * std::min(kLaunchTiles, runs - first), kRasterThreads, 0, s>>>(
-                tris, vb.Current(), run_tile + first, run_len + first, run_off + first, g, d_solid, d_sdf,
-                mask + (size_t)first * kTileRows * 2);
-            VX_TRY(cudaGetLastError());
-        }
+        // as many tiles as can have a long list, a block per box, and a block per tile:
+        // below 2^31 blocks (pairs < 2^31, and runs <= 2^29, since a grid of below 2^32
+        // cells has at least eight for each of its tiles)
+        const unsigned most = std::min<unsigned>(runs, (unsigned)(pairs / (kShortList + 1)));
+        k_vox_raster<<<kTileBoxes * most + runs, kRasterThreads, 0, s>>>(tris, vb.Current(), run_tile, run_len, run_off,
+                                                                       runs, long_tiles, most, d_st, g, d_solid, d_sdf,
+                                                                       mask);
+        VX_TRY(cudaGetLastError());
     }
     VX_RC(wide ? flood(g, ntiles, runs, slot, mask, run_tile, reinterpret_cast<unsigned long long*>(labels),
                        tile_reached, row_reached, d_st, s)
