@@ -1475,9 +1475,10 @@ struct fc_lbm_batch {
     unsigned long long total = 0;   // bulk work items
     unsigned long long btotal = 0;  // boundary-list entries
     int rows = 8, mult = 1, grid = 0;  // rows 0: every member's own step launches
-    cudaGraphExec_t exec = nullptr;
+    cudaGraphExec_t exec = nullptr;       // two steps
+    cudaGraphExec_t exec_long = nullptr;  // batch_long_steps(): rows 0 only
     // forked streams of the per-member bulk launches (rows 0)
-    static constexpr int kFork = 16;
+    static constexpr int kFork = 16;  // at most, and one per member
     cudaStream_t fork[kFork] = {};
     cudaEvent_t ev_fork = nullptr, ev_join[kFork] = {};
     std::vector<uint64_t> sig;  // member state the descriptors and the graph were built for
@@ -1527,6 +1528,13 @@ std::vector<uint64_t> batch_signature(const fc_lbm_batch* b) {
                     ((uint64_t)h->params.free_slip_y << 33) | ((uint64_t)h->params.free_slip_z << 34));
     }
     return v;
+}
+
+void batch_drop_graphs(fc_lbm_batch* b) {
+    for (cudaGraphExec_t* e : {&b->exec, &b->exec_long}) {
+        if (*e) cudaGraphExecDestroy(*e);
+        *e = nullptr;
+    }
 }
 
 // Descriptors of every member for the current block shape, uploaded.
@@ -1643,15 +1651,25 @@ int batch_members(fc_lbm_batch* b, int parity, int steps) {
     return bcuda(b, e, "batch member step");
 }
 
-// Whether the members' launches go out one by one rather than as graph
-// replays of two steps: where a launch takes longer on the device than on the
-// host (about 2.5 us), the host stays ahead, and no join comes between pairs
-// of steps.
-bool batch_members_direct(const fc_lbm_batch* b) {
+// Whether the members' steps take longer on the device than their launches on
+// the host (about 2.5 us each).
+bool batch_members_large(const fc_lbm_batch* b) {
     size_t cells = 0;
     for (const fc_lbm* h : b->m) cells += h->g.n;
-    return b->rows == 0 && cells / b->m.size() >= (size_t(1) << 17);
+    return cells / b->m.size() >= (size_t(1) << 17);
 }
+
+// Steps in the long graph of the members' launches (an even number, about
+// kLongNodes launches). It is for calls of more than kDirectLaunches launches:
+// one by one those fill the driver's launch queues, and the caller is held
+// until the device has caught up (16 lattices of 64x32x32 to 256x128x128, 1000
+// steps, 494 ms on the device: the call returned after 237 ms, with the graph
+// after 1.7). Below, a graph would cost a first call more than it saves: 2 ms to
+// build, against 2.6 ms for 1024 launches. Between graphs of 256 launches the
+// joins do not show (0.482 ms per step both ways; 16 of 64x32x32 26.6 us per
+// step, in graphs of two steps 33.6).
+constexpr int kLongNodes = 256, kDirectLaunches = 1024;
+int batch_long_steps(const fc_lbm_batch* b) { return std::max(2, kLongNodes / (int)b->m.size() / 2 * 2); }
 
 // One step of every member (parity relative to the members' current sets).
 int batch_step_direct(fc_lbm_batch* b, int parity) {
@@ -1668,37 +1686,35 @@ int batch_step_direct(fc_lbm_batch* b, int parity) {
     return FC_LBM_OK;
 }
 
-int batch_prepare(fc_lbm_batch* b, bool want_graph) {
+int batch_prepare(fc_lbm_batch* b) {
     const std::vector<uint64_t> sig = batch_signature(b);
-    if (sig != b->sig) {
-        if (b->exec) {
-            cudaGraphExecDestroy(b->exec);
-            b->exec = nullptr;
-        }
-        FC_RC(batch_build(b));
-        b->sig = sig;
+    if (sig == b->sig) return FC_LBM_OK;
+    batch_drop_graphs(b);
+    FC_RC(batch_build(b));
+    b->sig = sig;
+    return FC_LBM_OK;
+}
+
+// `steps` steps as a graph, an even number: a replay leaves every member on
+// its own set.
+int batch_graph(fc_lbm_batch* b, cudaGraphExec_t& exec, int steps) {
+    if (exec) return FC_LBM_OK;
+    cudaGraph_t graph = nullptr;
+    FB_TRY(b, cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal), "begin capture");
+    int rc = FC_LBM_OK;
+    if (b->rows == 0)
+        rc = batch_members(b, 0, steps);
+    else
+        for (int k = 0; k < steps && rc == FC_LBM_OK; ++k) rc = batch_step_direct(b, k & 1);
+    const cudaError_t e = cudaStreamEndCapture(b->stream, &graph);
+    if (rc != FC_LBM_OK) {
+        if (graph) cudaGraphDestroy(graph);
+        return rc;
     }
-    if (want_graph && !b->exec) {
-        // two steps, one of each parity: a replay leaves every member on its own set
-        cudaGraph_t graph = nullptr;
-        FB_TRY(b, cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal), "begin capture");
-        int rc = FC_LBM_OK;
-        if (b->rows == 0) {
-            rc = batch_members(b, 0, 2);
-        } else {
-            rc = batch_step_direct(b, 0);
-            if (rc == FC_LBM_OK) rc = batch_step_direct(b, 1);
-        }
-        const cudaError_t e = cudaStreamEndCapture(b->stream, &graph);
-        if (rc != FC_LBM_OK) {
-            if (graph) cudaGraphDestroy(graph);
-            return rc;
-        }
-        FB_TRY(b, e, "end capture");
-        const cudaError_t ie = cudaGraphInstantiate(&b->exec, graph, 0);
-        cudaGraphDestroy(graph);
-        FB_TRY(b, ie, "instantiate graph");
-    }
+    FB_TRY(b, e, "end capture");
+    const cudaError_t ie = cudaGraphInstantiate(&exec, graph, 0);
+    cudaGraphDestroy(graph);
+    FB_TRY(b, ie, "instantiate graph");
     return FC_LBM_OK;
 }
 
@@ -1777,7 +1793,7 @@ int fc_lbm_batch_create(fc_lbm* const* members, int32_t count, fc_lbm_batch** ou
     cudaError_t e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming);
-    for (int j = 0; j < fc_lbm_batch::kFork && e == cudaSuccess; ++j) {
+    for (int j = 0; j < std::min(count, fc_lbm_batch::kFork) && e == cudaSuccess; ++j) {
         e = cudaStreamCreateWithFlags(&b->fork[j], cudaStreamNonBlocking);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_join[j], cudaEventDisableTiming);
     }
@@ -1794,7 +1810,7 @@ void fc_lbm_batch_destroy(fc_lbm_batch* b) {
     if (!b) return;
     DeviceGuard dg(b->device);
     if (b->stream) cudaStreamSynchronize(b->stream);
-    if (b->exec) cudaGraphExecDestroy(b->exec);
+    batch_drop_graphs(b);
     if (b->d_lat) cudaFree(b->d_lat);
     if (b->ev) cudaEventDestroy(b->ev);
     if (b->ev_fork) cudaEventDestroy(b->ev_fork);
@@ -1817,14 +1833,22 @@ int fc_lbm_batch_step(fc_lbm_batch* b, int32_t n) {
     if (n == 0) return FC_LBM_OK;
     DeviceGuard dg(b->device);
     FC_RC(batch_enter(b));
-    if (batch_members_direct(b)) {
-        FC_RC(batch_members(b, 0, n));
-        batch_advance(b, n, 1);
-        return batch_leave(b);
+    int left = n;
+    const int many = batch_long_steps(b);
+    if (b->rows == 0 && left >= many && (long long)n * (long long)b->m.size() > kDirectLaunches) {
+        FC_RC(batch_prepare(b));
+        FC_RC(batch_graph(b, b->exec_long, many));
+        for (; left >= many; left -= many) FB_TRY(b, cudaGraphLaunch(b->exec_long, b->stream), "graph launch");
     }
-    FC_RC(batch_prepare(b, n >= 2));
-    for (int k = 0; k + 1 < n; k += 2) FB_TRY(b, cudaGraphLaunch(b->exec, b->stream), "graph launch");
-    if (n & 1) FC_RC(batch_step_direct(b, 0));
+    if (b->rows == 0 && batch_members_large(b)) {
+        // few launches, the host stays ahead of them, and no join comes between two steps
+        if (left > 0) FC_RC(batch_members(b, 0, left));
+    } else if (left > 0) {
+        FC_RC(batch_prepare(b));
+        if (left >= 2) FC_RC(batch_graph(b, b->exec, 2));
+        for (; left >= 2; left -= 2) FB_TRY(b, cudaGraphLaunch(b->exec, b->stream), "graph launch");
+        if (left) FC_RC(batch_step_direct(b, 0));
+    }
     batch_advance(b, n, b->rows == 0 ? 1 : 2);
     return batch_leave(b);
 }
@@ -1858,7 +1882,7 @@ int fc_lbm_batch_tune(fc_lbm_batch* b, int32_t steps, int32_t* rows, int32_t* gr
         if (rc != FC_LBM_OK) break;
         b->rows = r;
         b->mult = mu;
-        rc = batch_prepare(b, false);
+        rc = batch_prepare(b);
         for (int k = 0; k < 2 && rc == FC_LBM_OK; ++k) rc = batch_step_direct(b, k);  // warm-up
         if (rc == FC_LBM_OK) rc = bcuda(b, cudaEventRecord(t0, b->stream), "timing");
         if (r == 0 && rc == FC_LBM_OK)

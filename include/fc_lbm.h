@@ -416,7 +416,8 @@ FC_LBM_API int fc_lbm_particles_set(fc_lbm* h, const float* points, size_t point
  * learned closure) step together. Every step is one persistent bulk launch
  * over a work-list of the tiles of all members and one launch over all their
  * boundary lists, pairs of steps replayed as one CUDA graph; or, when that is
- * faster, each member's own step kernels, side by side on forked streams.
+ * faster, each member's own step kernels, side by side on forked streams (a
+ * long call as graphs of many steps).
  * Results are bit-identical to stepping every member with fc_lbm_step. The members keep
  * their own state and API; they must outlive the batch and must not step on
  * their own while a batch step is queued. */
@@ -425,8 +426,8 @@ typedef struct fc_lbm_batch fc_lbm_batch;
 FC_LBM_API int fc_lbm_batch_create(fc_lbm* const* members, int32_t count, fc_lbm_batch** out);
 FC_LBM_API void fc_lbm_batch_destroy(fc_lbm_batch* b);
 FC_LBM_API const char* fc_lbm_batch_last_error(const fc_lbm_batch* b);
-/* n steps of every member; asynchronous, ordered after and before the
- * members' own streams. An odd n leaves the next call to rebuild its graph. */
+/* n steps of every member; asynchronous for any n (the call does not wait
+ * for the device), ordered after and before the members' own streams. An odd n leaves the next call to rebuild its graph. */
 FC_LBM_API int fc_lbm_batch_step(fc_lbm_batch* b, int32_t n);
 /* The block shape of the batch's bulk launch: rows in {4, 8, 16} (a block is
  * 32 x rows threads over 64 x rows cells) with grid_mult in {1, 2} (a
