@@ -5,7 +5,8 @@
 // solid mask and SDF (for readback forces), the bit-packed bulk mask, the
 // compacted boundary list with its Bouzidi coefficients, a stream, and
 // pinned staging for transfers. Device memory is allocated in fc_lbm_init
-// and released in fc_lbm_shutdown; stepping and readback allocate nothing.
+// and released in fc_lbm_shutdown; stepping allocates nothing, and neither does
+// a blocking readback, but for the threads that copy a large one to the caller.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -431,8 +432,10 @@ int check_ready(fc_lbm* h) {
 // ring of slots, so that the kernel and the transfer of one run while host
 // threads copy others out of the pinned buffer: a fresh destination costs a
 // page fault every 4 KB. 50 steps of 191x97x83 and the 24.6 MB field on a B200
-// box: 5.32 ms with one chunk at a time and one thread, 3.61 so. A small download is one chunk, copied by the
-// caller's thread.
+// box: 5.32 ms with one chunk at a time and one thread, 3.61 so. A small
+// download is one chunk, copied by the caller's thread. Every wait sleeps once
+// it gets long (host_wait.h), so a download behind seconds of steps keeps no
+// core busy, and all of them end when one chunk fails or times out.
 constexpr int kSlots = 8;
 constexpr size_t kMinChunk = size_t(1) << 20;
 constexpr int kCopyThreads = 4;
@@ -470,7 +473,7 @@ int download(fc_lbm* h, void* dst, size_t bytes, size_t unit, Issue&& issue) {
     auto copy_chunk = [&](size_t j) {
         const int slot = (int)(j % kSlots);
         cudaError_t e = cudaErrorNotReady;
-        while (!failed.load() && issued.load(std::memory_order_acquire) <= j) std::this_thread::yield();
+        fc::wait_until([&] { return failed.load() || issued.load(std::memory_order_acquire) > j; });
         if (!failed.load()) e = fc::poll_until([&] { return cudaEventQuery(h->ev_slot[slot]); }, kTransferTimeoutMs);
         if (e != cudaSuccess) {
             int none = 0;
@@ -506,8 +509,8 @@ int download(fc_lbm* h, void* dst, size_t bytes, size_t unit, Issue&& issue) {
                 copy_chunk(j - kSlots);
             else
                 copy_missing(prev);
-            while (!failed.load() && copied[j % kSlots].load(std::memory_order_acquire) < prev)
-                std::this_thread::yield();
+            fc::wait_until(
+                [&] { return failed.load() || copied[j % kSlots].load(std::memory_order_acquire) >= prev; });
             if (failed.load()) break;
         }
         rc = enqueue(j);

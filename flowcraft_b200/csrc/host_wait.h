@@ -10,6 +10,8 @@
 // us, 6.70 ms so.
 #pragma once
 
+#include <cuda_runtime.h>
+
 #include <algorithm>
 #include <chrono>
 #include <thread>
@@ -35,6 +37,13 @@ cudaError_t poll_until(F&& done, long long timeout_ms) {
         else
             std::this_thread::sleep_for(std::chrono::nanoseconds(std::clamp<long long>(ns / 64, 20'000, 500'000)));
     }
+}
+
+// The same for a condition that another host thread makes true, and which is
+// sure to become true.
+template <class P>
+void wait_until(P&& ready) {
+    poll_until([&] { return ready() ? cudaSuccess : cudaErrorNotReady; }, -1);
 }
 
 }  // namespace fc
