@@ -91,9 +91,9 @@ __device__ __forceinline__ size_t out_slot(uint32_t c, int x, int y, int z, cons
     if constexpr (Odd) {
         const int tx = x + L::ex(I), ty = y + L::ey(I), tz = z + L::ez(I);
         if (tx >= 0 && ty >= 0 && tz >= 0 && tx < g.nx && ty < g.ny && tz < g.nz)
-            return (size_t)I * g.ps + (size_t)((long long)c + link_offset<Q>(I, g));
+            return (size_t)I * g.n + (size_t)((long long)c + link_offset<Q>(I, g));
     }
-    return (size_t)L::opp(I) * g.ps + c;
+    return (size_t)L::opp(I) * g.n + c;
 }
 
 // One interior bulk cell (the one-cell path of k_bulk_pairs).
@@ -104,15 +104,15 @@ __device__ __forceinline__ void aa_interior_cell(typename S::T* f, const Geom& g
     float v[Q];
     static_for<0, Q>([&](auto I) {
         constexpr int i = decltype(I)::value;
-        const size_t s = Odd ? (size_t)L::opp(i) * g.ps + (size_t)((long long)c - link_offset<Q>(i, g))
-                             : (size_t)i * g.ps + c;
+        const size_t s = Odd ? (size_t)L::opp(i) * g.n + (size_t)((long long)c - link_offset<Q>(i, g))
+                             : (size_t)i * g.n + c;
         v[i] = S::dec(ld_plain<S>(f + s), L::w(i));
     });
     if (collide<Q, S::kExact>(v, p.tau, p.cs)) atomicOr(diverged, 1);
     static_for<0, Q>([&](auto I) {
         constexpr int i = decltype(I)::value;
-        const size_t d = Odd ? (size_t)i * g.ps + (size_t)((long long)c + link_offset<Q>(i, g))
-                             : (size_t)L::opp(i) * g.ps + c;
+        const size_t d = Odd ? (size_t)i * g.n + (size_t)((long long)c + link_offset<Q>(i, g))
+                             : (size_t)L::opp(i) * g.n + c;
         f[d] = S::enc(v[i], L::w(i));
     });
 }
@@ -161,12 +161,12 @@ __device__ __forceinline__ void aa_row_end_cell(typename S::T* f, const Geom& g,
     }
     // the slot out_slot<Q, i, Odd> names, for the run-time direction
     const unsigned opp = i == 0 ? 0u : ((i - 1u) ^ 1u) + 1u;
-    size_t slot = (size_t)opp * g.ps + pc;
+    size_t slot = (size_t)opp * g.n + pc;
     if constexpr (Odd) {
         const int ex = (int)lattice_e_rt<Q, 0>(i), ey = (int)lattice_e_rt<Q, 1>(i), ez = (int)lattice_e_rt<Q, 2>(i);
         const int tx = px + ex, ty = y + ey, tz = z + ez;
         if (tx >= 0 && ty >= 0 && tz >= 0 && tx < g.nx && ty < g.ny && tz < g.nz)
-            slot = (size_t)i * g.ps + (size_t)((long long)pc + ex + (long long)ey * g.nx + (long long)ez * g.nxy);
+            slot = (size_t)i * g.n + (size_t)((long long)pc + ex + (long long)ey * g.nx + (long long)ez * g.nxy);
     }
     if (mine) f[slot] = S::enc(v, lattice_w_rt<Q>(i));
 }
@@ -234,13 +234,13 @@ __device__ __forceinline__ void aa_boundary_entry(typename S::T* f, const Bounda
         const size_t off = (size_t)link_offset<Q>(i, g);
         size_t sa;
         if (kind == kLinkStream) {  // f*_i(c - e_i)
-            sa = Odd ? (size_t)op * g.ps + (c - off) : (size_t)i * g.ps + c;
+            sa = Odd ? (size_t)op * g.n + (c - off) : (size_t)i * g.n + c;
         } else if (kind == kLinkEdge) {  // f*_m(c) for the mirrored / bounced m
             const int py = y - L::ey(i), pz = z - L::ez(i);
             const int m = edge_plane<Q, i>(py < 0 || py >= g.ny, pz < 0 || pz >= g.nz, p);
-            sa = (size_t)L::opp(m) * g.ps + c;
+            sa = (size_t)L::opp(m) * g.n + c;
         } else {  // f*_op(c); before an even step it sits in the solid neighbour c - e_i
-            sa = Odd ? (size_t)i * g.ps + c : (size_t)op * g.ps + (c - off);
+            sa = Odd ? (size_t)i * g.n + c : (size_t)op * g.n + (c - off);
         }
         const float va = S::dec(ld_plain<S>(f + sa), L::w(i));
         float r = va;
@@ -249,7 +249,7 @@ __device__ __forceinline__ void aa_boundary_entry(typename S::T* f, const Bounda
             const float2 kc = __ldg(bl.coef + slot);
             float vb;
             if (kind == kLinkBzNear) {  // f*_op(c + e_i)
-                const size_t sb = Odd ? (size_t)i * g.ps + (c + off) : (size_t)op * g.ps + c;
+                const size_t sb = Odd ? (size_t)i * g.n + (c + off) : (size_t)op * g.n + c;
                 vb = S::dec(ld_plain<S>(f + sb), L::w(i));
             } else {  // f*_i(c), kept from the previous step
                 vb = S::dec(bz[slot], L::w(i));
@@ -318,13 +318,13 @@ __device__ __forceinline__ void aa_boundary_entry_learned(typename S::T* f, cons
             const size_t off = (size_t)link_offset<Q>(i, g);
             size_t sa;
             if (kind == kLinkStream) {  // f*_i(c - e_i)
-                sa = Odd ? (size_t)op * g.ps + (c - off) : (size_t)i * g.ps + c;
+                sa = Odd ? (size_t)op * g.n + (c - off) : (size_t)i * g.n + c;
             } else if (kind == kLinkEdge) {  // f*_m(c) for the mirrored / bounced m
                 const int py = y - L::ey(i), pz = z - L::ez(i);
                 const int m = edge_plane<Q, i>(py < 0 || py >= g.ny, pz < 0 || pz >= g.nz, p);
-                sa = (size_t)L::opp(m) * g.ps + c;
+                sa = (size_t)L::opp(m) * g.n + c;
             } else {  // f*_op(c); before an even step it sits in the solid neighbour c - e_i
-                sa = Odd ? (size_t)i * g.ps + c : (size_t)op * g.ps + (c - off);
+                sa = Odd ? (size_t)i * g.n + c : (size_t)op * g.n + (c - off);
             }
             const float va = S::dec(ld_plain<S>(f + sa), L::w(i));
             float r = va;
@@ -333,7 +333,7 @@ __device__ __forceinline__ void aa_boundary_entry_learned(typename S::T* f, cons
                 const float2 kc = __ldg(bl.coef + slot);
                 float vb;
                 if (kind == kLinkBzNear) {  // f*_op(c + e_i)
-                    const size_t sb = Odd ? (size_t)i * g.ps + (c + off) : (size_t)op * g.ps + c;
+                    const size_t sb = Odd ? (size_t)i * g.n + (c + off) : (size_t)op * g.n + c;
                     vb = S::dec(ld_plain<S>(f + sb), L::w(i));
                 } else {  // f*_i(c), kept from the previous step
                     vb = S::dec(bz[slot], L::w(i));
@@ -377,7 +377,19 @@ __device__ __forceinline__ void aa_boundary_entry_learned(typename S::T* f, cons
 }  // namespace
 
 // Bulk cells (bulk mask) of lattices with even nx; see the file comment.
-template <int Q, class S, bool Odd>
+// WithList: also the boundary list, and chained steps (step_common.cuh). The
+// FP32 kernel has no register to spare for either and loses 2-5 % of its bulk
+// time, which is more than the list's own launch costs from aa_list_apart()
+// cells on: there the two run apart and unchained. B200, us per step, list
+// inside / apart: D3Q19 256x128x128 151 / 156, 384x192x192 437 / 441,
+// 512x256x256 979 / 976, 640x320x320 2009 / 1930, 1024x512x512 8315 / 7834;
+// D3Q15 256x128x128 136 / 139, 320x160x160 241 / 239, 640x320x320 1605 / 1580.
+// (The 16-bit kernels, plain and learned, are within 0.6 % at 1024x512x512.)
+template <int Q>
+constexpr size_t aa_list_apart() {
+    return Q == 19 ? size_t(1) << 25 : size_t(1) << 23;
+}
+template <int Q, class S, bool Odd, bool WithList>
 __global__ void __launch_bounds__(32 * kBulkRows, 4) k_bulk_pairs_aa(typename S::T* f,
                                                                    const uint32_t* __restrict__ bulk_bits, Geom g,
                                                                    StepParams p, PlanePtrs pp, int z0,
@@ -386,14 +398,17 @@ __global__ void __launch_bounds__(32 * kBulkRows, 4) k_bulk_pairs_aa(typename S:
     using L = Lattice<Q>;
     using T = typename S::T;
     using T2 = typename S::T2;
-    step_enter();
-    uint32_t e;
-    if (boundary_block(bnd, e)) {
-        if (e < bnd.end) aa_boundary_entry<Q, S, Odd>(f, bnd.list, e, g, p, diverged, sd);
-        return;
+    if constexpr (WithList) {
+        step_enter();
+        uint32_t e;
+        if (boundary_block(bnd, e)) {
+            if (e < bnd.end) aa_boundary_entry<Q, S, Odd>(f, bnd.list, e, g, p, diverged, sd);
+            return;
+        }
     }
     const int y = blockIdx.y * kBulkRows + threadIdx.y;
-    const int z = z0 + (int)(blockIdx.z - bnd.slabs);
+    int z = z0 + (int)blockIdx.z;
+    if constexpr (WithList) z -= (int)bnd.slabs;
     if (y >= g.ny) return;
     const size_t row = (size_t)z * g.ny + y;
     const int k = 2 * threadIdx.x;
@@ -411,7 +426,7 @@ __global__ void __launch_bounds__(32 * kBulkRows, 4) k_bulk_pairs_aa(typename S:
         pair &= ~2u;
     }
     const uint32_t c = (uint32_t)(row * g.nx + x);
-    previous_step_done();
+    if constexpr (WithList) previous_step_done();
     if constexpr (!S::kExact) {  // the row-end cells by the whole warp
         aa_row_end_cells<Q, S, Odd>(f, g, p, sd, plane, x, y, z, c, row);
         plane = 0;
@@ -515,7 +530,7 @@ __global__ void __launch_bounds__(32 * kBulkRows, 4) k_bulk_pairs_aa(typename S:
         const uint32_t off = (out || !Odd) ? 0u : (uint32_t)link_offset<Q>(i, g);
         const uint32_t sa = va ? c - off : c;
         const uint32_t sb = vb ? c + 1u - off : c + 1u;
-        const T* base = f + (size_t)rplane * g.ps;
+        const T* base = f + (size_t)rplane * g.n;
         const T ha = ld_plain<S>(base + sa), hb = ld_plain<S>(base + sb);
         if constexpr (S::kExact)
             v[i] = make_float2(S::dec(ha, L::w(i)), S::dec(hb, L::w(i)));
@@ -535,8 +550,8 @@ __global__ void __launch_bounds__(32 * kBulkRows, 4) k_bulk_pairs_aa(typename S:
         const int ty = y + L::ey(i), tz = z + L::ez(i);
         const bool inside = ty >= 0 && ty < g.ny && tz >= 0 && tz < g.nz;
         const bool push = Odd && inside;
-        T* dst = f + (push ? (size_t)i * g.ps + (size_t)((long long)c + link_offset<Q>(i, g))
-                           : (size_t)L::opp(i) * g.ps + c);
+        T* dst = f + (push ? (size_t)i * g.n + (size_t)((long long)c + link_offset<Q>(i, g))
+                           : (size_t)L::opp(i) * g.n + c);
         if (pair == 3u && (!push || L::ex(i) == 0)) {
             *reinterpret_cast<T2*>(dst) = h;
         } else {
@@ -588,8 +603,8 @@ __device__ __forceinline__ void aa_store_pair(typename S::T* f, const PlanePtrs&
         const int ty = y + L::ey(i), tz = z + L::ez(i);
         const bool inside = ty >= 0 && ty < g.ny && tz >= 0 && tz < g.nz;
         const bool push = Odd && inside;
-        T* dst = f + (push ? (size_t)i * g.ps + (size_t)((long long)c + link_offset<Q>(i, g))
-                           : (size_t)L::opp(i) * g.ps + c);
+        T* dst = f + (push ? (size_t)i * g.n + (size_t)((long long)c + link_offset<Q>(i, g))
+                           : (size_t)L::opp(i) * g.n + c);
         if (pair == 3u && (!push || L::ex(i) == 0)) {
             *reinterpret_cast<T2*>(dst) = h;
         } else {
@@ -682,7 +697,7 @@ __global__ void __launch_bounds__(32 * kBulkRows, 4) k_bulk_pairs_aa_learned(typ
             const uint32_t off = (out || !Odd) ? 0u : (uint32_t)link_offset<Q>(i, g);
             const uint32_t sa = va ? c - off : cs;
             const uint32_t sb = vb ? c + 1u - off : cs + 1u;
-            const T* base = f + (size_t)rplane * g.ps;
+            const T* base = f + (size_t)rplane * g.n;
             v[i] = make_float2(S::raw(ld_plain<S>(base + sa)), S::raw(ld_plain<S>(base + sb)));
         });
     }
@@ -805,15 +820,29 @@ static cudaError_t bulk_aa_t(void* f, const uint32_t* bits, const Geom& g, const
     for (int i = 0; i < Q; ++i) {
         const long long off = (long long)Lattice<Q>::ex(i) + (long long)Lattice<Q>::ey(i) * g.nx +
                               (long long)Lattice<Q>::ez(i) * g.nxy;
-        const long long pi = (long long)i * (long long)g.ps, po = (long long)Lattice<Q>::opp(i) * (long long)g.ps;
+        const long long pi = (long long)i * (long long)g.n, po = (long long)Lattice<Q>::opp(i) * (long long)g.n;
         pp.src[i] = base + (odd ? po - off : pi);
         pp.dst[i] = base + (odd ? pi + off : po);
     }
     dim3 block(32, kBulkRows, 1);
     dim3 grid((unsigned)((g.nx + 63) / 64), (unsigned)((g.ny + kBulkRows - 1) / kBulkRows), 1);
-    const auto kernel = odd ? k_bulk_pairs_aa<Q, S, true> : k_bulk_pairs_aa<Q, S, false>;
-    return launch_with_slabs(bnd, grid.x, grid.y, zc > 0 ? zc : 0, launched, [&](const BoundarySpan& bs, unsigned layers) {
-        grid.z = layers + bs.slabs;
+    BoundarySpan list = bnd;
+    unsigned layers = zc > 0 ? zc : 0;
+    if constexpr (S::kExact) {
+        if (layers > 0 && g.n >= aa_list_apart<Q>()) {
+            grid.z = layers;
+            const cudaError_t e =
+                launch_step_kernel(odd ? k_bulk_pairs_aa<Q, S, true, false> : k_bulk_pairs_aa<Q, S, false, false>, grid,
+                                   block, s, false, base, bits, g, p, pp, z0, dv, sd, BoundarySpan{});
+            if (e != cudaSuccess) return e;
+            ++*launched;
+            layers = 0;
+            list.chained = false;
+        }
+    }
+    const auto kernel = odd ? k_bulk_pairs_aa<Q, S, true, true> : k_bulk_pairs_aa<Q, S, false, true>;
+    return launch_with_slabs(list, grid.x, grid.y, layers, launched, [&](const BoundarySpan& bs, unsigned nz) {
+        grid.z = nz + bs.slabs;
         return launch_step_kernel(kernel, grid, block, s, bs.chained, base, bits, g, p, pp, z0, dv, sd, bs);
     });
 }
@@ -834,7 +863,7 @@ static cudaError_t bulk_aa_learned_t(void* f, const uint32_t* bits, const Geom& 
         for (int i = 0; i < Q; ++i) {
             const long long off = (long long)Lattice<Q>::ex(i) + (long long)Lattice<Q>::ey(i) * g.nx +
                                   (long long)Lattice<Q>::ez(i) * g.nxy;
-            const long long pi = (long long)i * (long long)g.ps, po = (long long)Lattice<Q>::opp(i) * (long long)g.ps;
+            const long long pi = (long long)i * (long long)g.n, po = (long long)Lattice<Q>::opp(i) * (long long)g.n;
             pp.src[i] = base + (odd ? po - off : pi);
             pp.dst[i] = base + (odd ? pi + off : po);
         }
