@@ -10,6 +10,7 @@
 // 16-byte-per-cell macro buffer the way the reference's GPU kernel does
 // (shaders/lbm_step.comp.glsl:360-363), which saves 16 B of HBM traffic per
 // cell update.
+#include <algorithm>
 #include <mutex>
 
 #include "aa.cuh"
@@ -109,6 +110,20 @@ __device__ __forceinline__ float4 fluid_moments(const typename S::T* __restrict_
     static_for<0, Q>([&](auto I) {
         constexpr int i = decltype(I)::value;
         p[i] = load_at<Q, S, i>(f, c, x, y, z, g, layout);
+    });
+    float rho, ux, uy, uz;
+    moments<Q>(p, rho, ux, uy, uz);
+    return make_float4(rho, ux, uy, uz);
+}
+
+// The same for a cell off every face in the layout an in-place even step
+// leaves: no neighbour is tested for being inside.
+template <int Q, class S>
+__device__ __forceinline__ float4 inner_moments(const typename S::T* __restrict__ f, const Geom& g, size_t c) {
+    float p[Q];
+    static_for<0, Q>([&](auto I) {
+        constexpr int i = decltype(I)::value;
+        p[i] = S::dec(S::ld(f + (size_t)i * g.ps + (size_t)((long long)c + aa_link<Q>(i, g))), Lattice<Q>::w(i));
     });
     float rho, ux, uy, uz;
     moments<Q>(p, rho, ux, uy, uz);
@@ -287,8 +302,14 @@ __device__ __forceinline__ void stat_block_reduce(StatAcc& acc, double* out) {
 constexpr int kGroup = 128;
 constexpr int kStatsWarps = kStatsThreads / 32;
 // Resident blocks per SM. The grids stop at one wave of them: each block ends
-// in a barrier and a reduction. (Four k_stats blocks spill: 444 us against 417.)
-constexpr int kStatsPerSm = 3, kAeroPerSm = 2;
+// in a barrier and a reduction. Plane-major k_stats holds four cells per lane
+// and takes three blocks (four spill: 444 us against 417; with three only D3Q15
+// in 16 bits does, 84 bytes, and 512x256x256 still take 347 us, 438 without
+// groups). The in-place ones hold one cell and take four: 512x256x256 after
+// an even step, D3Q19 FP16 780 us, D3Q15 663, with three 809 and 705.
+constexpr int kAeroPerSm = 2;
+constexpr int stats_per_sm(int layout) { return layout == kLayoutPlanes ? 3 : 4; }
+constexpr int kMostStatsBlocks = 148 * 4;
 
 __device__ __forceinline__ size_t group_cell(size_t base, int lane, int j, bool planes) {
     return base + (planes ? 4 * lane + j : lane + 32 * j);
@@ -409,7 +430,7 @@ __device__ __forceinline__ void load4(const typename S::T* p, float w, float2& l
 // 2-byte loads, the force in the lanes that hit a solid cell, before); what is
 // left is arithmetic: the IEEE divisions and roots of four cells per lane.
 template <int Q, class S, int Lay>
-__global__ void __launch_bounds__(kStatsThreads, kStatsPerSm) k_stats(const typename S::T* __restrict__ f,
+__global__ void __launch_bounds__(kStatsThreads, stats_per_sm(Lay)) k_stats(const typename S::T* __restrict__ f,
                                                          const uint8_t* __restrict__ solid,
                                                          const float* __restrict__ sdf, Geom g,
                                                          double* __restrict__ partials, bool words, bool vec) {
@@ -431,55 +452,67 @@ __global__ void __launch_bounds__(kStatsThreads, kStatsPerSm) k_stats(const type
             sol = solid_bits(group_word(solid, base, g.n, lane, planes, words));
             fluid = inside_bits(base, g.n, lane, planes) & ~sol;
         }
-        float4 m[4];
-        if (planes && vec && base + kGroup <= g.n) {  // moments<Q> of four cells
-            if (fluid) {
-                const float2 zero = bc2(0.0f);
-                float2 r[2] = {zero, zero}, a[2] = {zero, zero}, b[2] = {zero, zero}, c[2] = {zero, zero};
-                static_for<0, Q>([&](auto I) {
-                    constexpr int i = decltype(I)::value;
-                    constexpr int X = L::ex(i), Y = L::ey(i), Z = L::ez(i);
-                    float2 v[2];
-                    load4<S>(f + (size_t)i * g.ps + base + 4 * lane, L::w(i), v[0], v[1]);
-                    for (int j = 0; j < 2; ++j) {
-                        r[j] = add2(r[j], v[j]);
-                        if constexpr (X > 0) a[j] = add2(a[j], v[j]);
-                        if constexpr (X < 0) a[j] = sub2(a[j], v[j]);
-                        if constexpr (Y > 0) b[j] = add2(b[j], v[j]);
-                        if constexpr (Y < 0) b[j] = sub2(b[j], v[j]);
-                        if constexpr (Z > 0) c[j] = add2(c[j], v[j]);
-                        if constexpr (Z < 0) c[j] = sub2(c[j], v[j]);
-                    }
-                });
-                for (int j = 0; j < 2; ++j) {
-                    if (r[j].x > 1e-6f) a[j].x /= r[j].x, b[j].x /= r[j].x, c[j].x /= r[j].x;
-                    if (r[j].y > 1e-6f) a[j].y /= r[j].y, b[j].y /= r[j].y, c[j].y /= r[j].y;
-                    m[2 * j] = make_float4(r[j].x, a[j].x, b[j].x, c[j].x);
-                    m[2 * j + 1] = make_float4(r[j].y, a[j].y, b[j].y, c[j].y);
-                }
+        auto add = [&](const float4& m) {
+            if (!isfinite(m.x) || !isfinite(m.y) || !isfinite(m.z) || !isfinite(m.w)) {
+                acc.nan = 1;
+                return;
             }
-        } else {
+            const float sp = sqrtf(speed2(m.y, m.z, m.w));
+            acc.mn = fminf(acc.mn, m.x);
+            acc.mx = fmaxf(acc.mx, m.x);
+            acc.vmax = fmaxf(acc.vmax, sp);
+            acc.dsum += (double)m.x;
+            acc.ssum += (double)sp;
+            acc.count += 1.0;
+        };
+        if constexpr (!planes) {
+            // One cell at a time, since four in flight spill, and without the
+            // tests for the faces where none is near: 1024x512x512 after an even
+            // step, D3Q15 FP16 9.1 -> 4.6 ms, D3Q19 FP32 9.4 -> 5.2.
+#pragma unroll 1
             for (int j = 0; j < 4; ++j) {
                 if (!((fluid >> j) & 1u)) continue;
                 const size_t c = group_cell(base, lane, j, planes);
-                int x = 0, y = 0, z = 0;
-                if (!planes) cell_xyz(g, c, x, y, z);
-                m[j] = fluid_moments<Q, S>(f, g, c, x, y, z, Lay);
+                int x, y, z;
+                cell_xyz(g, c, x, y, z);
+                const bool inner = x > 0 && y > 0 && z > 0 && x < g.nx - 1 && y < g.ny - 1 && z < g.nz - 1;
+                add(Lay == kLayoutAAEven && inner ? inner_moments<Q, S>(f, g, c)
+                                                  : fluid_moments<Q, S>(f, g, c, x, y, z, Lay));
             }
-        }
-        for (int j = 0; j < 4; ++j) {
-            if (!((fluid >> j) & 1u)) continue;
-            if (!isfinite(m[j].x) || !isfinite(m[j].y) || !isfinite(m[j].z) || !isfinite(m[j].w)) {
-                acc.nan = 1;
-                continue;
+        } else {
+            float4 m[4];
+            if (vec && base + kGroup <= g.n) {  // moments<Q> of four cells
+                if (fluid) {
+                    const float2 zero = bc2(0.0f);
+                    float2 r[2] = {zero, zero}, a[2] = {zero, zero}, b[2] = {zero, zero}, c[2] = {zero, zero};
+                    static_for<0, Q>([&](auto I) {
+                        constexpr int i = decltype(I)::value;
+                        constexpr int X = L::ex(i), Y = L::ey(i), Z = L::ez(i);
+                        float2 v[2];
+                        load4<S>(f + (size_t)i * g.ps + base + 4 * lane, L::w(i), v[0], v[1]);
+                        for (int j = 0; j < 2; ++j) {
+                            r[j] = add2(r[j], v[j]);
+                            if constexpr (X > 0) a[j] = add2(a[j], v[j]);
+                            if constexpr (X < 0) a[j] = sub2(a[j], v[j]);
+                            if constexpr (Y > 0) b[j] = add2(b[j], v[j]);
+                            if constexpr (Y < 0) b[j] = sub2(b[j], v[j]);
+                            if constexpr (Z > 0) c[j] = add2(c[j], v[j]);
+                            if constexpr (Z < 0) c[j] = sub2(c[j], v[j]);
+                        }
+                    });
+                    for (int j = 0; j < 2; ++j) {
+                        if (r[j].x > 1e-6f) a[j].x /= r[j].x, b[j].x /= r[j].x, c[j].x /= r[j].x;
+                        if (r[j].y > 1e-6f) a[j].y /= r[j].y, b[j].y /= r[j].y, c[j].y /= r[j].y;
+                        m[2 * j] = make_float4(r[j].x, a[j].x, b[j].x, c[j].x);
+                        m[2 * j + 1] = make_float4(r[j].y, a[j].y, b[j].y, c[j].y);
+                    }
+                }
+            } else {
+                for (int j = 0; j < 4; ++j)
+                    if ((fluid >> j) & 1u) m[j] = fluid_moments<Q, S>(f, g, group_cell(base, lane, j, planes), 0, 0, 0, Lay);
             }
-            const float sp = sqrtf(speed2(m[j].y, m[j].z, m[j].w));
-            acc.mn = fminf(acc.mn, m[j].x);
-            acc.mx = fmaxf(acc.mx, m[j].x);
-            acc.vmax = fmaxf(acc.vmax, sp);
-            acc.dsum += (double)m[j].x;
-            acc.ssum += (double)sp;
-            acc.count += 1.0;
+            for (int j = 0; j < 4; ++j)
+                if ((fluid >> j) & 1u) add(m[j]);
         }
         group_solids<Q>(s_lists[warp], queued, base, lane, planes, sol, last, solid, g, [](int, int, int) {},
                         [&](size_t c) {
@@ -729,8 +762,7 @@ static bool words_of(const uint8_t* solid) { return reinterpret_cast<uintptr_t>(
 
 int stats_blocks(const Geom& g) {
     const size_t want = (g.n + kStatsThreads * 8 - 1) / (kStatsThreads * 8);
-    const size_t cap = 148 * 16;
-    return (int)(want < 1 ? 1 : (want > cap ? cap : want));
+    return (int)std::min<size_t>(std::max<size_t>(want, 1), kMostStatsBlocks);
 }
 
 // Launches KERNEL<Q, S, layout> for the run-time `layout` (PopLayout).
@@ -784,7 +816,7 @@ static cudaError_t stats_t(const void* f, const uint8_t* solid, const float* sdf
                            int blocks, double* result, int layout, cudaStream_t s) {
     // four populations at a time where every plane and cell group starts on
     // such a boundary
-    blocks = blocks < kStatsPerSm * 148 ? blocks : kStatsPerSm * 148;
+    blocks = std::min(blocks, stats_per_sm(layout) * 148);
     const bool vec = g.ps % 4 == 0 && reinterpret_cast<uintptr_t>(f) % (4 * S::kBytes) == 0;
     FC_LAYOUT_LAUNCH(k_stats, blocks, kStatsThreads, (const typename S::T*)f, solid, sdf, g, partials, words_of(solid),
                      vec);
@@ -837,7 +869,7 @@ template <int Q, class S>
 static cudaError_t aero_t(const void* f, const uint8_t* solid, const float* sdf, const Geom& g, float cs, float ox,
                           float oy, float oz, double* partials, int blocks, double* result, int layout,
                           cudaStream_t s) {
-    blocks = blocks < kAeroPerSm * 148 ? blocks : kAeroPerSm * 148;
+    blocks = std::min(blocks, kAeroPerSm * 148);
     FC_LAYOUT_LAUNCH(k_aero, blocks, kStatsThreads, (const typename S::T*)f, solid, sdf, g, cs, ox, oy, oz, partials,
                      words_of(solid));
     cudaError_t e = cudaGetLastError();
@@ -857,14 +889,10 @@ cudaError_t launch_aero(int q, int storage, const void* f, const uint8_t* solid,
 // ---- statistics without allocation (fc_lbm_stats_noalloc) ----
 // The same k_stats / k_stats_final kernels as fc_lbm_readback_stats, with the
 // per-block partials in a fixed file-scope device array instead of memory the
-// solver allocated. The array holds 4096 blocks' partials (4096 * 12 doubles
-// = 384 KiB). The block count follows the allocating path's rule, one block
-// per 2048 cells, capped here by the array instead of at 148 * 16: the
-// reduction is grid-stride, so every cell is covered whatever the count, and
-// below the allocating path's cap (4.8M cells) both paths form the same
-// partial sums. Lattices are limited to 2^29 cells. Each launch writes every
-// slot of the partials it uses before the final kernel reads them, so nothing
-// has to be cleared between calls.
+// solver allocated: as many blocks' as a launch of either path has at most
+// (592 * 12 doubles = 56 KiB). Both paths take the same number of blocks. Lattices are limited
+// to 2^29 cells. Each launch writes every slot of the partials it uses before
+// the final kernel reads them, so nothing has to be cleared between calls.
 //
 // The device address of the array is looked up once per device and cached for
 // the life of the process. A cudaDeviceReset destroys the module that holds
@@ -872,11 +900,9 @@ cudaError_t launch_aero(int q, int storage, const void* f, const uint8_t* solid,
 // documents this.
 namespace {
 
-constexpr int kNoAllocMaxBlocks = 4096;
-constexpr size_t kNoAllocCellsPerBlock = size_t(1) << 11;  // kStatsThreads * 8, as stats_blocks()
 static_assert(fc::kStatsSlots == FC_LBM_STATS_SLOTS, "slot count must match the header");
 
-static __device__ __align__(256) double g_noalloc_partials[kNoAllocMaxBlocks * fc::kStatsSlots];
+static __device__ __align__(256) double g_noalloc_partials[fc::kMostStatsBlocks * fc::kStatsSlots];
 
 constexpr int kNoAllocMaxDevices = 64;
 std::mutex g_noalloc_mutex;
@@ -916,10 +942,8 @@ extern "C" FC_LBM_API int fc_lbm_stats_noalloc(const void* populations, const ui
     g.nxy = (long long)nx * ny;
     g.n = n;
     g.ps = n;  // the caller's planes: no padding
-    const size_t want = (n + kNoAllocCellsPerBlock - 1) / kNoAllocCellsPerBlock;
-    const int blocks = (int)(want < 1 ? 1 : (want > (size_t)kNoAllocMaxBlocks ? (size_t)kNoAllocMaxBlocks : want));
     const int q = model == FC_LATTICE_D3Q19 ? 19 : 15;
-    const cudaError_t e = fc::launch_stats(q, storage, populations, solid, signed_distance, g, scratch, blocks,
-                                           out_slots, fc::kLayoutPlanes, static_cast<cudaStream_t>(stream));
+    const cudaError_t e = fc::launch_stats(q, storage, populations, solid, signed_distance, g, scratch,
+                                           fc::stats_blocks(g), out_slots, fc::kLayoutPlanes, static_cast<cudaStream_t>(stream));
     return e == cudaSuccess ? FC_LBM_OK : FC_LBM_ERR_CUDA;
 }

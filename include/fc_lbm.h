@@ -469,7 +469,7 @@ FC_LBM_API int fc_lbm_batch_tune(fc_lbm_batch* b, int32_t steps, int32_t* rows, 
  * speed, max stress, NaN flag), asynchronously on `stream` (a cudaStream_t;
  * NULL = the default stream).
  *
- * The reduction's per-block partial sums live in one fixed 384 KiB array
+ * The reduction's per-block partial sums live in one fixed 56 KiB array
  * inside the library, which every GPU that loads the library holds until the
  * process exits. It covers lattices up to FC_LBM_NOALLOC_MAX_CELLS cells;
  * larger ones are refused with FC_LBM_ERR_TOO_LARGE before any work is
