@@ -410,7 +410,22 @@ def run_reference_arm(args, cfg, rank, world):
     return 0
 
 
+def timed_steps(s, steps) -> float:
+    """Device ms of `steps` steps as a program takes them (LbmSolver.Step)."""
+    import torch
+    stream = torch.cuda.ExternalStream(s.Stream())
+    start, stop = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+    start.record(stream)
+    s.Step(None, steps)
+    stop.record(stream)
+    stop.synchronize()
+    return start.elapsed_time(stop)
+
+
 def time_variant(args, cfg, solid, sdf, variant, dev_index, dist_on, sample_clocks):
+    """`args.steps` timed steps, then as many with events around a launch each
+    for the bulk cells and the boundary list (StepTimed takes a step apart, so
+    its total is not a step's time)."""
     s = make_solver(cfg, solid, sdf, variant, dev_index)
     info = s.BoundaryInfo()
     s.Step(None, spinup_of(args, variant) + args.warmup)
@@ -418,12 +433,13 @@ def time_variant(args, cfg, solid, sdf, variant, dev_index, dist_on, sample_cloc
     barrier_sync(dist_on)
     sampler = ClockSampler(dev_index) if sample_clocks else None
     l0 = s.LaunchCount()
-    t = s.StepTimed(args.steps)  # events around every launch, waits at the end
+    rank_ms = timed_steps(s, args.steps)
     launches = s.LaunchCount() - l0
-    coverage = s.ClosureCoverage() if variant.endswith("_learned") else None
     clocks = sampler.stop() if sampler else None
+    coverage = s.ClosureCoverage() if variant.endswith("_learned") else None
+    t = s.StepTimed(args.steps)
     barrier_sync(dist_on)
-    total_ms = allreduce_max(t["total_ms"], dist_on)
+    total_ms = allreduce_max(rank_ms, dist_on)
     stats = s.ReadbackStats()
     s.close()
     cells = cfg["nx"] * cfg["ny"] * cfg["nz"]
@@ -433,7 +449,7 @@ def time_variant(args, cfg, solid, sdf, variant, dev_index, dist_on, sample_cloc
     bulk_bytes = info["bulk_cells"] * per_cell
     return {
         "variant": variant, "total_ms": total_ms, "ms_per_step": total_ms / args.steps,
-        "glups_rank": cells * args.steps / (t["total_ms"] / 1e3) / 1e9,
+        "glups_rank": cells * args.steps / (rank_ms / 1e3) / 1e9,
         "bulk_ms_per_launch": t["bulk_ms"] / args.steps, "boundary_ms_per_launch": t["boundary_ms"] / args.steps,
         "bulk_cells": info["bulk_cells"], "boundary_cells": info["boundary_cells"],
         "bouzidi_links": info["bouzidi_links"], "bulk_bytes_per_launch": bulk_bytes,
