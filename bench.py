@@ -357,6 +357,11 @@ def cpu_subbox(cfg, solid, sdf, cores):
     return s, d, z0
 
 
+# what the CPU baseline times
+CPU_KINDS = {"reference": "LbmReference::Step",
+             "port": "this repository's C restatement of LbmReference::Step (no reference build here)"}
+
+
 def run_cpu_reference(cfg, solid_np, sdf_np, steps, warmup, seconds=None):
     """Times FlowCraft's own LbmReference (oracle/_ref, -O3) — or the restated
     oracle if the reference build is absent — on the given sub-box."""
@@ -387,6 +392,11 @@ def run_cpu_reference(cfg, solid_np, sdf_np, steps, warmup, seconds=None):
 def run_reference_arm(args, cfg, rank, world):
     import numpy as np
     if rank != 0:
+        return 0
+    from oracle import oracle as orc
+    if not orc.available("ref_fast"):
+        print(json.dumps({"impl": "reference", "unavailable": "no build of the reference's LbmReference "
+                          "(oracle/_ref): its source tree is not here"}), flush=True)
         return 0
     cores = os.cpu_count() or 1
     # the same procedural geometry, built on the host for the sub-box only
@@ -735,7 +745,7 @@ def run_ours(args, cfg, rank, world, local_rank):
         s_np, d_np, z0 = cpu_subbox(cfg, solid, sdf, cores)
         r = run_cpu_reference(cfg, s_np, d_np, 10 ** 6, 1, seconds=args.cpu_seconds)
         cpu = {"value": r["glups"], "unit": "GLUPS", "cores": cores, "kind": r["kind"],
-               "sample": f"LbmReference::Step, {cfg['nx']}x{cfg['ny']}x{s_np.shape[0]} sub-box (z0={z0}) of the "
+               "sample": f"{CPU_KINDS[r['kind']]}, {cfg['nx']}x{cfg['ny']}x{s_np.shape[0]} sub-box (z0={z0}) of the "
                          f"lattice, {r['steps']} steps in {r['seconds']:.1f}s after 1 warm-up"}
     if rank != 0:
         return 0
