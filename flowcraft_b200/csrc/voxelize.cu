@@ -44,6 +44,7 @@
 // Every loop over the union-find forest is bounded: labels strictly decrease
 // along a parent chain, and the loops also stop after a fixed iteration count,
 // setting an error bit the host turns into FC_LBM_ERR_CUDA.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -918,20 +919,63 @@ struct Scratch {
     }
 };
 
+// A driver function, or null.
+template <class Fn>
+Fn driver_function(const char* name) {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q{};
+    if (cudaGetDriverEntryPoint(name, &p, cudaEnableDefault, &q) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return q == cudaDriverEntryPointSuccess ? reinterpret_cast<Fn>(p) : nullptr;
+}
+
+// The id of the calling thread's current context, never given twice in a
+// process; 0 if there is none.
+unsigned long long context_id() {
+    using Current = CUresult (*)(CUcontext*);
+    using Id = CUresult (*)(CUcontext, unsigned long long*);
+    static const auto current = driver_function<Current>("cuCtxGetCurrent");
+    static const auto id_of = driver_function<Id>("cuCtxGetId");
+    CUcontext c = nullptr;
+    unsigned long long id = 0;
+    return current && id_of && current(&c) == CUDA_SUCCESS && c && id_of(c, &id) == CUDA_SUCCESS ? id : 0;
+}
+
 // A few pinned bytes per host thread for the sizes and status a call reads
 // back. A copy to pageable memory waits for the stream inside the driver, and
 // the memory pool gives its memory back at such waits: the next call then maps
-// it anew, which costs more than the call's kernels.
+// it anew, which costs more than the call's kernels. The bytes die with the
+// context they were allocated in (cudaDeviceReset): where another one is
+// current, the call takes pageable memory.
 struct HostWords {
     void* p = nullptr;
+    int device = -1;
+    unsigned long long context = 0;
     HostWords() {
-        if (cudaHostAlloc(&p, 64, cudaHostAllocPortable) != cudaSuccess) {
+        context = context_id();
+        if (!context || cudaGetDevice(&device) != cudaSuccess || cudaHostAlloc(&p, 64, cudaHostAllocDefault) != cudaSuccess) {
             cudaGetLastError();  // the caller falls back to pageable memory
             p = nullptr;
         }
     }
+    bool usable() const { return p && context_id() == context; }
     ~HostWords() {
-        if (p) cudaFreeHost(p);
+        if (!p) return;
+        if (!usable()) {  // the thread has moved to another device since, or the context is gone
+            using Get = CUresult (*)(CUdevice*, int);
+            using State = CUresult (*)(CUdevice, unsigned*, int*);
+            const auto get = driver_function<Get>("cuDeviceGet");
+            const auto state = driver_function<State>("cuDevicePrimaryCtxGetState");
+            CUdevice d = 0;
+            unsigned flags = 0;
+            int active = 0;
+            if (!get || !state || get(&d, device) != CUDA_SUCCESS || state(d, &flags, &active) != CUDA_SUCCESS ||
+                !active || cudaSetDevice(device) != cudaSuccess || !usable())
+                return;
+        }
+        cudaFreeHost(p);
     }
 };
 
@@ -944,7 +988,7 @@ static_assert(sizeof(Answer) <= 64, "one HostWords block");
 
 Answer* host_answer(Answer* fallback) {
     static thread_local HostWords w;
-    return w.p ? static_cast<Answer*>(w.p) : fallback;
+    return w.usable() ? static_cast<Answer*>(w.p) : fallback;
 }
 
 int code_of(cudaError_t e) {
