@@ -18,7 +18,9 @@
 
 namespace fc {
 
-constexpr long long kSpinNs = 500'000;  // polled without sleeping up to here
+// Polled without sleeping up to here: the first sleep adds some 50 us, which a
+// wait of half a millisecond (the voxelizer's second) would feel.
+constexpr long long kSpinNs = 1'000'000;
 
 // Polls done() (a cudaError_t: cudaErrorNotReady to go on) until it returns
 // something else or `timeout_ms` (negative: none) have passed; then

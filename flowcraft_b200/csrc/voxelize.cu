@@ -256,11 +256,11 @@ struct GridDev {
     float ox, oy, oz;
 };
 
-// Status words of a call: error bits, the tiles that hold a triangle, the
-// triangles in `big`, and the tiles with long lists.
+// Status words of a call: error bits, the tiles that hold a triangle, and the
+// tiles with long lists.
 struct Status {
     int err;
-    unsigned occupied, big, longest, long_tiles;
+    unsigned occupied, longest, long_tiles;
 };
 
 // Marks tile (x, y, z) in `slot`; 1 where it was not marked before.
@@ -269,25 +269,23 @@ __device__ __forceinline__ unsigned mark_tile(uint32_t* __restrict__ slot, const
     return __ldcg(m) == 0u && atomicExch(m, 1u) == 0u ? 1u : 0u;
 }
 
-// Also marks the tiles a triangle's box touches in `slot` (zeroed) and counts
-// the marked ones. A tile costs a thread a trip to memory, so the boxes of
-// more than kOwnTiles tiles go into the list `big` for k_tri_mark: two facets
-// across a 1024x512x512 grid took 316 ms with all of a triangle's tiles on its own thread.
+// The record and pair count of triangle t, and where its box holds at most
+// kOwnTiles tiles their marks in `slot`; true where it holds more.
 constexpr unsigned kOwnTiles = 32;
-__global__ void k_tri_prep(const float* __restrict__ pos, unsigned nv, const uint32_t* __restrict__ idx,
-                           unsigned ntri, GridDev g, Tri* __restrict__ tris, unsigned long long* __restrict__ counts,
-                           uint32_t* __restrict__ slot, uint32_t* __restrict__ big, Status* __restrict__ st) {
-    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t > ntri) return;
+__device__ __forceinline__ bool prep_triangle(const float* __restrict__ pos, unsigned nv,
+                                              const uint32_t* __restrict__ idx, unsigned ntri, const GridDev& g,
+                                              Tri* tris, unsigned long long* __restrict__ counts, uint32_t* slot,
+                                              Status* st, unsigned t) {
+    if (t > ntri) return false;
     if (t == ntri) {  // the scan's trailing slot, so offsets[ntri] is the pair total
         counts[t] = 0;
-        return;
+        return false;
     }
     const uint32_t i0 = idx[3 * (size_t)t], i1 = idx[3 * (size_t)t + 1], i2 = idx[3 * (size_t)t + 2];
     if (i0 >= nv || i1 >= nv || i2 >= nv) {
         atomicOr(&st->err, kErrBadIndex);
         counts[t] = 0;
-        return;
+        return false;
     }
     const V3 a{pos[3 * (size_t)i0], pos[3 * (size_t)i0 + 1], pos[3 * (size_t)i0 + 2]};
     const V3 b{pos[3 * (size_t)i1], pos[3 * (size_t)i1 + 1], pos[3 * (size_t)i1 + 2]};
@@ -325,9 +323,7 @@ __global__ void k_tri_prep(const float* __restrict__ pos, unsigned nv, const uin
         if (lo0 <= hi0 && lo1 <= hi1 && lo2 <= hi2) {
             cnt = (unsigned long long)(hi0 / kTile - lo0 / kTile + 1) * (hi1 / kTile - lo1 / kTile + 1) *
                   (hi2 / kTile - lo2 / kTile + 1);
-            if (cnt > kOwnTiles) {
-                big[atomicAdd(&st->big, 1u)] = t;
-            } else {
+            if (cnt <= kOwnTiles) {
                 unsigned fresh = 0;
                 for (int z = lo2 / kTile; z <= hi2 / kTile; ++z)
                     for (int y = lo1 / kTile; y <= hi1 / kTile; ++y)
@@ -338,33 +334,46 @@ __global__ void k_tri_prep(const float* __restrict__ pos, unsigned nv, const uin
     }
     tris[t] = r;
     counts[t] = cnt;
+    return cnt > kOwnTiles;
 }
 
-// Marks the tiles of the triangles in `big`, kMarkParts warps each (the ones
-// past a box's tiles leave at once), a tile per lane. Not where the call is
-// about to be refused for its number of pairs, which these boxes make up.
-constexpr unsigned kMarkParts = 128;
-constexpr unsigned kMarkBlocks = 148 * 8;
-__global__ void __launch_bounds__(256) k_tri_mark(const Tri* __restrict__ tris, const uint32_t* __restrict__ big,
-                                                  const unsigned long long* __restrict__ pairs, GridDev g,
-                                                  uint32_t* __restrict__ slot, Status* __restrict__ st) {
-    const unsigned lane = threadIdx.x & 31u;
-    const size_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, warps = (gridDim.x * blockDim.x) >> 5;
-    const size_t items = (size_t)st->big * kMarkParts;
-    if (items == 0 || *pairs > (unsigned long long)INT32_MAX) return;
-    for (size_t i = warp; i < items; i += warps) {
-        const Tri& r = tris[big[i / kMarkParts]];
+// Also marks every tile a triangle's box touches in `slot` (zeroed) and counts
+// the marked tiles. A tile is a trip to memory, so a box of many is marked by
+// the whole block, four tiles per thread in flight: two facets across a
+// 1024x512x512 grid took 316 ms with all tiles of a box on its thread.
+constexpr int kPrepThreads = 256;
+__global__ void __launch_bounds__(kPrepThreads) k_tri_prep(const float* __restrict__ pos, unsigned nv,
+                                                           const uint32_t* __restrict__ idx, unsigned ntri, GridDev g,
+                                                           Tri* tris, unsigned long long* __restrict__ counts,
+                                                           uint32_t* slot, Status* st) {
+    __shared__ unsigned s_big[kPrepThreads], s_count;
+    if (threadIdx.x == 0) s_count = 0;
+    __syncthreads();
+    const unsigned t = blockIdx.x * kPrepThreads + threadIdx.x;
+    if (prep_triangle(pos, nv, idx, ntri, g, tris, counts, slot, st, t)) s_big[atomicAdd(&s_count, 1u)] = t;
+    __syncthreads();
+    unsigned fresh = 0;
+    for (unsigned b = 0; b < s_count; ++b) {
+        const Tri& r = tris[s_big[b]];
         const int x0 = r.lo[0] / kTile, y0 = r.lo[1] / kTile, z0 = r.lo[2] / kTile;
         const unsigned wx = r.hi[0] / kTile - x0 + 1, wy = r.hi[1] / kTile - y0 + 1, wz = r.hi[2] / kTile - z0 + 1;
-        const size_t count = (size_t)wx * wy * wz;
-        unsigned fresh = 0;
-        for (size_t k = (i % kMarkParts) * 32 + lane; k < count; k += kMarkParts * 32) {
-            const size_t row = k / wx;
-            fresh += mark_tile(slot, g, x0 + (int)(k - row * wx), y0 + (int)(row % wy), z0 + (int)(row / wy));
+        const uint64_t count = (uint64_t)wx * wy * wz;
+        for (uint64_t k0 = threadIdx.x; k0 < count; k0 += 4 * kPrepThreads) {
+            uint32_t* m[4];
+            uint32_t old[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const uint64_t k = k0 + u * kPrepThreads < count ? k0 + u * kPrepThreads : k0;
+                const uint64_t row = k / wx;
+                m[u] = slot + (((size_t)z0 + row / wy) * g.ty + y0 + row % wy) * g.tx + x0 + (k - row * wx);
+                old[u] = __ldcg(m[u]);
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (old[u] == 0u && atomicExch(m[u], 1u) == 0u) ++fresh;
         }
-        fresh = __reduce_add_sync(0xffffffffu, fresh);
-        if (lane == 0 && fresh) atomicAdd(&st->occupied, fresh);
     }
+    if (fresh) atomicAdd(&st->occupied, fresh);
 }
 
 __global__ void k_tri_emit(const Tri* __restrict__ tris, const unsigned long long* __restrict__ offsets,
@@ -502,7 +511,7 @@ __device__ __forceinline__ void raster_tile(unsigned tile_at, uint32_t tile, uns
 constexpr int kRasterWarps = kRasterThreads / 32;
 constexpr int kRasterChunk = 64;  // distances kept at a time
 constexpr int kTileBoxes = kTileCells / 32;
-__global__ void __launch_bounds__(kRasterThreads) k_vox_raster(
+__global__ void __launch_bounds__(kRasterThreads, 4) k_vox_raster(
     const Tri* __restrict__ tris, const uint32_t* __restrict__ tile_tris, const uint32_t* __restrict__ run_tile,
     const uint32_t* __restrict__ run_len, const unsigned long long* __restrict__ run_off, unsigned runs,
     const uint32_t* __restrict__ long_tiles, unsigned most, const Status* __restrict__ st, GridDev g,
@@ -1071,14 +1080,14 @@ int voxelize_on_device(const float* d_pos, size_t nv, const uint32_t* d_idx, siz
 
     // the first half: triangle records, tile marks, and the sizes of the rest
     Status* d_st = nullptr;
-    uint32_t *slot = nullptr, *big = nullptr;
+    uint32_t* slot = nullptr;
     Tri* tris = nullptr;
     unsigned long long *counts = nullptr, *offsets = nullptr;
     void* tmp = nullptr;
     size_t tmp_bytes = 0;
     if (ntri > 0)
         VX_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, counts, offsets, (int64_t)ntri + 1, s));
-    VX_TRY(sc.get_all({{&d_st, 1}, {&slot, ntiles}, {&big, ntri}, {&tris, ntri}, {&counts, (size_t)ntri + 1},
+    VX_TRY(sc.get_all({{&d_st, 1}, {&slot, ntiles}, {&tris, ntri}, {&counts, (size_t)ntri + 1},
                        {&offsets, (size_t)ntri + 1}, {&tmp, tmp_bytes}}));
     VX_TRY(cudaMemsetAsync(d_st, 0, sizeof(Status), s));
     VX_TRY(cudaMemsetAsync(slot, 0, sizeof(uint32_t) * ntiles, s));
@@ -1087,12 +1096,10 @@ int voxelize_on_device(const float* d_pos, size_t nv, const uint32_t* d_idx, siz
     Answer own;
     Answer* ans = host_answer(&own);
     if (ntri > 0) {
-        k_tri_prep<<<(ntri + 1 + 255) / 256, 256, 0, s>>>(d_pos, (unsigned)nv, d_idx, ntri, g, tris, counts, slot, big,
-                                                          d_st);
+        k_tri_prep<<<(ntri + kPrepThreads) / kPrepThreads, kPrepThreads, 0, s>>>(d_pos, (unsigned)nv, d_idx, ntri, g,
+                                                                               tris, counts, slot, d_st);
         VX_TRY(cudaGetLastError());
         VX_TRY(cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, counts, offsets, (int64_t)ntri + 1, s));
-        k_tri_mark<<<kMarkBlocks, 256, 0, s>>>(tris, big, offsets + ntri, g, slot, d_st);
-        VX_TRY(cudaGetLastError());
         VX_TRY(cudaMemcpyAsync(&ans->pairs, offsets + ntri, sizeof(pairs), cudaMemcpyDeviceToHost, s));
         VX_TRY(cudaMemcpyAsync(&ans->st, d_st, sizeof(st), cudaMemcpyDeviceToHost, s));
         VX_RC(wait_on(s));
