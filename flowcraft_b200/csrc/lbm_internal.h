@@ -79,7 +79,8 @@ struct BoundaryList {
 // Against a kernel of their own behind the bulk kernel (10-25 us per step on a
 // B200): 48x24x24 FP32, 20 steps and a field, 562 -> 381 us; 256x128x128 FP32
 // with smoke, 20 frames of 2 steps, 7.31 -> 6.63 ms; 384x192x192 with the
-// learned closure, 50 steps, 24.85 -> 24.26 ms; no change at 268M cells.
+// learned closure, 50 steps, 24.85 -> 24.26 ms; no change at 268M cells. (In
+// place, large FP32 lattices keep the two apart: aa_list_apart.)
 struct BoundarySpan {
     BoundaryList list;
     uint32_t begin, end;

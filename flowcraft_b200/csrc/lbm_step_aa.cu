@@ -14,16 +14,16 @@
 //                     accesses otherwise). Row-end warps take the same
 //                     loads plus the inlet / outlet rules; face warps take
 //                     the general path with the edge rules.
-//   k_boundary_aa     the boundary list. The Bouzidi far-side partner
-//                     f*_i(c), which the pulling cell c + e_i overwrites in
-//                     place, comes from the side buffer the entry itself
-//                     filled last step.
+//   aa_boundary_entry one entry of the boundary list, in the first blocks of
+//                     the same kernel (large FP32 lattices: in a launch of
+//                     its own). The Bouzidi far-side partner f*_i(c), which
+//                     the pulling cell c + e_i overwrites in place, comes
+//                     from the side buffer the entry itself filled last step.
 //   k_aa_prime_*      fill the side buffers from a state set by a seed or
 //                     a population load.
-//   *_learned         the bulk and boundary kernels with the learned
-//                     closure (16-bit formats), the same slots around the
-//                     collision and warp-wide MLP of the ping-pong learned
-//                     kernels.
+//   *_learned         the same with the learned closure (16-bit formats): the
+//                     slots around the collision and warp-wide MLP of the
+//                     ping-pong learned kernel.
 //
 // Outlet moments: the outlet reads the moments of its upstream neighbour's
 // post-collision populations (LbmReference.cpp:275-327), which in place sit

@@ -1215,7 +1215,7 @@ FC_LBM_API int fc_lbm_voxelize(const float* positions, size_t vertex_count, cons
     if (index_count >= 3 && (!positions || !indices || vertex_count == 0)) return FC_LBM_ERR_INVALID_ARG;
     if (vertex_count >= 0xffffffffu || index_count / 3 >= 0xffffffffu) return FC_LBM_ERR_TOO_LARGE;
     const size_t n = (size_t)dims[0] * dims[1] * dims[2];
-    if (n >= 0xffffffffull) return FC_LBM_ERR_TOO_LARGE;  // labels are 32-bit cell indices
+    if (n >= 0xffffffffull) return FC_LBM_ERR_TOO_LARGE;  // tiles and cells count below 2^32
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     Scratch sc(s);
     const float* d_pos = positions;

@@ -594,8 +594,10 @@ class LbmSolver:
         return {"boundary_cells": a.value, "bouzidi_links": b.value, "bulk_cells": c.value}
 
     def StepTimed(self, n: int) -> dict:
-        """n substeps on the solver's stream with CUDA events around every
-        launch: device ms of the sequence and of the bulk / boundary kernels."""
+        """n substeps on the solver's stream, each taken apart into a launch of
+        the bulk cells and one of the boundary list with CUDA events around
+        them: device ms of the sequence and of the two (Step's own time is
+        less)."""
         t, b, d = ctypes.c_float(), ctypes.c_float(), ctypes.c_float()
         self._check(self._lib.fc_lbm_step_timed(self._h, int(n), ctypes.byref(t), ctypes.byref(b), ctypes.byref(d)),
                     "StepTimed")

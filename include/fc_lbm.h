@@ -225,10 +225,12 @@ FC_LBM_API int fc_lbm_get_stream(const fc_lbm* h, void** stream);
 /* Number of cells handled by the boundary-list kernel and of interpolated
  * (Bouzidi) links; diagnostics for tests and the bench. */
 FC_LBM_API int fc_lbm_boundary_info(const fc_lbm* h, uint64_t* boundary_cells, uint64_t* bouzidi_links, uint64_t* bulk_cells);
-/* Runs n full substeps on the solver's own stream with CUDA events around
- * every kernel launch, waits, and reports the device time of the whole
- * sequence and the summed durations of the bulk and boundary-list kernels
- * (ms). Measurement aid for benchmarks; results equal fc_lbm_step's. */
+/* Runs n full substeps on the solver's own stream, each taken apart into a
+ * launch of the bulk cells and one of the boundary list with CUDA events
+ * around them, waits, and reports the device time of the whole sequence and
+ * the summed durations of the two (ms). Measurement aid for benchmarks; results
+ * equal fc_lbm_step's, whose own time is less: it runs both in one launch and
+ * chains the launches of a call. */
 FC_LBM_API int fc_lbm_step_timed(fc_lbm* h, int32_t n, float* total_ms, float* bulk_ms, float* boundary_ms);
 /* Kernel launches this handle has enqueued since init (bench accounting). */
 FC_LBM_API int fc_lbm_launch_count(const fc_lbm* h, uint64_t* launches);
