@@ -64,7 +64,6 @@ namespace {
 constexpr int kTile = 8;                    // raster tile edge (cells)
 constexpr int kTileCells = kTile * kTile * kTile;
 constexpr int kTileRows = kTile * kTile;    // 8-cell x rows of a tile
-constexpr int kTileNodes = kTileRows * kTile / 2;  // runs an occupied tile can hold
 constexpr int kTriWords = 20;               // a[3] b[3] c[3] n[3] lo[3] hi[3] pad[2]
 constexpr int kBoundsBlocks = 148;
 constexpr int kBoundsThreads = 256;
@@ -646,12 +645,15 @@ __global__ void __launch_bounds__(kRasterThreads, 4) k_vox_raster(
 // ---- 4. flood fill (connected components of fluid nodes) ----
 
 // Node ids: a tile without triangles is its tile index; the run of fluid
-// cells that starts at bit b of row r of occupied tile k is ntiles +
-// kTileNodes k + 4 r + b / 2 (two runs of a row are at least two bits apart).
-// Id is 32 bits wherever the ids fit.
+// cells that starts at bit b of row (y, z) of occupied tile k is ntiles +
+// nodes k + (ry z + y) rx + b / 2 (two runs of a row are at least two bits
+// apart), with rx = 4 and ry = 8 and fewer in grids thinner than a tile, so that
+// there are no more nodes than a tile has cells. Id is 32 bits wherever the ids
+// fit.
 template <class Id>
 struct Flood {
     int tx, ty, tz;
+    int rx, ry, nodes;
     Id ntiles;
     const uint32_t* slot;
     const uint8_t* mask;  // fluid bits of the occupied tiles' rows: a byte per four cells
@@ -660,7 +662,7 @@ struct Flood {
     __device__ __forceinline__ Id run(uint32_t slot1, int row, unsigned m, int bit) const {
         const unsigned starts = m & ~(m << 1);
         const int b = 31 - __clz(starts & ((2u << bit) - 1u));
-        return ntiles + (Id)(slot1 - 1u) * kTileNodes + (Id)(row * (kTile / 2) + (b >> 1));
+        return ntiles + (Id)(slot1 - 1u) * (Id)nodes + (Id)((row / kTile * ry + row % kTile) * rx + (b >> 1));
     }
     __device__ __forceinline__ unsigned row_mask(uint32_t slot1, int row) const {
         const unsigned v = reinterpret_cast<const uint16_t*>(mask)[(size_t)(slot1 - 1u) * kTileRows + row];
@@ -715,7 +717,7 @@ __global__ void k_ff_label(Flood<Id> f, unsigned occupied) {
             f.L[i] = empty ? start : i;
         }
     }
-    for (size_t k = t; k < (size_t)occupied * kTileNodes; k += step) f.L[f.ntiles + k] = (Id)(f.ntiles + k);
+    for (size_t k = t; k < (size_t)occupied * f.nodes; k += step) f.L[f.ntiles + k] = (Id)(f.ntiles + k);
 }
 
 // Joins empty tiles with the row below and the layer below, once per stretch
@@ -1043,12 +1045,17 @@ int grid_on_device(const float* d_pos, size_t nv, const fc_voxel_params* p, cuda
     return FC_LBM_OK;
 }
 
+// Runs that a row of a tile, and a tile, of the grid can hold.
+int row_nodes(const GridDev& g) { return (std::min(g.nx, kTile) + 1) / 2; }
+int tile_nodes(const GridDev& g) { return row_nodes(g) * std::min(g.ny, kTile) * std::min(g.nz, kTile); }
+
 // The flood fill's kernels: labels, joins, reached flags.
 template <class Id>
 int flood(const GridDev& g, uint64_t ntiles, unsigned occupied, const uint32_t* slot, const uint8_t* mask,
           const uint32_t* run_tile, Id* L, uint8_t* tile_reached, uint8_t* row_reached, Status* st, cudaStream_t s) {
-    const Flood<Id> f{g.tx, g.ty, g.tz, (Id)ntiles, slot, mask, L, &st->err};
-    const uint64_t rows = std::max<uint64_t>((uint64_t)g.ty * g.tz, (uint64_t)occupied * kTileNodes);
+    const int rx = row_nodes(g), ry = std::min(g.ny, kTile), nodes = tile_nodes(g);
+    const Flood<Id> f{g.tx, g.ty, g.tz, rx, ry, nodes, (Id)ntiles, slot, mask, L, &st->err};
+    const uint64_t rows = std::max<uint64_t>((uint64_t)g.ty * g.tz, (uint64_t)occupied * nodes);
     k_ff_label<Id><<<(unsigned)std::min<uint64_t>((rows + 127) / 128, 148 * 32), 128, 0, s>>>(f, occupied);
     VX_TRY(cudaGetLastError());
     const uint64_t tile_blocks = (ntiles + 127) / 128;
@@ -1110,7 +1117,7 @@ int voxelize_on_device(const float* d_pos, size_t nv, const uint32_t* d_idx, siz
     }
     // the second half: the tiles' triangle lists and the flood fill's nodes
     const unsigned runs = st.occupied;  // the runs of equal tile ids after the sort
-    const uint64_t nodes = ntiles + (uint64_t)runs * kTileNodes;
+    const uint64_t nodes = ntiles + (uint64_t)runs * tile_nodes(g);
     const bool wide = nodes >= 0xffffffffull;
     uint32_t *k0 = nullptr, *k1 = nullptr, *v0 = nullptr, *v1 = nullptr;
     uint32_t *run_tile = nullptr, *run_len = nullptr, *long_tiles = nullptr;

@@ -102,7 +102,7 @@ typedef struct fc_params {
  * >= 3) through a kernel that stages 8-row tiles of the source rows in
  * shared memory with TMA tensor copies, instead of loading them directly;
  * results are identical. It is off by default: on B200 the direct loads are
- * faster (the step is issue-bound, not latency-bound). */
+ * faster. */
 #define FC_OPTION_TMA_STAGING 1
 /* TC_CLOSURE evaluates the learned closure's MLP in the ping-pong bulk step
  * on the tcgen05 tensor cores, once per block of 512 cells (shared-memory
