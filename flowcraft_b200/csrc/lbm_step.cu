@@ -1100,6 +1100,23 @@ __global__ void __launch_bounds__(128) k_boundary_pull_batch(const BatchLattice*
                          (uint32_t)(w - L.bnd_first), L.g, L.p, L.diverged);
 }
 
+// Boundary-list entries [begin, end) in a launch of their own, where there are
+// very many (a porous body): the step kernel's blocks hold 32 warps per SM, this
+// one 40 and more. B200, cells solid at random, a fifth (almost every fluid cell on
+// the list) / a fiftieth (a third), us per step inside -> apart: 256x128x128 FP16
+// 307 -> 248 / 242 -> 230, 384x192x192 with a fiftieth 775 -> 709; FP32, whose
+// step kernel calls the entry with registers of its own, 299 -> 277 / 339 -> 353,
+// so there only a list of more than half of the cells goes apart. 128x64x64 is
+// faster inside (34 against 40).
+constexpr size_t kListApart = size_t(1) << 20;
+template <int Q, class S>
+__global__ void __launch_bounds__(128) k_boundary_pull(const typename S::T* fin, typename S::T* fout, BoundaryList bl,
+                                                        uint32_t begin, uint32_t end, Geom g, StepParams p,
+                                                        int* __restrict__ diverged) {
+    const size_t e = (size_t)begin + (size_t)blockIdx.x * 128 + threadIdx.x;
+    if (e < end) boundary_entry<Q, S>(fin, fout, bl, (uint32_t)e, g, p, diverged);
+}
+
 // Plane pointers of a ping-pong step (PlanePtrs in lbm_internal.h).
 template <int Q, class S>
 static PlanePtrs pp_of(const void* fin, void* fout, const Geom& g) {
@@ -1154,11 +1171,20 @@ static cudaError_t bulk_t(const void* fin, void* fout, const uint32_t* bits, con
     const auto kernel = par == kNxEven ? k_bulk_pairs<Q, S, kNxEven>
                                        : (par == kNxOddNyOdd ? k_bulk_pairs<Q, S, kNxOddNyOdd>
                                                              : k_bulk_pairs<Q, S, kNxOddNyEven>);
-    return launch_with_slabs(bnd, grid.x, grid.y, zc > 0 ? zc : 0, launched, [&](const BoundarySpan& bs, unsigned layers) {
-        grid.z = layers + bs.slabs;
-        return launch_step_kernel(kernel, grid, block, s, bs.chained, (const typename S::T*)fin, (typename S::T*)fout,
-                                  bits, g, p, pp, z0, dv, sh, bs);
-    });
+    BoundarySpan inside = bnd;
+    const size_t entries = bnd.end - bnd.begin, cells = (size_t)g.nxy * (zc > 0 ? zc : 0);
+    const bool apart = entries >= kListApart && (!S::kExact || entries > cells / 2);
+    if (apart) inside.end = inside.begin;
+    const cudaError_t e =
+        launch_with_slabs(inside, grid.x, grid.y, zc > 0 ? zc : 0, launched, [&](const BoundarySpan& bs, unsigned layers) {
+            grid.z = layers + bs.slabs;
+            return launch_step_kernel(kernel, grid, block, s, bs.chained, (const typename S::T*)fin,
+                                      (typename S::T*)fout, bits, g, p, pp, z0, dv, sh, bs);
+        });
+    if (e != cudaSuccess || !apart) return e;
+    ++*launched;
+    return launch_step_kernel(k_boundary_pull<Q, S>, dim3((unsigned)((entries + 127) / 128)), dim3(128), s, false,
+                              (const typename S::T*)fin, (typename S::T*)fout, bnd.list, bnd.begin, bnd.end, g, p, dv);
 }
 
 template <int Q, class S>
